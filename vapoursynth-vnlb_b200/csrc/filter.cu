@@ -16,7 +16,7 @@
 //   jacobi   the cyclic Jacobi of many groups per warp, one lane per matrix
 //            row (a latency-bound chain of dependent rotations, so throughput
 //            comes from the number of groups in flight);
-//   apply    one CTA per group: dual -> primal basis, Wiener coefficients,
+//   apply    a warp or a CTA per group: dual -> primal basis, Wiener coefficients,
 //            precision and volume, then every retained row streamed once per
 //            warp for its membership score and its shrunken reconstruction,
 //            and finally the aggregation weights.
@@ -563,31 +563,18 @@ __device__ __forceinline__ float model_log_weight(const StageConfig& P, bool mem
 //   per-warp scratch (3 rows of ldb), row bases[max_rows] (size_t).
 // Row strides are padded (ldx = D + 1, ldb = D + 8) so that lanes reading
 // different rows at the same column hit different banks.
-// Row tiles of the tiled row loop: kTileRows rows per warp, at most
-// kTileComps components, and per row the folded dot products in kTileSlots
-// floats (membership dots [0, 16), reconstruction dots [16, 32), norm at 32).
-constexpr int kTileRows = 2;
-constexpr int kTileComps = 16;
-constexpr int kTileSlots = 33;
-
 struct ApplyLayout {
-    int D, Bmax, R, ldx, ldb, ldu, colpad;
-    size_t means, X, basis, dual, scal, scores, scratch, tile_floats, bases, bytes;
+    int D, Bmax, R, ldx, ldb, colpad;
+    size_t means, X, basis, dual, scal, scores, scratch, bases, bytes;
 };
 
-// tiled: the row loop of apply_kernel<true>, whose per-warp row tiles (the
-// centred rows at stride ldu = 8 mod 32, and the Final stage's noisy rows)
-// share their space with the model rows X, which are dead by then.
-__host__ __device__ inline ApplyLayout apply_layout(int D, int Bmax, int R, int max_rows, int warps,
-                                                    bool tiled = false, bool final_stage = false) {
+__host__ __device__ inline ApplyLayout apply_layout(int D, int Bmax, int R, int max_rows, int warps) {
     ApplyLayout a{};
     a.D = D;
     a.Bmax = Bmax;
     a.R = R;
     a.ldx = D + 1;
-    a.ldu = ((D + 23) & ~31) + 8;  // smallest stride >= D that is 8 mod 32
-    // basis rows: the tiled loop reads four components at one column, 8 banks apart
-    a.ldb = tiled ? a.ldu : D + 8;
+    a.ldb = D + 8;
     a.colpad = (D + 3) & ~3;
     size_t off = static_cast<size_t>(a.colpad);
     a.means = off;   off += 2 * static_cast<size_t>(D);
@@ -596,20 +583,12 @@ __host__ __device__ inline ApplyLayout apply_layout(int D, int Bmax, int R, int 
     a.scal = off;    off += 5 * static_cast<size_t>(R);
     a.scores = off;  off += static_cast<size_t>(max_rows);
     a.scratch = off;
-    if (tiled) {
-        a.tile_floats = static_cast<size_t>(final_stage ? 2 : 1) * kTileRows * a.ldu + kTileRows * kTileSlots;
-        a.X = off;
-        const size_t tiles = static_cast<size_t>(warps) * a.tile_floats;
-        const size_t model = static_cast<size_t>(Bmax) * a.ldx;
-        off += tiles > model ? tiles : model;
-    } else {
-        // the centred model rows are read only while the basis is built,
-        // before any warp uses its row scratch: they share the space
-        a.X = off;
-        const size_t rows = static_cast<size_t>(warps) * (2 * a.ldb + R + 1);
-        const size_t model = static_cast<size_t>(Bmax) * a.ldx;
-        off += rows > model ? rows : model;
-    }
+    // the centred model rows are read only while the basis is built,
+    // before any warp uses its row scratch: they share the space
+    a.X = off;
+    const size_t rows = static_cast<size_t>(warps) * (2 * a.ldb + R + 1);
+    const size_t model = static_cast<size_t>(Bmax) * a.ldx;
+    off += rows > model ? rows : model;
     off = (off + 1) & ~static_cast<size_t>(1);
     a.bases = off;   off += 2 * static_cast<size_t>(max_rows);
     a.bytes = off * sizeof(float);
@@ -625,15 +604,13 @@ __device__ __forceinline__ float octet_fold(float v) {
     return __fadd_rn(v, __shfl_xor_sync(0xffffffffu, v, 1));
 }
 
-// kTiled: rows in tiles of kTileRows per warp (rank <= kTileComps, dimension
-// above 16), else one row per warp with the components four at a time.
-template <bool kTiled>
+// One row per warp with the components four at a time: any shape.
 __global__ void __launch_bounds__(kApplyThreads, 3) apply_kernel(FilterLaunch L) {
     extern __shared__ __align__(16) float sm[];
     const int D = L.dim;
     const int Bmax = bmax_of(L);
     const int R = L.rank;
-    const ApplyLayout lay = apply_layout(D, Bmax, R, L.max_rows, kApplyWarps, kTiled, L.stage == 1);
+    const ApplyLayout lay = apply_layout(D, Bmax, R, L.max_rows, kApplyWarps);
     const int ldx = lay.ldx, ldb = lay.ldb;
     int* coloff = reinterpret_cast<int*>(sm);
     float* means = sm + lay.means;  // membership mean, reconstruction centre
@@ -770,238 +747,82 @@ __global__ void __launch_bounds__(kApplyThreads, 3) apply_kernel(FilterLaunch L)
         __syncthreads();
         const float lgw = s_misc[0];
         const float volume = s_misc[1];
-        if constexpr (kTiled) {
-            // Rows in tiles of kTileRows per warp.  Lane (j, g) runs the pinned
-            // chain j (elements j + 8m) of both tile rows against components
-            // g, g + 4, g + 8 and g + 12, so one basis load feeds the membership
-            // and the reconstruction chains of two rows; octet_fold folds the
-            // chains, and one lane per (row, dot) adds the unfused tail
-            // (dot_contiguous_highway: the operations of octet_dot8).
-            float* U = scratch + warp * lay.tile_floats;  // centred membership rows
-            float* V = U + kTileRows * lay.ldu;            // centred noisy rows (Final)
-            float* res = U + (final_stage ? 2 : 1) * kTileRows * lay.ldu;  // [row][kTileSlots]
-            const int ldu = lay.ldu;
-            const int j = lane & 7;
-            const int grp = lane >> 3;
-            const int full = D / kLanes;
-            const float score_scale = __fsqrt_rn(__fmul_rn(2.0f, static_cast<float>(D)));
-            for (int t0 = warp * kTileRows; t0 < S; t0 += kApplyWarps * kTileRows) {
-                const int nrows = min(kTileRows, S - t0);
-                for (int r = 0; r < nrows; ++r) {
-                    const size_t b = bases[t0 + r];
-                    for (int col = lane; col < D; col += 32) {
-                        const float xn = __ldg(L.noisy + b + coloff[col]);
-                        if (final_stage) {
-                            U[r * ldu + col] = __fsub_rn(__ldg(L.basic + b + coloff[col]), member_mean[col]);
-                            V[r * ldu + col] = __fsub_rn(xn, center_vec[col]);
-                        } else {
-                            U[r * ldu + col] = __fsub_rn(xn, member_mean[col]);
-                        }
+        // per row: membership score and reconstruction.  In the Basic stage the
+        // membership row and the reconstruction row are the same centred noisy
+        // row, so its projections serve both.
+        float* u = scratch + warp * (2 * ldb + R + 1);  // centred membership row
+        float* v = u + ldb;                             // centred noisy row (Final)
+        float* proj = v + ldb;                          // projections for the reconstruction
+        const int j8 = lane & 7;
+        const int oct = lane >> 3;
+        const float score_scale = __fsqrt_rn(__fmul_rn(2.0f, static_cast<float>(D)));
+        for (int i = warp; i < S; i += kApplyWarps) {
+            const size_t b = bases[i];
+            for (int col = lane; col < D; col += 32) {
+                const float xn = __ldg(L.noisy + b + coloff[col]);
+                if (final_stage) {
+                    u[col] = __fsub_rn(__ldg(L.basic + b + coloff[col]), member_mean[col]);
+                    v[col] = __fsub_rn(xn, center_vec[col]);
+                } else {
+                    u[col] = __fsub_rn(xn, member_mean[col]);
+                }
+            }
+            __syncwarp();
+            float distance = 0.0f, projected = 0.0f, norm2 = 0.0f;
+            // pass over c0 = -1 (norm), 0, 4, ...: octet k computes component c0 + k
+            for (int c0 = membership_on ? -1 : 0; c0 < R; c0 += 4) {
+                const int c = min(c0 + oct, R - 1);
+                const float dm = (membership_on || !final_stage) ? octet_dot8(u, c < 0 ? u : basis + c * ldb, D, j8)
+                                                                 : 0.0f;
+                const float dr = final_stage ? octet_dot8(v, basis + max(c, 0) * ldb, D, j8) : dm;
+                for (int k = 0; k < 4; ++k) {
+                    const int ck = c0 + k;
+                    const float mk = __shfl_sync(0xffffffffu, dm, k * 8);
+                    const float rk = __shfl_sync(0xffffffffu, dr, k * 8);
+                    if (ck >= R) break;
+                    if (ck < 0) {
+                        norm2 = mk;
+                        continue;
                     }
-                }
-                __syncwarp();
-                const int r1 = nrows > 1 ? 1 : 0;  // a missing second row repeats the first
-                float am[kTileRows][4], ar[kTileRows][4], an[kTileRows];
-#pragma unroll
-                for (int r = 0; r < kTileRows; ++r) {
-                    an[r] = 0.0f;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) am[r][k] = ar[r][k] = 0.0f;
-                }
-                for (int m = 0; m < full; ++m) {
-                    const int col = j + kLanes * m;
-                    const float u0 = U[col], u1 = U[r1 * ldu + col];
-                    an[0] = __fmaf_rn(u0, u0, an[0]);
-                    an[1] = __fmaf_rn(u1, u1, an[1]);
-                    if (final_stage) {
-                        const float v0 = V[col], v1 = V[r1 * ldu + col];
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (grp + 4 * k < R) {
-                                const float bv = basis[(grp + 4 * k) * ldb + col];
-                                am[0][k] = __fmaf_rn(u0, bv, am[0][k]);
-                                am[1][k] = __fmaf_rn(u1, bv, am[1][k]);
-                                ar[0][k] = __fmaf_rn(v0, bv, ar[0][k]);
-                                ar[1][k] = __fmaf_rn(v1, bv, ar[1][k]);
-                            }
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            if (grp + 4 * k < R) {
-                                const float bv = basis[(grp + 4 * k) * ldb + col];
-                                am[0][k] = __fmaf_rn(u0, bv, am[0][k]);
-                                am[1][k] = __fmaf_rn(u1, bv, am[1][k]);
-                            }
-                    }
-                }
-                // fold; lane j of octet grp stores (row j / 4, component grp + 4 (j % 4))
-#pragma unroll
-                for (int r = 0; r < kTileRows; ++r) {
-                    an[r] = octet_fold(an[r]);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        am[r][k] = octet_fold(am[r][k]);
-                        if (final_stage) ar[r][k] = octet_fold(ar[r][k]);
-                    }
-                }
-#pragma unroll
-                for (int r = 0; r < kTileRows; ++r)
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (j == 4 * r + k && grp + 4 * k < R) {
-                            res[r * kTileSlots + grp + 4 * k] = am[r][k];
-                            if (final_stage) res[r * kTileSlots + 16 + grp + 4 * k] = ar[r][k];
-                        }
-                if (lane < kTileRows) res[lane * kTileSlots + 32] = lane == 0 ? an[0] : an[1];
-                __syncwarp();
-                if (full * kLanes < D) {
-                    // the unfused tail of each dot: lane -> (row, slot)
-                    for (int e = lane; e < kTileRows * kTileSlots; e += 32) {
-                        const int r = e / kTileSlots;
-                        const int slot = e - r * kTileSlots;
-                        const bool norm = slot == 32;
-                        const bool recon = slot >= 16 && !norm;
-                        const int c = norm ? 0 : (recon ? slot - 16 : slot);
-                        if (r >= nrows || (!norm && (c >= R || (recon && !final_stage)))) continue;
-                        const float* l = (recon ? V : U) + r * ldu;
-                        const float* rgt = norm ? U + r * ldu : basis + c * ldb;
-                        float total = res[e];
-                        for (int idx = full * kLanes; idx < D; ++idx)
-                            total = __fadd_rn(total, __fmul_rn(l[idx], rgt[idx]));
-                        res[e] = total;
-                    }
-                    __syncwarp();
-                }
-                // membership score of each row, components in order
-                if (lane < nrows && membership_on) {
-                    const float* rr = res + lane * kTileSlots;
-                    float distance = 0.0f, projected = 0.0f;
-                    for (int ck = 0; ck < R; ++ck) {
-                        const float mk = rr[ck];
+                    if (membership_on) {
                         const float proj2 = __fmul_rn(mk, mk);
                         distance = __fadd_rn(distance, __fdiv_rn(proj2, denom[ck]));
                         projected = __fadd_rn(projected, proj2);
                     }
-                    const float resid = __fsub_rn(rr[32], projected);
-                    distance = __fadd_rn(distance, __fdiv_rn(resid > 0.0f ? resid : 0.0f, mem2));
-                    scores[t0 + lane] = __fdiv_rn(__fsub_rn(distance, static_cast<float>(D)), score_scale);
+                    if (lane == 0) proj[ck] = rk;
                 }
-                // reconstruction (project_bayes_estimate) of the tile's rows,
-                // components in order, in registers over blocks of 32 * kRecCols
-                const int proj_slot = final_stage ? 16 : 0;
-                for (int base = 0; base < D; base += 32 * kRecCols) {
-                    float o[kTileRows][kRecCols];
-#pragma unroll
-                    for (int r = 0; r < kTileRows; ++r)
-#pragma unroll
-                        for (int jj = 0; jj < kRecCols; ++jj) o[r][jj] = 0.0f;
-                    for (int c = 0; c < R; ++c) {
-                        const float cf = coef[c];
-                        if (cf == 0.0f) continue;
-                        const float sc0 = __fmul_rn(cf, res[proj_slot + c]);
-                        const float sc1 = __fmul_rn(cf, res[kTileSlots + proj_slot + c]);
-                        const float* bc = basis + c * ldb;
-#pragma unroll
-                        for (int jj = 0; jj < kRecCols; ++jj) {
-                            const int col = base + lane + 32 * jj;
-                            if (col < D) {
-                                const float bv = bc[col];
-                                o[0][jj] = add_scaled_elem(o[0][jj], bv, sc0, col, D);
-                                o[1][jj] = add_scaled_elem(o[1][jj], bv, sc1, col, D);
-                            }
-                        }
-                    }
-#pragma unroll
-                    for (int r = 0; r < kTileRows; ++r) {
-                        if (r >= nrows) break;
-                        float* out = L.filtered + static_cast<size_t>(r0 + t0 + r) * L.row_dim + mc * D;
-#pragma unroll
-                        for (int jj = 0; jj < kRecCols; ++jj) {
-                            const int col = base + lane + 32 * jj;
-                            if (col < D) out[col] = __fadd_rn(o[r][jj], center_vec[col]);
-                        }
-                    }
-                }
-                __syncwarp();
             }
-        } else {
-            // per row: membership score and reconstruction.  In the Basic stage the
-            // membership row and the reconstruction row are the same centred noisy
-            // row, so its projections serve both.
-            float* u = scratch + warp * (2 * ldb + R + 1);  // centred membership row
-            float* v = u + ldb;                             // centred noisy row (Final)
-            float* proj = v + ldb;                          // projections for the reconstruction
-            const int j8 = lane & 7;
-            const int oct = lane >> 3;
-            const float score_scale = __fsqrt_rn(__fmul_rn(2.0f, static_cast<float>(D)));
-            for (int i = warp; i < S; i += kApplyWarps) {
-                const size_t b = bases[i];
-                for (int col = lane; col < D; col += 32) {
-                    const float xn = __ldg(L.noisy + b + coloff[col]);
-                    if (final_stage) {
-                        u[col] = __fsub_rn(__ldg(L.basic + b + coloff[col]), member_mean[col]);
-                        v[col] = __fsub_rn(xn, center_vec[col]);
-                    } else {
-                        u[col] = __fsub_rn(xn, member_mean[col]);
-                    }
-                }
-                __syncwarp();
-                float distance = 0.0f, projected = 0.0f, norm2 = 0.0f;
-                // pass over c0 = -1 (norm), 0, 4, ...: octet k computes component c0 + k
-                for (int c0 = membership_on ? -1 : 0; c0 < R; c0 += 4) {
-                    const int c = min(c0 + oct, R - 1);
-                    const float dm = (membership_on || !final_stage) ? octet_dot8(u, c < 0 ? u : basis + c * ldb, D, j8)
-                                                                     : 0.0f;
-                    const float dr = final_stage ? octet_dot8(v, basis + max(c, 0) * ldb, D, j8) : dm;
-                    for (int k = 0; k < 4; ++k) {
-                        const int ck = c0 + k;
-                        const float mk = __shfl_sync(0xffffffffu, dm, k * 8);
-                        const float rk = __shfl_sync(0xffffffffu, dr, k * 8);
-                        if (ck >= R) break;
-                        if (ck < 0) {
-                            norm2 = mk;
-                            continue;
-                        }
-                        if (membership_on) {
-                            const float proj2 = __fmul_rn(mk, mk);
-                            distance = __fadd_rn(distance, __fdiv_rn(proj2, denom[ck]));
-                            projected = __fadd_rn(projected, proj2);
-                        }
-                        if (lane == 0) proj[ck] = rk;
-                    }
-                }
-                if (membership_on) {
-                    const float res = __fsub_rn(norm2, projected);
-                    distance = __fadd_rn(distance, __fdiv_rn(res > 0.0f ? res : 0.0f, mem2));
-                    const float score = __fdiv_rn(__fsub_rn(distance, static_cast<float>(D)), score_scale);
-                    if (lane == 0) scores[i] = score;
-                }
-                __syncwarp();
-                // reconstruction (project_bayes_estimate), components in order,
-                // accumulated in registers over blocks of 32 * kRecCols columns
-                float* out = L.filtered + static_cast<size_t>(r0 + i) * L.row_dim + mc * D;
-                for (int base = 0; base < D; base += 32 * kRecCols) {
-                    float o[kRecCols];
+            if (membership_on) {
+                const float res = __fsub_rn(norm2, projected);
+                distance = __fadd_rn(distance, __fdiv_rn(res > 0.0f ? res : 0.0f, mem2));
+                const float score = __fdiv_rn(__fsub_rn(distance, static_cast<float>(D)), score_scale);
+                if (lane == 0) scores[i] = score;
+            }
+            __syncwarp();
+            // reconstruction (project_bayes_estimate), components in order,
+            // accumulated in registers over blocks of 32 * kRecCols columns
+            float* out = L.filtered + static_cast<size_t>(r0 + i) * L.row_dim + mc * D;
+            for (int base = 0; base < D; base += 32 * kRecCols) {
+                float o[kRecCols];
 #pragma unroll
-                    for (int j = 0; j < kRecCols; ++j) o[j] = 0.0f;
-                    for (int c = 0; c < R; ++c) {
-                        if (coef[c] == 0.0f) continue;
-                        const float scaled = __fmul_rn(coef[c], proj[c]);
-                        const float* bc = basis + c * ldb;
-#pragma unroll
-                        for (int j = 0; j < kRecCols; ++j) {
-                            const int col = base + lane + 32 * j;
-                            if (col < D) o[j] = add_scaled_elem(o[j], bc[col], scaled, col, D);
-                        }
-                    }
+                for (int j = 0; j < kRecCols; ++j) o[j] = 0.0f;
+                for (int c = 0; c < R; ++c) {
+                    if (coef[c] == 0.0f) continue;
+                    const float scaled = __fmul_rn(coef[c], proj[c]);
+                    const float* bc = basis + c * ldb;
 #pragma unroll
                     for (int j = 0; j < kRecCols; ++j) {
                         const int col = base + lane + 32 * j;
-                        if (col < D) out[col] = __fadd_rn(o[j], center_vec[col]);
+                        if (col < D) o[j] = add_scaled_elem(o[j], bc[col], scaled, col, D);
                     }
                 }
-                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < kRecCols; ++j) {
+                    const int col = base + lane + 32 * j;
+                    if (col < D) out[col] = __fadd_rn(o[j], center_vec[col]);
+                }
             }
+            __syncwarp();
         }
         __syncthreads();
         // aggregation weights (accumulate_aggregation_model + finalize)
@@ -1033,6 +854,553 @@ __global__ void __launch_bounds__(kApplyThreads, 3) apply_kernel(FilterLaunch L)
                 } else {
                     lw = __fadd_rn(0.0f, lgw);
                 }
+                lw = lw < -80.0f ? -80.0f : (80.0f < lw ? 80.0f : lw);
+                w = cr_expf(lw);
+            }
+            L.weights[r0 + i] = w;
+        }
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// apply, row tiles: a CTA of up to kTileWarps warps per group, for ranks up to
+// 4 * 4 * kQ that the warp-per-group kernel does not take (large groups and
+// dimensions: blocks of 7 over two frames and three planes, groups of 16 grown
+// to 64 rows).
+//
+// Measured against one group per 8-warp CTA with two rows per warp and scalar
+// shared loads (B200, one launch alone, 57k groups of dimension 294, rank 15):
+// Basic 2.75 -> 1.19 ms, Final 3.72 -> 2.17 ms; 130k groups of dimension 128,
+// rank 16: 6.7 -> 2.87 and 7.7 -> 3.34 ms.
+// Bound by shared-memory wavefronts and FP32 issue, so the layouts serve wide
+// loads: the basis is [column][component], padded to 4 mod 8 quads so that the
+// 8 columns of a quarter warp start on different banks, and a warp's tile of
+// kTileRows rows is [column][row].  One 16-byte load then brings four
+// components (or all four rows) of a column.  Lane (j, g) runs the pinned
+// chain j (columns j + 8 m) of four rows against components 4 g .. 4 g + 3 of
+// each block of 16; the chains are folded by halving exchanges (the additions
+// of reduce8: xor 4, 2, 1), which leaves each lane with one row's dots of two
+// components, and the unfused tail, the division by the component's
+// variance and the shrinkage follow there.  The reconstruction takes blocks of
+// 32 columns, one per lane and block, all components of a column in registers.
+constexpr int kTileRows = 4;
+constexpr int kTileWarps = 4;
+
+struct TileApplyLayout {
+    int ldb, coloff, means, basis, dual, scal, scores, bases, tiles, tile_floats, bytes;
+};
+
+// kq: components in blocks of 16; per warp U [D][4], V [D][4] (Final), and per
+// block of 16 the scaled projections [16][4], quotients [4][16] and squares
+// [4][16], then the 4 norms.
+__host__ __device__ inline TileApplyLayout tile_apply_layout(int D, int Bmax, int kq, int max_rows, int warps,
+                                                             bool final_stage) {
+    TileApplyLayout a{};
+    const int comps = 16 * kq;
+    a.ldb = comps + 4;
+    int off = 0;
+    a.coloff = off;  off += (D + 3) & ~3;
+    a.means = off;   off += (2 * D + 3) & ~3;
+    a.basis = off;   off += D * a.ldb;
+    a.dual = off;    off += Bmax * comps;
+    a.scal = off;    off += 5 * comps;
+    a.scores = off;  off += (max_rows + 3) & ~3;
+    a.bases = off;   off += 2 * ((max_rows + 1) & ~1);
+    a.tiles = off;
+    a.tile_floats = (final_stage ? 2 : 1) * kTileRows * D + 3 * kTileRows * comps + 4;
+    off += warps * a.tile_floats;
+    a.bytes = off * static_cast<int>(sizeof(float));
+    return a;
+}
+
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+
+// Dual -> primal basis of kCols columns (tid + 128-strided) of one thread:
+// acc[c] += dual[c][s] * x_s[col], the samples in order, then the scale.
+template <int kQ, int kCols>
+__device__ __forceinline__ void tile_basis_columns(const FilterLaunch& L, const float* model_video, const size_t* bases,
+                                                   const int* coloff, const float* mean, const float* dual,
+                                                   const float* inv_sqrt, float* basis, int ldb, int D, int B, int col0,
+                                                   int stride) {
+    constexpr int kComps = 16 * kQ;
+    const int full = (D / kLanes) * kLanes;
+    int off[kCols];
+    float mm[kCols];
+    bool tail = false;
+#pragma unroll
+    for (int k = 0; k < kCols; ++k) {
+        const int col = min(col0 + k * stride, D - 1);
+        off[k] = coloff[col];
+        mm[k] = mean[col];
+        tail |= col >= full;
+    }
+#pragma unroll
+    for (int c0 = 0; c0 < kComps; c0 += 16) {
+        float2 acc[kCols][8];
+#pragma unroll
+        for (int k = 0; k < kCols; ++k)
+#pragma unroll
+            for (int p = 0; p < 8; ++p) acc[k][p] = make_float2(0.0f, 0.0f);
+        if (!tail) {
+#pragma unroll 4
+            for (int s = 0; s < B; ++s) {
+                const float* src = model_video + bases[s];
+                float x[kCols];
+#pragma unroll
+                for (int k = 0; k < kCols; ++k) x[k] = __fsub_rn(__ldg(src + off[k]), mm[k]);
+                const float4* w4 = reinterpret_cast<const float4*>(dual + s * kComps + c0);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float4 w = w4[q];
+#pragma unroll
+                    for (int k = 0; k < kCols; ++k) {
+                        acc[k][2 * q] = fma2_rn(dup2(x[k]), make_float2(w.x, w.y), acc[k][2 * q]);
+                        acc[k][2 * q + 1] = fma2_rn(dup2(x[k]), make_float2(w.z, w.w), acc[k][2 * q + 1]);
+                    }
+                }
+            }
+        } else {
+            // a column past the last full chunk of 8 is among them: unfused there
+            for (int s = 0; s < B; ++s) {
+                const float* src = model_video + bases[s];
+                const float* w = dual + s * kComps + c0;
+#pragma unroll
+                for (int k = 0; k < kCols; ++k) {
+                    const float x = __fsub_rn(__ldg(src + off[k]), mm[k]);
+                    const bool fused = col0 + k * stride < full;
+#pragma unroll
+                    for (int p = 0; p < 8; ++p) {
+                        const float2 a = acc[k][p];
+                        const float w0 = w[2 * p], w1 = w[2 * p + 1];
+                        acc[k][p] = fused ? make_float2(__fmaf_rn(w0, x, a.x), __fmaf_rn(w1, x, a.y))
+                                          : make_float2(__fadd_rn(a.x, __fmul_rn(w0, x)),
+                                                        __fadd_rn(a.y, __fmul_rn(w1, x)));
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kCols; ++k) {
+            const int col = col0 + k * stride;
+            if (col >= D) continue;
+            float4* out = reinterpret_cast<float4*>(basis + col * ldb + c0);
+            const float* is = inv_sqrt + c0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                out[q] = make_float4(__fmul_rn(acc[k][2 * q].x, is[4 * q]), __fmul_rn(acc[k][2 * q].y, is[4 * q + 1]),
+                                     __fmul_rn(acc[k][2 * q + 1].x, is[4 * q + 2]),
+                                     __fmul_rn(acc[k][2 * q + 1].y, is[4 * q + 3]));
+        }
+    }
+}
+
+// Reconstruction (project_bayes_estimate) of a tile's rows over kBlocks blocks
+// of 32 columns, components in order, and its store.
+template <int kBlocks, bool kTail>
+__device__ __forceinline__ void tile_reconstruct(const float* basis, int ldb, const float* coef, const float* sc,
+                                                 const float* center, int R, int D, int base, int lane, float* out,
+                                                 size_t row_stride, int nrows) {
+    float2 o[kBlocks][2];  // rows (0, 1) and (2, 3)
+    int col[kBlocks];
+    const int full = (D / kLanes) * kLanes;
+#pragma unroll
+    for (int k = 0; k < kBlocks; ++k) {
+        col[k] = min(base + 32 * k + lane, D - 1);
+        o[k][0] = o[k][1] = make_float2(0.0f, 0.0f);
+    }
+    for (int c0 = 0; c0 < R; c0 += 4) {
+        float b[kBlocks][4];
+#pragma unroll
+        for (int k = 0; k < kBlocks; ++k) {
+            const float4 t = *reinterpret_cast<const float4*>(basis + col[k] * ldb + c0);
+            b[k][0] = t.x;
+            b[k][1] = t.y;
+            b[k][2] = t.z;
+            b[k][3] = t.w;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c0 + c >= R || coef[c0 + c] == 0.0f) continue;
+            const float4 s = *reinterpret_cast<const float4*>(sc + (c0 + c) * kTileRows);
+            const float2 s01 = make_float2(s.x, s.y), s23 = make_float2(s.z, s.w);
+#pragma unroll
+            for (int k = 0; k < kBlocks; ++k) {
+                if (kTail && col[k] >= full) {
+                    const float v = b[k][c];
+                    o[k][0] = make_float2(__fadd_rn(o[k][0].x, __fmul_rn(s.x, v)),
+                                          __fadd_rn(o[k][0].y, __fmul_rn(s.y, v)));
+                    o[k][1] = make_float2(__fadd_rn(o[k][1].x, __fmul_rn(s.z, v)),
+                                          __fadd_rn(o[k][1].y, __fmul_rn(s.w, v)));
+                } else {
+                    o[k][0] = fma2_rn(s01, dup2(b[k][c]), o[k][0]);
+                    o[k][1] = fma2_rn(s23, dup2(b[k][c]), o[k][1]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kBlocks; ++k) {
+        if (base + 32 * k + lane >= D) continue;
+        const float mid = center[col[k]];
+        float* at = out + col[k];
+        at[0] = __fadd_rn(o[k][0].x, mid);
+        if (nrows > 1) at[row_stride] = __fadd_rn(o[k][0].y, mid);
+        if (nrows > 2) at[2 * row_stride] = __fadd_rn(o[k][1].x, mid);
+        if (nrows > 3) at[3 * row_stride] = __fadd_rn(o[k][1].y, mid);
+    }
+}
+
+// One step of the halving fold: keeps `keep`, adds the partner's copy of it.
+__device__ __forceinline__ float fold_half(float keep, float send, int mask) {
+    return __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, mask));
+}
+
+// Folds the octet chains v[row][component]: lane j ends with row r =
+// (j & 4) / 2 + (j & 2) / 2 and components 2 (j & 1), 2 (j & 1) + 1.
+__device__ __forceinline__ float2 fold_tile(const float2 (&v)[kTileRows][2], int j) {
+    float2 a[2][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const float2 lo = v[r][p], hi = v[r + 2][p];
+            a[r][p].x = fold_half((j & 4) ? hi.x : lo.x, (j & 4) ? lo.x : hi.x, 4);
+            a[r][p].y = fold_half((j & 4) ? hi.y : lo.y, (j & 4) ? lo.y : hi.y, 4);
+        }
+    float2 b[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        b[p].x = fold_half((j & 2) ? a[1][p].x : a[0][p].x, (j & 2) ? a[0][p].x : a[1][p].x, 2);
+        b[p].y = fold_half((j & 2) ? a[1][p].y : a[0][p].y, (j & 2) ? a[0][p].y : a[1][p].y, 2);
+    }
+    float2 c;
+    c.x = fold_half((j & 1) ? b[1].x : b[0].x, (j & 1) ? b[0].x : b[1].x, 1);
+    c.y = fold_half((j & 1) ? b[1].y : b[0].y, (j & 1) ? b[0].y : b[1].y, 1);
+    return c;
+}
+
+template <int kQ, bool kFinal>
+__global__ void __launch_bounds__(32 * kTileWarps, kQ == 1 ? 4 : 2) apply_tile_kernel(FilterLaunch L) {
+    constexpr int kComps = 16 * kQ;
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float s_misc[4];
+    const int D = L.dim;
+    const int Bmax = bmax_of(L);
+    const int R = L.rank;
+    const int threads = blockDim.x;
+    const TileApplyLayout lay = tile_apply_layout(D, Bmax, kQ, L.max_rows, threads / 32, kFinal);
+    const int ldb = lay.ldb;
+    int* coloff = reinterpret_cast<int*>(sm);
+    float* means = sm + lay.means;  // membership mean, reconstruction centre
+    float* basis = sm + lay.basis;
+    float* dual = sm + lay.dual;    // [sample][component]
+    float* eig = sm + lay.scal;
+    float* coef = eig + kComps;      // Wiener coefficients
+    float* denom = coef + kComps;    // signal eigenvalue + membership noise
+    float* inv_sqrt = denom + kComps;  // 1 / sqrt(eigenvalue), 0 below the floor
+    float* terms = inv_sqrt + kComps;  // log1p(signal / membership noise)
+    float* scores = sm + lay.scores;
+    size_t* bases = reinterpret_cast<size_t*>(sm + lay.bases);
+    const int tid = threadIdx.x;
+    const int warp = tid >> 5;
+    const int lane = tid & 31;
+    const int warps = threads >> 5;
+    const int j = lane & 7;
+    const int grp = lane >> 3;
+    float* U = sm + lay.tiles + warp * lay.tile_floats;  // centred membership rows [D][4]
+    float* V = U + kTileRows * D;                         // centred noisy rows (Final)
+    float* sc = U + (kFinal ? 2 : 1) * kTileRows * D;     // scaled projections [component][row]
+    float* quot = sc + kTileRows * kComps;                // projection^2 / variance [row][component]
+    float* square = quot + kTileRows * kComps;            // projection^2 [row][component]
+    float* norms = square + kTileRows * kComps;           // [row]
+    for (int col = tid; col < D; col += threads) coloff[col] = column_offset(L, col);
+    const StageConfig& P = L.cfg;
+    const float* model_video = kFinal ? L.basic : L.noisy;
+    const bool weights_enabled = P.weight_alpha != 0.0f || P.weight_beta != 0.0f || P.weight_gamma != 0.0f;
+    const float sigma2 = __fmul_rn(__fmul_rn(P.beta, P.sigma), P.sigma);
+    const float model_noise2 = kFinal ? __fmul_rn(__fmul_rn(P.beta, P.sigma_basic), P.sigma_basic) : sigma2;
+    const float match_sigma = kFinal ? P.sigma_basic : P.sigma;
+    const float mem2 = std_max(__fmul_rn(match_sigma, match_sigma),
+                               __fmul_rn(__fmul_rn(P.membership_noise_floor, P.sigma), P.sigma));
+    const bool membership_on = P.weight_beta != 0.0f;
+    const int total = L.counters->active * L.models;
+    const int models = L.models;  // models per group (planes when uncoupled)
+    const size_t hw = static_cast<size_t>(L.height) * L.width;
+    const int full = D / kLanes;
+    const bool has_tail = full * kLanes < D;
+    const float score_scale = __fsqrt_rn(__fmul_rn(2.0f, static_cast<float>(D)));
+    // the next group's flag and anchor are loaded an iteration ahead
+    int mi = blockIdx.x;
+    int flag = 0, g = 0;
+    if (mi < total) {
+        flag = L.flags[mi];
+        g = L.active[mi / models];
+    }
+    __syncthreads();
+    for (; mi < total;) {
+        const int a = mi / models;
+        const int mc = mi - a * models;
+        const int cur = mi, cur_flag = flag, cur_g = g;
+        mi += gridDim.x;
+        if (mi < total) {
+            flag = L.flags[mi];
+            g = L.active[mi / models];
+        }
+        if (cur_flag != 0) continue;  // uniform: equal groups are done, skipped ones reported
+        const int S = L.row_counts[cur_g];
+        const MatchRow* rows = L.rows + static_cast<size_t>(cur_g) * L.max_rows;
+        const int r0 = L.row_offset[a];
+        const int B = min(S, L.model_cap);
+        const int N = L.nmax;  // row stride of the eigenvector rows
+        const bool dual_model = D >= 64 && B < D;  // use_dual_pca (core.cpp:656-658)
+        const float* gm = L.means + static_cast<size_t>(cur) * 2 * D;
+        const float* gd = L.dual + static_cast<size_t>(cur) * R * N;
+        for (int i = tid; i < S; i += threads) bases[i] = row_base(L, rows[i]) + mc * hw;  // this model's plane
+        for (int i = tid; i < 2 * D; i += threads) means[i] = gm[i];
+        if (dual_model)
+            for (int i = tid; i < B * kComps; i += threads) {
+                const int c = i / B, s = i - c * B;
+                dual[s * kComps + c] = c < R ? gd[c * N + s] : 0.0f;
+            }
+        // per-component scalars, once per group
+        if (tid < kComps) {
+            const int c = tid;
+            const float lambda = c < R ? L.eig[static_cast<size_t>(cur) * R + c] : 0.0f;
+            eig[c] = lambda;
+            const float diff = __fsub_rn(lambda, model_noise2);
+            const float signal = diff > 0.0f ? diff : 0.0f;
+            denom[c] = __fadd_rn(signal, mem2);
+            inv_sqrt[c] = lambda > kEigenFloor ? __fdiv_rn(1.0f, __fsqrt_rn(lambda)) : 0.0f;
+            terms[c] = (membership_on && signal > 0.0f) ? cr_log1pf(__fdiv_rn(signal, mem2)) : 0.0f;
+            const float sigma_basic2 = kFinal ? model_noise2 : sigma2;
+            const float threshold = __fmul_rn(P.variance_threshold, sigma2);
+            float variance = lambda;
+            if (sigma_basic2 > 0.0f) variance = __fsub_rn(variance, std_min(variance, sigma_basic2));
+            coef[c] = c < R && variance > threshold ? __fdiv_rn(1.0f, __fadd_rn(1.0f, __fdiv_rn(sigma2, variance)))
+                                                    : 0.0f;
+        }
+        __syncthreads();
+        const float* member_mean = means;
+        const float* center_vec = means + D;
+        if (dual_model) {
+            // dual -> primal basis (map_dual_eigenvectors_to_basis); components
+            // at or below the floor are zero
+            for (int col = tid; col < D; col += 2 * threads) {
+                if (col - lane + threads < D)
+                    tile_basis_columns<kQ, 2>(L, model_video, bases, coloff, member_mean, dual, inv_sqrt, basis, ldb, D,
+                                              B, col, threads);
+                else
+                    tile_basis_columns<kQ, 1>(L, model_video, bases, coloff, member_mean, dual, inv_sqrt, basis, ldb, D,
+                                              B, col, threads);
+            }
+            __syncthreads();
+            for (int b0 = 4 * warp; b0 < R; b0 += 4 * warps) {
+                const int b = min(b0 + grp, kComps - 1);  // an octet per component
+                const float* col = basis + j * ldb + b;
+                float v = 0.0f;
+#pragma unroll 4
+                for (int m = 0; m < full; ++m) {
+                    const float x = col[m * kLanes * ldb];
+                    v = __fmaf_rn(x, x, v);
+                }
+                float norm2 = octet_fold(v);
+                for (int idx = full * kLanes; idx < D; ++idx) {
+                    const float x = basis[idx * ldb + b];
+                    norm2 = __fadd_rn(norm2, __fmul_rn(x, x));
+                }
+                __syncwarp();  // every lane has read its component's column
+                const bool live = b < R && eig[b] > kEigenFloor;
+                const bool none = !live || norm2 <= kEigenFloor;
+                const float s = none ? 0.0f : __fdiv_rn(1.0f, __fsqrt_rn(norm2));
+                for (int c = j; c < D; c += kLanes) {
+                    float* at = basis + c * ldb + b;
+                    *at = none ? 0.0f : __fmul_rn(*at, s);
+                }
+            }
+        } else {
+            // covariance model: the canonicalised eigenvectors are the basis
+            for (int i = tid; i < kComps * D; i += threads) {
+                const int c = i / D, col = i - c * D;
+                basis[col * ldb + c] = c < R ? gd[static_cast<size_t>(c) * N + col] : 0.0f;
+            }
+        }
+        // group precision and volume (group_precision_tau, core.cpp:222-241,
+        // 346-358): the terms are ready, the sums run in component order
+        if (tid == threads - 1) {
+            float trace = 0.0f, volume = 0.0f;
+            for (int c = 0; c < R; ++c) {
+                const float diff = __fsub_rn(eig[c], model_noise2);
+                const float lambda = diff > 0.0f ? diff : 0.0f;
+                if (lambda > 0.0f) {
+                    trace = __fadd_rn(trace, __fdiv_rn(lambda, __fadd_rn(lambda, sigma2)));
+                    volume = __fadd_rn(volume, terms[c]);
+                }
+            }
+            const float tau = __fadd_rn(
+                __fadd_rn(P.weight_epsilon, __fdiv_rn(static_cast<float>(D), static_cast<float>(B))), trace);
+            s_misc[0] = P.weight_alpha == 0.0f ? 0.0f : __fmul_rn(-P.weight_alpha, cr_logf(tau));
+            s_misc[1] = __fdiv_rn(volume, static_cast<float>(D));
+        }
+        __syncthreads();
+        for (int t0 = warp * kTileRows; t0 < S; t0 += warps * kTileRows) {
+            const int nrows = min(kTileRows, S - t0);
+            {
+                // a missing row repeats the first
+                const size_t b0 = bases[t0], b1 = bases[t0 + (nrows > 1 ? 1 : 0)];
+                const size_t b2 = bases[t0 + (nrows > 2 ? 2 : 0)], b3 = bases[t0 + (nrows > 3 ? 3 : 0)];
+#pragma unroll 2
+                for (int col = lane; col < D; col += 32) {
+                    const int off = coloff[col];
+                    const float m = member_mean[col];
+                    const float* nz = L.noisy + off;
+                    const float x0 = __ldg(nz + b0), x1 = __ldg(nz + b1), x2 = __ldg(nz + b2), x3 = __ldg(nz + b3);
+                    if constexpr (kFinal) {
+                        const float* bs = L.basic + off;
+                        const float y0 = __ldg(bs + b0), y1 = __ldg(bs + b1), y2 = __ldg(bs + b2), y3 = __ldg(bs + b3);
+                        const float c = center_vec[col];
+                        *reinterpret_cast<float4*>(U + 4 * col) = make_float4(__fsub_rn(y0, m), __fsub_rn(y1, m),
+                                                                              __fsub_rn(y2, m), __fsub_rn(y3, m));
+                        *reinterpret_cast<float4*>(V + 4 * col) = make_float4(__fsub_rn(x0, c), __fsub_rn(x1, c),
+                                                                              __fsub_rn(x2, c), __fsub_rn(x3, c));
+                    } else {
+                        *reinterpret_cast<float4*>(U + 4 * col) = make_float4(__fsub_rn(x0, m), __fsub_rn(x1, m),
+                                                                              __fsub_rn(x2, m), __fsub_rn(x3, m));
+                    }
+                }
+            }
+            __syncwarp();
+            const int r = ((j >> 2) << 1) | ((j >> 1) & 1);  // this lane's row after the folds
+#pragma unroll
+            for (int q = 0; q < kQ; ++q) {
+                float2 am[kTileRows][2], ar[kTileRows][2], an[2];
+                an[0] = an[1] = make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int i = 0; i < kTileRows; ++i)
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) am[i][p] = ar[i][p] = make_float2(0.0f, 0.0f);
+                const float* bp = basis + j * ldb + 16 * q + 4 * grp;
+                const float* up = U + 4 * j;
+                const float* vp = V + 4 * j;
+#pragma unroll 2
+                for (int m = 0; m < full; ++m) {
+                    const float4 bv = *reinterpret_cast<const float4*>(bp + m * kLanes * ldb);
+                    const float2 b01 = make_float2(bv.x, bv.y), b23 = make_float2(bv.z, bv.w);
+                    const float4 u = *reinterpret_cast<const float4*>(up + m * 4 * kLanes);
+                    am[0][0] = fma2_rn(dup2(u.x), b01, am[0][0]);
+                    am[0][1] = fma2_rn(dup2(u.x), b23, am[0][1]);
+                    am[1][0] = fma2_rn(dup2(u.y), b01, am[1][0]);
+                    am[1][1] = fma2_rn(dup2(u.y), b23, am[1][1]);
+                    am[2][0] = fma2_rn(dup2(u.z), b01, am[2][0]);
+                    am[2][1] = fma2_rn(dup2(u.z), b23, am[2][1]);
+                    am[3][0] = fma2_rn(dup2(u.w), b01, am[3][0]);
+                    am[3][1] = fma2_rn(dup2(u.w), b23, am[3][1]);
+                    if (q == 0) {
+                        const float2 u01 = make_float2(u.x, u.y), u23 = make_float2(u.z, u.w);
+                        an[0] = fma2_rn(u01, u01, an[0]);
+                        an[1] = fma2_rn(u23, u23, an[1]);
+                    }
+                    if constexpr (kFinal) {
+                        const float4 v = *reinterpret_cast<const float4*>(vp + m * 4 * kLanes);
+                        ar[0][0] = fma2_rn(dup2(v.x), b01, ar[0][0]);
+                        ar[0][1] = fma2_rn(dup2(v.x), b23, ar[0][1]);
+                        ar[1][0] = fma2_rn(dup2(v.y), b01, ar[1][0]);
+                        ar[1][1] = fma2_rn(dup2(v.y), b23, ar[1][1]);
+                        ar[2][0] = fma2_rn(dup2(v.z), b01, ar[2][0]);
+                        ar[2][1] = fma2_rn(dup2(v.z), b23, ar[2][1]);
+                        ar[3][0] = fma2_rn(dup2(v.w), b01, ar[3][0]);
+                        ar[3][1] = fma2_rn(dup2(v.w), b23, ar[3][1]);
+                    }
+                }
+                float2 dm = fold_tile(am, j), dr = dm;
+                if constexpr (kFinal) dr = fold_tile(ar, j);
+                const int c = 16 * q + 4 * grp + 2 * (j & 1);  // this lane's components c, c + 1
+                if (has_tail) {
+                    // the unfused tail of each dot (dot_contiguous_highway)
+                    for (int idx = full * kLanes; idx < D; ++idx) {
+                        const float2 b = *reinterpret_cast<const float2*>(basis + idx * ldb + c);
+                        const float u = U[4 * idx + r];
+                        dm.x = __fadd_rn(dm.x, __fmul_rn(u, b.x));
+                        dm.y = __fadd_rn(dm.y, __fmul_rn(u, b.y));
+                        if constexpr (kFinal) {
+                            const float v = V[4 * idx + r];
+                            dr.x = __fadd_rn(dr.x, __fmul_rn(v, b.x));
+                            dr.y = __fadd_rn(dr.y, __fmul_rn(v, b.y));
+                        }
+                    }
+                    if constexpr (!kFinal) dr = dm;
+                }
+                sc[c * kTileRows + r] = __fmul_rn(coef[c], dr.x);
+                sc[(c + 1) * kTileRows + r] = __fmul_rn(coef[c + 1], dr.y);
+                if (membership_on) {
+                    const float p0 = __fmul_rn(dm.x, dm.x), p1 = __fmul_rn(dm.y, dm.y);
+                    *reinterpret_cast<float2*>(square + r * kComps + c) = make_float2(p0, p1);
+                    *reinterpret_cast<float2*>(quot + r * kComps + c) =
+                        make_float2(__fdiv_rn(p0, denom[c]), __fdiv_rn(p1, denom[c + 1]));
+                    if (q == 0) {
+                        // the rows' norms, folded like the dots
+                        const float x = fold_half((j & 4) ? an[1].x : an[0].x, (j & 4) ? an[0].x : an[1].x, 4);
+                        const float y = fold_half((j & 4) ? an[1].y : an[0].y, (j & 4) ? an[0].y : an[1].y, 4);
+                        float n = fold_half((j & 2) ? y : x, (j & 2) ? x : y, 2);
+                        n = __fadd_rn(n, __shfl_xor_sync(0xffffffffu, n, 1));
+                        for (int idx = full * kLanes; idx < D; ++idx) {
+                            const float u = U[4 * idx + r];
+                            n = __fadd_rn(n, __fmul_rn(u, u));
+                        }
+                        if (grp == 0 && !(j & 1)) norms[r] = n;
+                    }
+                }
+            }
+            __syncwarp();
+            // membership score of each row, components in order
+            if (lane < nrows && membership_on) {
+                const float* qr = quot + lane * kComps;
+                const float* pr = square + lane * kComps;
+                float distance = 0.0f, projected = 0.0f;
+#pragma unroll 4
+                for (int c = 0; c < R; ++c) {
+                    distance = __fadd_rn(distance, qr[c]);
+                    projected = __fadd_rn(projected, pr[c]);
+                }
+                const float resid = __fsub_rn(norms[lane], projected);
+                distance = __fadd_rn(distance, __fdiv_rn(resid > 0.0f ? resid : 0.0f, mem2));
+                scores[t0 + lane] = __fdiv_rn(__fsub_rn(distance, static_cast<float>(D)), score_scale);
+            }
+            float* out = L.filtered + static_cast<size_t>(r0 + t0) * L.row_dim + mc * D;
+            int base = 0;
+            for (; base + 128 <= full * kLanes; base += 128)
+                tile_reconstruct<4, false>(basis, ldb, coef, sc, center_vec, R, D, base, lane, out, L.row_dim, nrows);
+            for (; base + 64 <= D; base += 64)
+                tile_reconstruct<2, true>(basis, ldb, coef, sc, center_vec, R, D, base, lane, out, L.row_dim, nrows);
+            for (; base < D; base += 32)
+                tile_reconstruct<1, true>(basis, ldb, coef, sc, center_vec, R, D, base, lane, out, L.row_dim, nrows);
+            __syncwarp();
+        }
+        __syncthreads();
+        // aggregation weights (accumulate_aggregation_model + finalize)
+        const float lgw = s_misc[0];
+        const float volume = s_misc[1];
+        if (warp == 0) {
+            float mn = kInf;
+            if (membership_on)
+                for (int i = lane; i < S; i += 32) mn = std_min(mn, scores[i]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) mn = std_min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+            if (lane == 0) s_misc[2] = mn;
+        }
+        __syncthreads();
+        const float min_score = s_misc[2];
+        for (int i = tid; i < S; i += threads) {
+            const float lw0 = model_log_weight(P, membership_on, lgw, volume, scores[i], min_score);
+            if (models > 1) {
+                // this plane's term of the row's log weight; combine_weights
+                // sums the planes in order and finalises
+                L.logw[static_cast<size_t>(r0 + i) * models + mc] = lw0;
+                continue;
+            }
+            float w = 1.0f;
+            if (weights_enabled) {
+                float lw = __fadd_rn(0.0f, lw0);
                 lw = lw < -80.0f ? -80.0f : (80.0f < lw ? 80.0f : lw);
                 w = cr_expf(lw);
             }
@@ -1598,6 +1966,21 @@ cudaError_t launch_apply_warp(const FilterLaunch& L, int max_groups, cudaStream_
     return cudaGetLastError();
 }
 
+// Warps per block of the row-tile apply for this shape, 0 where the
+// row-per-warp kernel runs: no rank, ranks above 32, dimensions of 16 and less
+// (their dots have an order of their own), and shapes whose block does not fit
+// even with one warp.  Fewer warps than kTileWarps only where four do not fit
+// (dimensions of about 1500 and more), so that such shapes keep the kernel.
+int tile_apply_warps(const FilterLaunch& L) {
+    if (L.rank < 1 || L.rank > 32 || L.dim <= 16) return 0;
+    const int Bmax = std::min(L.model_cap, L.max_rows);
+    for (int warps = kTileWarps; warps >= 1; warps /= 2)
+        if (static_cast<size_t>(tile_apply_layout(L.dim, Bmax, L.rank > 16 ? 2 : 1, L.max_rows, warps, L.stage == 1)
+                                    .bytes) <= kFilterSharedLimit)
+            return warps;
+    return 0;
+}
+
 }  // namespace
 
 size_t filter_shared_bytes(const FilterLaunch& L) {
@@ -1613,8 +1996,20 @@ size_t filter_shared_bytes(const FilterLaunch& L) {
         const JacobiShape js = jacobi_shape(L.nmax);
         need = std::max(need, static_cast<size_t>(32 / js.seg) * js.gstride * sizeof(float));
     }
-    const bool tiled = R >= 1 && R <= kTileComps && D > 16;
-    need = std::max(need, apply_layout(D, Bmax, R, L.max_rows, kApplyWarps, tiled, L.stage == 1).bytes);
+    // the largest apply block.  The row tiles are sized to what is there
+    // (tile_apply_warps), so this bound is the row-per-warp block's; ranks up
+    // to 16 above dimension 16 keep the bound they have always been refused at
+    // (eight warps of two-row tiles), which does not change with the kernels
+    need = std::max(need, apply_layout(D, Bmax, R, L.max_rows, kApplyWarps).bytes);
+    if (R >= 1 && R <= 16 && D > 16) {
+        const size_t ldu = static_cast<size_t>((D + 23) & ~31) + 8;
+        const size_t tiles = kApplyWarps * ((L.stage == 1 ? 2 : 1) * 2 * ldu + 66);
+        const size_t model = static_cast<size_t>(Bmax) * (D + 1);
+        const size_t fixed = colpad + 2 * static_cast<size_t>(D) + R * ldu + static_cast<size_t>(R) * Bmax +
+                             5 * static_cast<size_t>(R) + L.max_rows;
+        need = std::max(need, (((fixed + std::max(tiles, model) + 1) & ~static_cast<size_t>(1)) +
+                               2 * static_cast<size_t>(L.max_rows)) * sizeof(float));
+    }
     return need;
 }
 
@@ -1694,17 +2089,24 @@ cudaError_t launch_filter(const FilterLaunch& L, int max_groups_in, cudaStream_t
                                      : launch_apply_warp<256>(L, max_groups, stream);
         if (err != cudaSuccess) return err;
     } else {
-        // tiled rows for rank <= kTileComps above dimension 16 (the special
-        // 8- and 16-element dot orders stay with the row-per-warp loop)
-        const bool tiled = R >= 1 && R <= kTileComps && D > 16;
-        const ApplyLayout lay = apply_layout(D, Bmax, R, L.max_rows, kApplyWarps, tiled, L.stage == 1);
-        const size_t smem = lay.bytes;
-        auto kernel = tiled ? apply_kernel<true> : apply_kernel<false>;
-        cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(kernel),
-                                               static_cast<int>(smem));
-        if (err != cudaSuccess) return err;
-        const int ctas = std::min(max_groups, 148 * 8);
-        kernel<<<ctas, kApplyThreads, smem, stream>>>(L);
+        const int tile_warps = tile_apply_warps(L);
+        cudaError_t err = cudaSuccess;
+        if (tile_warps > 0) {
+            const bool wide = R > 16, final_stage = L.stage == 1;
+            auto kernel = wide ? (final_stage ? apply_tile_kernel<2, true> : apply_tile_kernel<2, false>)
+                               : (final_stage ? apply_tile_kernel<1, true> : apply_tile_kernel<1, false>);
+            const TileApplyLayout lay = tile_apply_layout(D, Bmax, wide ? 2 : 1, L.max_rows, tile_warps, final_stage);
+            err = raise_smem_limit(reinterpret_cast<const void*>(kernel), lay.bytes);
+            if (err != cudaSuccess) return err;
+            const int ctas = std::min(max_groups, 148 * 8);
+            kernel<<<ctas, 32 * tile_warps, lay.bytes, stream>>>(L);
+        } else {
+            const ApplyLayout lay = apply_layout(D, Bmax, R, L.max_rows, kApplyWarps);
+            err = raise_smem_limit(reinterpret_cast<const void*>(apply_kernel), static_cast<int>(lay.bytes));
+            if (err != cudaSuccess) return err;
+            const int ctas = std::min(max_groups, 148 * 8);
+            apply_kernel<<<ctas, kApplyThreads, lay.bytes, stream>>>(L);
+        }
         if ((err = cudaGetLastError()) != cudaSuccess) return err;
     }
     if (L.models > 1) {
