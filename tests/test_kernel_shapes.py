@@ -38,6 +38,10 @@ APPLY_TILES = [
     ("alpha_only", 48, 40, 3, 1, dict(block_size=7, patch_time=2, group_size=12, rank=10, weight_beta=0.0)),
 ]
 
+# eigen problems on both sides of each register and lane split (8, 16, 24, 32
+# rows), with fewer rows than the matrix they are stored in
+JACOBI = [(k, r) for k, r in ((1, 1), (2, 2), (7, 7), (8, 8), (9, 4), (15, 15), (23, 23), (24, 24), (25, 25), (31, 8))]
+
 
 def check(w, h, f, planes, sigma, kw, seed):
     _, noisy = synth.make_clip(w, h, f, planes, sigma, seed=seed)
@@ -54,3 +58,8 @@ def check(w, h, f, planes, sigma, kw, seed):
 @pytest.mark.parametrize("name,w,h,f,planes,kw", APPLY_TILES, ids=[c[0] for c in APPLY_TILES])
 def test_apply_row_tiles(name, w, h, f, planes, kw):
     check(w, h, f, planes, 20.0, kw, seed=len(name))
+
+
+@pytest.mark.parametrize("k,rank", JACOBI)
+def test_jacobi_sizes(k, rank):
+    check(48, 40, 3, 1, 20.0, dict(patch_time=2, group_size=k, rank=rank, cap_factor=1.0), seed=k)

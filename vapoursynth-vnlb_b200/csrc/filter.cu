@@ -381,6 +381,30 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
     }
 }
 
+// The rotation (c, s) that zeroes apq (jacobi_rotate, linalg.cpp:152-196).
+// kMixed (chosen forms): in FP64, so that near-degenerate pairs (aqq - app
+// tiny against apq) keep their angle; t = sgn 2 apq / (|d| + sqrt(d^2 +
+// 4 apq^2)) is the same tangent with one division and two square roots.
+template <bool kMixed>
+__device__ __forceinline__ void jacobi_angle(float app, float aqq, float apq, float& c, float& s) {
+    if constexpr (kMixed) {
+        const double d = static_cast<double>(aqq) - static_cast<double>(app);
+        const double b = 2.0 * static_cast<double>(apq);
+        const double t_abs = fabs(b) / (fabs(d) + sqrt(d * d + b * b));
+        const double t = d != 0.0 && (d < 0.0) != (b < 0.0) ? -t_abs : t_abs;
+        const double cd = rsqrt(1.0 + t * t);
+        c = static_cast<float>(cd);
+        s = static_cast<float>(t * cd);
+    } else {
+        const float tau = __fdiv_rn(__fsub_rn(aqq, app), __fmul_rn(2.0f, apq));
+        const float t_abs =
+            __fdiv_rn(1.0f, __fadd_rn(fabsf(tau), __fsqrt_rn(__fadd_rn(1.0f, __fmul_rn(tau, tau)))));
+        const float t = tau < 0.0f ? -t_abs : t_abs;
+        c = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(1.0f, __fmul_rn(t, t))));
+        s = __fmul_rn(t, c);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // jacobi: topk_symmetric_eigen_jacobi (linalg.cpp:447-519) for many groups per
 // warp.  A group owns a segment of `seg` lanes (a power of two >= its rows,
@@ -445,27 +469,9 @@ __global__ void __launch_bounds__(256) jacobi_kernel(FilterLaunch L, int seg, in
                         }
                         __syncwarp();
                         if (rot) {
-                            // jacobi_rotate (linalg.cpp:152-196)
                             float c, s;
-                            if (L.mixed) {
-                                // chosen forms: the rotation angle in FP64, so that near-degenerate
-                                // pairs (aqq - app tiny against apq) keep their angle
-                                const double tau = (static_cast<double>(aqq) - static_cast<double>(app)) /
-                                                   (2.0 * static_cast<double>(apq));
-                                const double t_abs = 1.0 / (fabs(tau) + sqrt(1.0 + tau * tau));
-                                const double t = tau < 0.0 ? -t_abs : t_abs;
-                                const double cd = 1.0 / sqrt(1.0 + t * t);
-                                c = static_cast<float>(cd);
-                                s = static_cast<float>(t * cd);
-                            } else {
-                                const float tau = __fdiv_rn(__fsub_rn(aqq, app), __fmul_rn(2.0f, apq));
-                                const float tau_abs = fabsf(tau);
-                                const float t_abs = __fdiv_rn(
-                                    1.0f, __fadd_rn(tau_abs, __fsqrt_rn(__fadd_rn(1.0f, __fmul_rn(tau, tau)))));
-                                const float t = tau < 0.0f ? -t_abs : t_abs;
-                                c = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(1.0f, __fmul_rn(t, t))));
-                                s = __fmul_rn(t, c);
-                            }
+                            if (L.mixed) jacobi_angle<true>(app, aqq, apq, c, s);
+                            else jacobi_angle<false>(app, aqq, apq, c, s);
                             for (int r = r0; r < B; r += seg) {
                                 if (r != p && r != q) {
                                     const float arp = m[r * ld + p];
@@ -542,6 +548,207 @@ __global__ void __launch_bounds__(256) jacobi_kernel(FilterLaunch L, int seg, in
         }
         __syncwarp();
         (void)seg_mask;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// jacobi, kSeg lanes per group, for matrices up to N x N (N = 8 to 32).  The
+// rotations of a group are one chain of dependent divisions and square roots:
+// latency bounds it, so as many groups as fit in shared memory are in flight,
+// and few lanes repeat each angle.  Against jacobi_kernel (B200, one launch
+// alone): N = 8, 32k groups 155 -> 81 us; N = 16, 57k groups 1.08 -> 0.65 ms,
+// 0.6k groups 421 -> 218 us; with FP64 angles, 130k groups, 5.0 -> 2.85 ms.  The strict upper triangle, the diagonal and the vectors lie in
+// shared memory as [element][group].  Lane h owns rows i kSeg + h; its part of
+// row p and of vector p stays in registers while q runs over an unrolled loop,
+// and the samples a rotation will need are loaded before its angle is known.
+// For row r = p the update works on the stale copy of (p, q); the write-back of
+// row p replaces it.  Same rotations in the same order on the same values as
+// jacobi_kernel, element by element.
+constexpr size_t jacobi_small_bytes(int N, int seg) {
+    return static_cast<size_t>(N * (N - 1) / 2 + N + N * N) * (32 / seg) * sizeof(float);
+}
+
+template <int N, int kSeg, bool kMixed>
+__global__ void __launch_bounds__(32) jacobi_small_kernel(FilterLaunch L) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int kTri = N * (N - 1) / 2;
+    constexpr int kG = 32 / kSeg;  // groups per warp: lane = h * kG + group
+    constexpr int kRows = N / kSeg;
+    const int lane = threadIdx.x;
+    const int gi = lane % kG, h = lane / kG;
+    float* tri = sm + gi;            // (r, c), r < c, at tri_at(r, c)
+    float* diag = tri + kTri * kG;   // [N]
+    float* vec = diag + N * kG;      // [vector][row]
+    const auto tri_at = [](int r, int c) { return (r * (2 * N - r - 1) / 2 + c - r - 1) * kG; };
+    const int total = L.counters->active * L.models;
+    const int a = blockIdx.x * kG + gi;
+    if (blockIdx.x * kG >= total) return;
+    const int R = L.rank, D = L.dim, M = L.nmax;  // M: stride of the stored matrices and vectors
+    const bool valid = a < total && L.flags[a] == 0;
+    int B = 0;  // matrix dimension: the dual Gram's B, or the covariance's D
+    if (valid) {
+        const int Bm = min(L.row_counts[L.active[a / L.models]], L.model_cap);
+        B = (D >= 64 && Bm < D) ? Bm : D;  // use_dual_pca (core.cpp:656-658)
+    }
+    const float* gram = L.gram + static_cast<size_t>(a) * M * M;
+    float mx = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+        const int r = i * kSeg + h;
+        if (B == N && M == N) {  // rows of whole 16-byte units
+#pragma unroll
+            for (int c0 = 0; c0 < N; c0 += 4) {
+                if (c0 + 3 < i * kSeg) continue;
+                const float4 q = __ldg(reinterpret_cast<const float4*>(gram + r * N + c0));
+                const float x[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    if (c0 + k < r) continue;
+                    mx = std_max(mx, fabsf(x[k]));
+                    *(c0 + k == r ? diag + r * kG : tri + tri_at(r, c0 + k)) = x[k];
+                }
+            }
+        } else {
+            for (int c = r; c < N; ++c) {
+                const float x = r < B && c < B ? gram[r * B + c] : 0.0f;
+                mx = std_max(mx, fabsf(x));
+                *(c == r ? diag + r * kG : tri + tri_at(r, c)) = x;
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < N; ++c) vec[(c * N + r) * kG] = r == c ? 1.0f : 0.0f;
+    }
+#pragma unroll
+    for (int o = kG; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float threshold = std_max(0.0f, __fmul_rn(64.0f * FLT_EPSILON, std_max(1.0f, mx)));
+    int row_of[kRows];  // (r, c) for r < c at row_of[i] + c * kG
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) row_of[i] = tri_at(i * kSeg + h, 0);
+    __syncwarp();
+    for (int sweep = 0; sweep < 64; ++sweep) {
+        float off = 0.0f;
+#pragma unroll 8
+        for (int e = h; e < kTri; e += kSeg) off = std_max(off, fabsf(tri[e * kG]));
+#pragma unroll
+        for (int o = kG; o < 32; o <<= 1) off = fmaxf(off, __shfl_xor_sync(0xffffffffu, off, o));
+        const bool busy = B > 1 && !(off <= threshold);
+        if (!__any_sync(0xffffffffu, busy)) break;
+#pragma unroll 1
+        for (int p = 0; p + 1 < N; ++p) {
+            float ap[kRows], vp[kRows];
+            const int row_p = tri_at(p, 0);
+            float app = diag[p * kG];
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                const int r = i * kSeg + h;
+                ap[i] = r == p ? 0.0f : tri[r < p ? row_of[i] + p * kG : row_p + r * kG];
+                vp[i] = vec[(p * N + r) * kG];
+            }
+#pragma unroll
+            for (int q = 1; q < N; ++q) {
+                if (q <= p) continue;
+                const float apq = __shfl_sync(0xffffffffu, ap[q / kSeg], (q % kSeg) * kG + gi);
+                const bool rot = busy && q < B && fabsf(apq) > threshold && apq != 0.0f;
+                if (!__any_sync(0xffffffffu, rot)) continue;
+                const float aqq = diag[q * kG];
+                float* at[kRows];
+                float arq[kRows], vrq[kRows];
+#pragma unroll
+                for (int i = 0; i < kRows; ++i) {
+                    // row r against column q: above the diagonal, below it, or
+                    // (in the block of q) either, by lane; r = q reads (and
+                    // does not write) a slot of its own row
+                    const int r = i * kSeg + h;
+                    at[i] = tri + (i * kSeg + kSeg <= q  ? row_of[i] + q * kG
+                                   : i * kSeg > q         ? tri_at(q, 0) + r * kG
+                                   : r < q                ? row_of[i] + q * kG
+                                                          : tri_at(q, 0) + (r == q ? (q < N - 1 ? q + 1 : 0) : r) * kG);
+                    if (i == q / kSeg && q == N - 1 && r == q) at[i] = tri;
+                    arq[i] = *at[i];
+                    vrq[i] = vec[(q * N + r) * kG];
+                }
+                if (rot) {
+                    float c, s;
+                    jacobi_angle<kMixed>(app, aqq, apq, c, s);
+#pragma unroll
+                    for (int i = 0; i < kRows; ++i) {
+                        const bool own = i == q / kSeg && i * kSeg + h == q;
+                        const float arp = ap[i];
+                        const float nrp = __fsub_rn(__fmul_rn(c, arp), __fmul_rn(s, arq[i]));
+                        ap[i] = own ? 0.0f : nrp;
+                        if (!own) *at[i] = __fadd_rn(__fmul_rn(s, arp), __fmul_rn(c, arq[i]));
+                        const float vrp = vp[i];
+                        vp[i] = __fsub_rn(__fmul_rn(c, vrp), __fmul_rn(s, vrq[i]));
+                        vec[(q * N + i * kSeg + h) * kG] = __fadd_rn(__fmul_rn(s, vrp), __fmul_rn(c, vrq[i]));
+                    }
+                    const float cc = __fmul_rn(c, c), ss = __fmul_rn(s, s);
+                    const float cs2 = __fmul_rn(2.0f, __fmul_rn(c, s));
+                    if (h == 0)
+                        diag[q * kG] = __fadd_rn(__fadd_rn(__fmul_rn(ss, app), __fmul_rn(cs2, apq)), __fmul_rn(cc, aqq));
+                    app = __fadd_rn(__fsub_rn(__fmul_rn(cc, app), __fmul_rn(cs2, apq)), __fmul_rn(ss, aqq));
+                }
+                if constexpr (kSeg > 1) __syncwarp();
+            }
+            if (h == 0) diag[p * kG] = app;
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                const int r = i * kSeg + h;
+                if (r != p) tri[r < p ? row_of[i] + p * kG : row_p + r * kG] = ap[i];
+                vec[(p * N + r) * kG] = vp[i];
+            }
+            __syncwarp();
+        }
+    }
+    // stable sort of the diagonal (descending), canonicalised top-rank
+    // eigenvectors (canonicalize_vector_row, linalg.cpp:198-227); the sorted
+    // order goes where the triangle was
+    for (int r = h; r < B; r += kSeg) {
+        const float dr = diag[r * kG];
+        int pos = 0;
+        for (int j = 0; j < B; ++j) {
+            const float dj = diag[j * kG];
+            if (dj > dr || (j < r && !(dr > dj))) ++pos;
+        }
+        tri[pos * kG] = __int_as_float(r);
+    }
+    __syncwarp();
+    if (!valid) return;
+    float* eig = L.eig + static_cast<size_t>(a) * R;
+    float* dual = L.dual + static_cast<size_t>(a) * R * M;
+    for (int out = h; out < R; out += kSeg) {
+        const int src = __float_as_int(tri[out * kG]);
+        const float* v = vec + src * N * kG;
+        eig[out] = diag[src * kG];
+        float x[N];
+        float norm2 = 0.0f, best = 0.0f, lead = 0.0f;
+#pragma unroll
+        for (int r = 0; r < N; ++r) {
+            x[r] = 0.0f;
+            if (r < B) {
+                x[r] = v[r * kG];
+                norm2 = __fadd_rn(norm2, __fmul_rn(x[r], x[r]));
+                if (r == 0) lead = x[r];
+                if (fabsf(x[r]) > best) {
+                    best = fabsf(x[r]);
+                    lead = x[r];
+                }
+            }
+        }
+        if (!(norm2 <= FLT_MIN)) {
+            float sc = __fdiv_rn(1.0f, __fsqrt_rn(norm2));
+            if (lead < 0.0f) sc = -sc;
+#pragma unroll
+            for (int r = 0; r < N; ++r) x[r] = __fmul_rn(x[r], sc);
+        }
+        if (B == N && M == N) {
+#pragma unroll
+            for (int r = 0; r < N; r += 4)
+                *reinterpret_cast<float4*>(dual + out * N + r) = make_float4(x[r], x[r + 1], x[r + 2], x[r + 3]);
+        } else {
+#pragma unroll
+            for (int r = 0; r < N; ++r)
+                if (r < B) dual[out * M + r] = x[r];
+        }
     }
 }
 
@@ -864,10 +1071,9 @@ __global__ void __launch_bounds__(kApplyThreads, 3) apply_kernel(FilterLaunch L)
 }
 
 // ---------------------------------------------------------------------------
-// apply, row tiles: a CTA of up to kTileWarps warps per group, for ranks up to
-// 4 * 4 * kQ that the warp-per-group kernel does not take (large groups and
-// dimensions: blocks of 7 over two frames and three planes, groups of 16 grown
-// to 64 rows).
+// apply, row tiles: a CTA of up to kTileWarps warps per group, for the shapes
+// with ranks up to 16 kQ that the warp-per-group kernel does not take (blocks
+// of 7 over two frames and three planes, groups of 16 grown to 64 rows).
 //
 // Measured against one group per 8-warp CTA with two rows per warp and scalar
 // shared loads (B200, one launch alone, 57k groups of dimension 294, rank 15):
@@ -1953,6 +2159,17 @@ JacobiShape jacobi_shape(int N) {
     return JacobiShape{seg, ld, gstride};
 }
 
+template <int N, int kSeg>
+cudaError_t launch_jacobi_small(const FilterLaunch& L, int max_groups, cudaStream_t stream) {
+    auto kernel = L.mixed ? jacobi_small_kernel<N, kSeg, true> : jacobi_small_kernel<N, kSeg, false>;
+    const size_t smem = jacobi_small_bytes(N, kSeg);
+    const cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
+    if (err != cudaSuccess) return err;
+    constexpr int kGroups = 32 / kSeg;
+    kernel<<<(max_groups + kGroups - 1) / kGroups, 32, smem, stream>>>(L);
+    return cudaGetLastError();
+}
+
 template <int D>
 cudaError_t launch_apply_warp(const FilterLaunch& L, int max_groups, cudaStream_t stream) {
     const bool scatter = L.scatter != nullptr;
@@ -2054,23 +2271,37 @@ cudaError_t launch_filter(const FilterLaunch& L, int max_groups_in, cudaStream_t
     }
     // jacobi
     if (R > 0) {
-        // a segment of `seg` lanes per group, each lane owning rows r0, r0 + seg,
-        // ...; two rows per lane from 8 rows up, which halves the rotation
-        // parameters every lane recomputes
         const int N = L.nmax;  // largest matrix: model rows, or the dimension of covariance models
-        const JacobiShape js = jacobi_shape(N);
-        const int seg = js.seg, ld = js.ld, gstride = js.gstride;
-        const size_t per_group = static_cast<size_t>(gstride) * sizeof(float);
-        int warps = 8;
-        while (warps > 1 && static_cast<size_t>(warps) * (32 / seg) * per_group > 160 * 1024) warps /= 2;
-        const size_t smem = static_cast<size_t>(warps) * (32 / seg) * per_group;
-        cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(jacobi_kernel),
-                                               static_cast<int>(smem));
-        if (err != cudaSuccess) return err;
-        const int per_cta = warps * (32 / seg);
-        const int ctas = std::max(1, std::min((max_groups + per_cta - 1) / per_cta, 148 * 32));
-        jacobi_kernel<<<ctas, 32 * warps, smem, stream>>>(L, seg, ld, gstride);
-        if ((err = cudaGetLastError()) != cudaSuccess) return err;
+        if (N <= 32) {
+            // lanes per group: more lanes repeat the angle on more lanes, but
+            // leave fewer rows per lane and more warps to hide its latency
+            // (1, 2 and 4 lanes: N = 8, 32k groups 77, 81, 86 us; N = 16, 57k
+            // groups 0.95, 0.65, 0.66 ms, 0.6k groups 440, 290, 218 us, and
+            // with FP64 angles, 130k groups, 4.1, 3.55, 2.85 ms)
+            cudaError_t err;
+            if (N <= 8) err = launch_jacobi_small<8, 2>(L, max_groups, stream);
+            else if (N <= 16) err = launch_jacobi_small<16, 4>(L, max_groups, stream);
+            else if (N <= 24) err = launch_jacobi_small<24, 4>(L, max_groups, stream);
+            else err = launch_jacobi_small<32, 8>(L, max_groups, stream);
+            if (err != cudaSuccess) return err;
+        } else {
+            // a segment of `seg` lanes per group, each lane owning rows r0, r0 + seg,
+            // ...; two rows per lane from 8 rows up, which halves the rotation
+            // parameters every lane recomputes
+            const JacobiShape js = jacobi_shape(N);
+            const int seg = js.seg, ld = js.ld, gstride = js.gstride;
+            const size_t per_group = static_cast<size_t>(gstride) * sizeof(float);
+            int warps = 8;
+            while (warps > 1 && static_cast<size_t>(warps) * (32 / seg) * per_group > 160 * 1024) warps /= 2;
+            const size_t smem = static_cast<size_t>(warps) * (32 / seg) * per_group;
+            cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(jacobi_kernel),
+                                                   static_cast<int>(smem));
+            if (err != cudaSuccess) return err;
+            const int per_cta = warps * (32 / seg);
+            const int ctas = std::max(1, std::min((max_groups + per_cta - 1) / per_cta, 148 * 32));
+            jacobi_kernel<<<ctas, 32 * warps, smem, stream>>>(L, seg, ld, gstride);
+            if ((err = cudaGetLastError()) != cudaSuccess) return err;
+        }
     }
     // apply
 #ifndef VNLB_APPLY_WARP
