@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
     constexpr int kGroups = kPrepareWarps / W;  // groups per CTA
     constexpr int kT = 32 * W;                  // threads per group
     extern __shared__ __align__(16) float sm[];
-    __shared__ double s_sums[2 * 4];            // flat-area sums per channel (W > 1)
+    __shared__ double s_sums[2 * 4];            // flat-area sums per warp (W > 1)
     const int D = L.dim;
     const int Bmax = bmax_of(L);
     int* coloff = reinterpret_cast<int*>(sm);
@@ -205,9 +205,11 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
             bases[i] = row_base(L, m);
         }
         group_sync();
-        // equal group (samples_are_equal / group_is_equal): independent loads
-        bool differs = S <= 1;
-        if (S > 1) {
+        // equal group (samples_are_equal / group_is_equal): the first two rows
+        // differ in the first columns of nearly every group, which settles it
+        bool differs = S <= 1 || (t < D && __ldg(L.noisy + bases[0] + coloff[t]) !=
+                                               __ldg(L.noisy + bases[1] + coloff[t]));
+        if (!group_any(differs)) {
             for (int col = t; col < D * models; col += kT) {
                 const int cm = col / D;  // plane of an uncoupled group (group_is_equal, core.cpp:516-531)
                 const float* src = L.noisy + cm * hw + coloff[col - cm * D];
@@ -220,6 +222,8 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
                 }
                 for (; i < S; ++i) differs |= __ldg(src + bases[i]) != v0;
             }
+        } else {
+            differs = true;
         }
         if (!group_any(differs)) {
             // filtered = input, default aggregation model (core.cpp:253-274)
@@ -241,24 +245,29 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
             if (t == 0) L.flags[v] = kGroupDone;
             continue;
         }
-        // flat area (Final): mean channel variance of the noisy rows; one warp
-        // sums a channel (lane-strided, then a fixed shuffle tree)
+        // flat area (Final): mean channel variance of the noisy rows, in
+        // double.  The warps of the group share a channel's rows; a lane sums
+        // its columns of kFlatRows rows at a time (their loads in flight
+        // together), then a fixed shuffle tree and the warps in order
         bool flat = false;
         if (final_stage && P.flat_areas) {
+            constexpr int kFlatRows = 4;
             const int pd = L.patch_dim;
             const int channels = models > 1 ? models : D / pd;
             const int per_channel = pd * S;
             float variance = 0.0f;
-            for (int c0 = 0; c0 < channels; c0 += W) {
-                const int c = c0 + gwarp;
+            for (int c = 0; c < channels; ++c) {
                 double sum = 0.0, sum2 = 0.0;
-                if (c < channels) {
-                    for (int i = 0; i < S; ++i) {
-                        const float* src = L.noisy + bases[i];
-                        for (int q = lane; q < pd; q += 32) {
-                            const float x = __ldg(src + (models > 1 ? c * hw + coloff[q] : coloff[c * pd + q]));
-                            sum += static_cast<double>(x);
-                            sum2 += static_cast<double>(x) * static_cast<double>(x);
+                for (int q = lane; q < pd; q += 32) {
+                    const float* src = L.noisy + (models > 1 ? c * hw + coloff[q] : coloff[c * pd + q]);
+                    for (int i0 = gwarp * kFlatRows; i0 < S; i0 += W * kFlatRows) {
+                        float x[kFlatRows];
+#pragma unroll
+                        for (int k = 0; k < kFlatRows; ++k) x[k] = i0 + k < S ? __ldg(src + bases[i0 + k]) : 0.0f;
+#pragma unroll
+                        for (int k = 0; k < kFlatRows; ++k) {
+                            sum += static_cast<double>(x[k]);
+                            sum2 += static_cast<double>(x[k]) * static_cast<double>(x[k]);
                         }
                     }
                 }
@@ -268,25 +277,22 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
                     sum2 += __shfl_xor_sync(0xffffffffu, sum2, o);
                 }
                 if constexpr (W > 1) {
-                    if (lane == 0 && c < channels) {
+                    if (lane == 0) {
                         s_sums[2 * gwarp] = sum;
                         s_sums[2 * gwarp + 1] = sum2;
                     }
                     group_sync();
-                }
-                // the channels of this round in order
-                for (int k = 0; k < W && c0 + k < channels; ++k) {
-                    double ks = sum, ks2 = sum2;
-                    if constexpr (W > 1) {
-                        ks = s_sums[2 * k];
-                        ks2 = s_sums[2 * k + 1];
+                    sum = sum2 = 0.0;
+                    for (int k = 0; k < W; ++k) {
+                        sum += s_sums[2 * k];
+                        sum2 += s_sums[2 * k + 1];
                     }
-                    if (per_channel > 1) {
-                        const double count = static_cast<double>(per_channel);
-                        variance = __fadd_rn(variance, static_cast<float>((ks2 - (ks * ks / count)) / (count - 1.0)));
-                    }
+                    group_sync();
                 }
-                if constexpr (W > 1) group_sync();
+                if (per_channel > 1) {
+                    const double count = static_cast<double>(per_channel);
+                    variance = __fadd_rn(variance, static_cast<float>((sum2 - (sum * sum / count)) / (count - 1.0)));
+                }
             }
             if (per_channel > 1) variance = __fdiv_rn(variance, static_cast<float>(channels));
             flat = variance < __fmul_rn(__fmul_rn(P.sigma, P.sigma), P.gamma);
@@ -298,34 +304,29 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
             }
             continue;
         }
-        // model rows, means over the first B rows (compute_mean), centring
-        if constexpr (W == 1) {
-            for (int s2 = 0; s2 < B; ++s2) {
-                const size_t b = bases[s2];
-                for (int col = lane; col < D; col += 32) X[s2 * ldx + col] = __ldg(model_video + b + cb + coloff[col]);
-            }
-        } else {
-            for (int e = t; e < B * D; e += kT) {
-                const int s2 = e / D;
-                const int col = e - s2 * D;
-                X[s2 * ldx + col] = __ldg(model_video + bases[s2] + cb + coloff[col]);
-            }
-        }
-        group_sync();
+        // model rows, means over the first B rows (compute_mean), centring: a
+        // thread owns a column, whose rows' loads are in flight together
         const float inv_b = __fdiv_rn(1.0f, static_cast<float>(B));
         float* means = L.means + static_cast<size_t>(v) * 2 * D;
         for (int col = t; col < D; col += kT) {
+            const float* src = model_video + cb + coloff[col];
+#pragma unroll 8
+            for (int s2 = 0; s2 < B; ++s2) X[s2 * ldx + col] = __ldg(src + bases[s2]);
             float mm = 0.0f;
+#pragma unroll 8
             for (int s2 = 0; s2 < B; ++s2) mm = __fadd_rn(mm, X[s2 * ldx + col]);
             mm = __fmul_rn(mm, inv_b);
             float center = mm;  // Basic: noisy mean; Final flat: basic mean
             if (final_stage && !flat) {
+                const float* noisy = L.noisy + cb + coloff[col];
                 float mn = 0.0f;
-                for (int s2 = 0; s2 < B; ++s2) mn = __fadd_rn(mn, __ldg(L.noisy + bases[s2] + cb + coloff[col]));
+#pragma unroll 8
+                for (int s2 = 0; s2 < B; ++s2) mn = __fadd_rn(mn, __ldg(noisy + bases[s2]));
                 center = __fmul_rn(mn, inv_b);
             }
             means[col] = mm;
             means[D + col] = center;
+#pragma unroll 8
             for (int s2 = 0; s2 < B; ++s2) X[s2 * ldx + col] = __fsub_rn(X[s2 * ldx + col], mm);
         }
         group_sync();
