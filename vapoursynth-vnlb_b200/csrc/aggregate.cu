@@ -7,13 +7,14 @@
 // 966-1045) sums the stacks of the contributing anchor frames in anchor order
 // and divides.
 //
-// Owner-computes tiles instead of atomics: a CTA owns one (tile, slot) of the
-// anchor frame's stack.  It finds the groups whose matches can reach the tile
-// (anchors within the search reach, a contiguous range of the raster-ordered
-// active list), collects the rows whose patch covers the tile in increasing
-// global row order (= CPU order), and every thread applies them to its pixels
-// in that order.  The result is bit-identical to the CPU's sequential
-// accumulation, needs no clear, and writes every stack value exactly once.
+// Owner-computes tiles instead of atomics: a CTA owns one tile of up to four
+// slots of the anchor frame's stack.  It finds the groups whose matches can
+// reach the tile (anchors within the search reach, a contiguous range of the
+// raster-ordered active list), collects the rows whose patch covers the tile
+// in increasing global row order (= CPU order), and every thread applies them
+// to its pixel in that order.  The result is bit-identical to the CPU's
+// sequential accumulation, needs no clear, and writes every stack value
+// exactly once.
 #include "vnlb_kernels.h"
 
 namespace vnlbgpu {
@@ -21,44 +22,117 @@ namespace {
 
 constexpr int kTileThreads = kTile * kTile;
 constexpr int kTileWarps = kTileThreads / 32;
-constexpr int kMaxGridRows = 64;  // grid rows per collection round
+constexpr int kMaxGridRows = 64;   // grid rows per collection round
+constexpr int kTileSlots = 4;      // slots per CTA
+constexpr int kTileEntries = 512;  // collected rows held before they are applied
+constexpr int kTileBatch = 4;      // rows whose samples a warp has in flight
 
-struct Entry {
+struct __align__(16) Entry {
     int r;     // global row
-    int xyt;   // x | y << 14 | layer (tile_kernel) or slot (tile_slots_kernel) << 28
+    int xy;    // x | y << 16
     float w;   // row weight
+    int slot;  // slot of the row's first layer, relative to the CTA's first slot
 };
 
-// One CTA per (16x16 tile, slot), one pixel per thread.  The rows that can
-// cover the tile form one contiguous row range per grid row in reach (reach
-// tables, built per grid); their concatenation is in increasing global row
-// order.  All threads test 256 rows at a time, an ordered block compaction
-// keeps the covering ones in that order, and every thread applies them to
-// its pixel before the next chunk: the CPU's accumulation order, with no
-// atomics and one write per stack value.
+// One CTA per (16x16 tile, four slots), one pixel per thread, 8 x 4 pixels
+// per warp.  The rows that can cover the tile form one contiguous row range
+// per grid row in reach (reach tables, built per grid); their concatenation is
+// in increasing global row order.  All threads test 256 rows at a time, an
+// ordered block compaction appends the covering ones to a list, and when the
+// list could overflow (or the rows end) every warp applies it: per 32 entries
+// and slot a ballot picks the rows whose patch touches the warp's 8 x 4 pixels
+// (8 x 8 patches: a third of the tile's; visiting all of them on every thread
+// left 7 of 8 lanes idle), and the samples of kTileBatch rows are loaded
+// before the first is added.  The additions are the CPU's accumulation order.
+// Bound by the latency of the scattered sample loads; one row at a time took
+// 305 us at 1920x1080 YUV (8 rows per group), 1.15 ms at 960x540 YUV (groups
+// of 16, patch_time 2); this takes 212 us and 0.67 ms.
+template <int kChannels>
 __global__ void __launch_bounds__(kTileThreads) tile_kernel(TileLaunch L) {
-    __shared__ Entry entries[kTileThreads];
+    __shared__ Entry entries[kTileEntries];
     __shared__ int s_rbeg[kMaxGridRows];
     __shared__ int s_rpre[kMaxGridRows + 1];
-    __shared__ int s_warp[kTileWarps + 1];
+    __shared__ int s_warp[2][kTileWarps];
     extern __shared__ float window[];
 
-    const int tx = blockIdx.x, ty = blockIdx.y, slot = blockIdx.z;
+    const int tx = blockIdx.x, ty = blockIdx.y;
     const int tx0 = tx * kTile, ty0 = ty * kTile;
+    const int first_slot = blockIdx.z * kTileSlots;
+    const int slots = min(kTileSlots, L.slots - first_slot);
     const int P = L.P;
-    const int C = L.channels;
+    const int Pt = L.Pt;
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
     for (int i = tid; i < P * P; i += blockDim.x) window[i] = L.window[i];
 
-    const int px = tx0 + (tid % kTile);
-    const int py = ty0 + (tid / kTile);
-    float num[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    float wt = 0.0f;
+    const int wx = tx0 + 8 * (warp & 1), wy = ty0 + 4 * (warp >> 1);  // the warp's pixels
+    const int px = wx + (lane & 7);
+    const int py = wy + (lane >> 3);
+    float num[kTileSlots][kChannels];
+    float wt[kTileSlots];
+#pragma unroll
+    for (int s = 0; s < kTileSlots; ++s) {
+        wt[s] = 0.0f;
+#pragma unroll
+        for (int c = 0; c < kChannels; ++c) num[s][c] = 0.0f;
+    }
     const int fused_cols = (P == kLanes || P == 2 * kLanes) ? P : (P / kLanes) * kLanes;
+    const bool unfused_window = !L.coupled || L.windowed;
     const int2 grid_rows = L.tile_grid_rows[ty];
+    const int slot_base = L.search_bwd - L.anchor_frame - first_slot;  // slot = frame + slot_base
 
+    const auto apply = [&](int count) {
+        for (int e0 = 0; e0 < count; e0 += 32) {
+            bool touches = false;
+            int slot0 = 0;
+            if (e0 + lane < count) {
+                const Entry en = entries[e0 + lane];
+                const int x = en.xy & 0xffff, y = en.xy >> 16;
+                touches = x < wx + 8 && x + P > wx && y < wy + 4 && y + P > wy;
+                slot0 = en.slot;
+            }
+            if (!__any_sync(0xffffffffu, touches)) continue;
+#pragma unroll
+            for (int s = 0; s < kTileSlots; ++s) {
+                if (s >= slots) break;
+                unsigned mask = __ballot_sync(0xffffffffu, touches && slot0 <= s && s < slot0 + Pt);
+                while (mask) {
+                    float val[kTileBatch][kChannels], w[kTileBatch];
+                    bool fused[kTileBatch], inside[kTileBatch];
+#pragma unroll
+                    for (int k = 0; k < kTileBatch; ++k) {
+                        inside[k] = false;
+                        if (!mask) continue;
+                        const Entry en = entries[e0 + __ffs(mask) - 1];
+                        mask &= mask - 1;
+                        const unsigned dx = static_cast<unsigned>(px - (en.xy & 0xffff));
+                        const unsigned dy = static_cast<unsigned>(py - (en.xy >> 16));
+                        inside[k] = dx < static_cast<unsigned>(P) && dy < static_cast<unsigned>(P);
+                        if (!inside[k]) continue;
+                        const int at = static_cast<int>(dy) * P + static_cast<int>(dx);
+                        const float* f = L.filtered + static_cast<size_t>(en.r) * L.dim + (s - en.slot) * P * P + at;
+#pragma unroll
+                        for (int c = 0; c < kChannels; ++c) val[k][c] = __ldg(f + c * L.patch_dim);
+                        fused[k] = !unfused_window && static_cast<int>(dx) < fused_cols;
+                        w[k] = unfused_window ? __fmul_rn(en.w, window[at]) : en.w;
+                    }
+#pragma unroll
+                    for (int k = 0; k < kTileBatch; ++k) {
+                        if (!inside[k]) continue;
+#pragma unroll
+                        for (int c = 0; c < kChannels; ++c)
+                            num[s][c] = fused[k] ? __fmaf_rn(w[k], val[k][c], num[s][c])
+                                                 : __fadd_rn(num[s][c], __fmul_rn(w[k], val[k][c]));
+                        wt[s] = __fadd_rn(wt[s], w[k]);
+                    }
+                }
+            }
+        }
+    };
+
+    int held = 0;  // entries collected and not applied (uniform)
+    int parity = 0;
     for (int k0 = grid_rows.x; k0 < grid_rows.y; k0 += kMaxGridRows) {
         const int nk = min(kMaxGridRows, grid_rows.y - k0);
         __syncthreads();
@@ -70,9 +144,21 @@ __global__ void __launch_bounds__(kTileThreads) tile_kernel(TileLaunch L) {
             s_rpre[tid + 1] = re - rb;
         }
         __syncthreads();
-        if (tid == 0) {
-            s_rpre[0] = 0;
-            for (int k = 1; k <= nk; ++k) s_rpre[k] += s_rpre[k - 1];
+        if (warp == 0) {
+            // inclusive prefix of the two halves of the 64 row ranges
+            int a = lane < nk ? s_rpre[lane + 1] : 0, b = lane + 32 < nk ? s_rpre[lane + 33] : 0;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int va = __shfl_up_sync(0xffffffffu, a, o), vb = __shfl_up_sync(0xffffffffu, b, o);
+                if (lane >= o) {
+                    a += va;
+                    b += vb;
+                }
+            }
+            b += __shfl_sync(0xffffffffu, a, 31);
+            s_rpre[lane + 1] = a;
+            s_rpre[lane + 33] = b;
+            if (lane == 0) s_rpre[0] = 0;
         }
         __syncthreads();
         const int total = s_rpre[nk];
@@ -80,7 +166,7 @@ __global__ void __launch_bounds__(kTileThreads) tile_kernel(TileLaunch L) {
             // test one virtual row per thread
             const int vrow = chunk + tid;
             bool hit = false;
-            Entry en;
+            Entry en{};
             if (vrow < total) {
                 int lo = 0, hi = nk - 1;  // last k with s_rpre[k] <= vrow
                 while (lo < hi) {
@@ -91,219 +177,53 @@ __global__ void __launch_bounds__(kTileThreads) tile_kernel(TileLaunch L) {
                 const int r = s_rbeg[lo] + (vrow - s_rpre[lo]);
                 const MatchRow m = L.row_info[r];
                 if (m.x <= tx0 + kTile - 1 && m.x + P - 1 >= tx0 && m.y <= ty0 + kTile - 1 && m.y + P - 1 >= ty0) {
-                    const int t = slot - L.search_bwd + L.anchor_frame - m.frame;
-                    if (t >= 0 && t < L.Pt) {
-                        hit = true;
-                        en.r = r;
-                        en.xyt = m.x | (m.y << 14) | (t << 28);
-                        en.w = L.weights[r];
-                    }
-                }
-            }
-            // ordered block compaction
-            const unsigned ballot = __ballot_sync(0xffffffffu, hit);
-            if (lane == 0) s_warp[warp + 1] = __popc(ballot);
-            __syncthreads();
-            if (tid == 0) {
-                s_warp[0] = 0;
-                for (int w = 1; w <= kTileWarps; ++w) s_warp[w] += s_warp[w - 1];
-            }
-            __syncthreads();
-            if (hit) entries[s_warp[warp] + __popc(ballot & ((1u << lane) - 1u))] = en;
-            const int n = s_warp[kTileWarps];
-            __syncthreads();
-            // apply, in order, to this thread's pixel
-            for (int e = 0; e < n; ++e) {
-                const Entry x = entries[e];
-                const unsigned dx = static_cast<unsigned>(px - (x.xyt & 0x3fff));
-                const unsigned dy = static_cast<unsigned>(py - ((x.xyt >> 14) & 0x3fff));
-                if (dx >= static_cast<unsigned>(P) || dy >= static_cast<unsigned>(P)) continue;
-                const int t = x.xyt >> 28;
-                const int pos = (t * P + static_cast<int>(dy)) * P + static_cast<int>(dx);
-                const float* f = L.filtered + static_cast<size_t>(x.r) * L.dim + pos;
-                if (L.coupled && !L.windowed) {
-                    const bool fused = static_cast<int>(dx) < fused_cols;
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (c >= C) break;
-                        const float v = __ldg(f + c * L.patch_dim);
-                        num[c] = fused ? __fmaf_rn(x.w, v, num[c]) : __fadd_rn(num[c], __fmul_rn(x.w, v));
-                    }
-                    wt = __fadd_rn(wt, x.w);
-                } else {
-                    const float cw = __fmul_rn(x.w, window[dy * P + dx]);
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        if (c >= C) break;
-                        const float v = __ldg(f + c * L.patch_dim);
-                        num[c] = __fadd_rn(num[c], __fmul_rn(cw, v));
-                    }
-                    wt = __fadd_rn(wt, cw);
-                }
-            }
-            __syncthreads();
-        }
-    }
-    // write this slot's tile: every pixel, so the stack needs no clearing
-    if (px < L.width && py < L.height) {
-        const size_t plane = static_cast<size_t>(L.width) * L.height;
-        float* base = L.stack + static_cast<size_t>(slot) * (C + 1) * plane + static_cast<size_t>(py) * L.width + px;
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-            if (c < C) base[c * plane] = num[c];
-        base[C * plane] = wt;
-    }
-}
-
-// All slots in one scan: a covering row's temporal layer t lands in slot
-// s0 + t, s0 its frame's offset in the window, so one CTA per tile scans the
-// candidate rows once for all slots (at most kMaxTileSlots) and keeps one
-// accumulator set per slot.  Each (pixel, slot) still sees its rows in
-// increasing global row order: the same sums as tile_kernel.  kLayers: the
-// patch spans more than one frame (patch_time > 1).
-constexpr int kMaxTileSlots = 4;
-
-template <bool kLayers>
-__global__ void __launch_bounds__(kTileThreads) tile_slots_kernel(TileLaunch L) {
-    __shared__ Entry entries[kTileThreads];
-    __shared__ int s_rbeg[kMaxGridRows];
-    __shared__ int s_rpre[kMaxGridRows + 1];
-    __shared__ int s_warp[kTileWarps + 1];
-    extern __shared__ float window[];
-
-    const int tx = blockIdx.x, ty = blockIdx.y;
-    const int tx0 = tx * kTile, ty0 = ty * kTile;
-    const int P = L.P;
-    const int C = L.channels;
-    const int tid = threadIdx.x;
-    const int warp = tid >> 5;
-    const int lane = tid & 31;
-    for (int i = tid; i < P * P; i += blockDim.x) window[i] = L.window[i];
-
-    const int px = tx0 + (tid % kTile);
-    const int py = ty0 + (tid / kTile);
-    float num[kMaxTileSlots][4];
-    float wt[kMaxTileSlots];
-#pragma unroll
-    for (int s = 0; s < kMaxTileSlots; ++s) {
-        wt[s] = 0.0f;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) num[s][c] = 0.0f;
-    }
-    const int fused_cols = (P == kLanes || P == 2 * kLanes) ? P : (P / kLanes) * kLanes;
-    const int2 grid_rows = L.tile_grid_rows[ty];
-    const int slot_base = L.search_bwd - L.anchor_frame;  // slot = frame + slot_base
-
-    for (int k0 = grid_rows.x; k0 < grid_rows.y; k0 += kMaxGridRows) {
-        const int nk = min(kMaxGridRows, grid_rows.y - k0);
-        __syncthreads();
-        if (tid < nk) {
-            const int2 anchors = L.tile_anchors[static_cast<size_t>(k0 + tid) * L.tiles_x + tx];
-            const int rb = L.row_offset[L.active_prefix[anchors.x]];
-            const int re = L.row_offset[L.active_prefix[anchors.y]];
-            s_rbeg[tid] = rb;
-            s_rpre[tid + 1] = re - rb;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            s_rpre[0] = 0;
-            for (int k = 1; k <= nk; ++k) s_rpre[k] += s_rpre[k - 1];
-        }
-        __syncthreads();
-        const int total = s_rpre[nk];
-        for (int chunk = 0; chunk < total; chunk += kTileThreads) {
-            const int vrow = chunk + tid;
-            bool hit = false;
-            Entry en;
-            if (vrow < total) {
-                int lo = 0, hi = nk - 1;  // last k with s_rpre[k] <= vrow
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (s_rpre[mid] <= vrow) lo = mid;
-                    else hi = mid - 1;
-                }
-                const int r = s_rbeg[lo] + (vrow - s_rpre[lo]);
-                const MatchRow m = L.row_info[r];
-                if (m.x <= tx0 + kTile - 1 && m.x + P - 1 >= tx0 && m.y <= ty0 + kTile - 1 && m.y + P - 1 >= ty0) {
-                    // slot of layer 0; with several layers it may lie before the
-                    // window (the temporal windows shift at the clip's ends)
-                    // while a later layer lands in it, so it is stored + 8
+                    // the temporal windows shift at the clip's ends: a row's
+                    // first layers may lie before the slots while a later one
+                    // lands in them
                     const int slot = m.frame + slot_base;
-                    if (slot >= (kLayers ? 1 - L.Pt : 0) && slot < L.slots) {
+                    if (slot > -Pt && slot < slots) {
                         hit = true;
                         en.r = r;
-                        en.xyt = static_cast<int>(static_cast<unsigned>(m.x) | (static_cast<unsigned>(m.y) << 14) |
-                                                  (static_cast<unsigned>(kLayers ? slot + 8 : slot) << 28));
+                        en.xy = m.x | (m.y << 16);
                         en.w = L.weights[r];
+                        en.slot = slot;
                     }
                 }
             }
+            // ordered append
             const unsigned ballot = __ballot_sync(0xffffffffu, hit);
-            if (lane == 0) s_warp[warp + 1] = __popc(ballot);
+            if (lane == 0) s_warp[parity][warp] = __popc(ballot);
             __syncthreads();
-            if (tid == 0) {
-                s_warp[0] = 0;
-                for (int w = 1; w <= kTileWarps; ++w) s_warp[w] += s_warp[w - 1];
+            int at = held;
+#pragma unroll
+            for (int w = 0; w < kTileWarps; ++w) {
+                const int n = s_warp[parity][w];
+                if (w < warp) at += n;
+                held += n;
             }
-            __syncthreads();
-            if (hit) entries[s_warp[warp] + __popc(ballot & ((1u << lane) - 1u))] = en;
-            const int n = s_warp[kTileWarps];
-            __syncthreads();
-            for (int e = 0; e < n; ++e) {
-                const Entry x = entries[e];
-                const unsigned dx = static_cast<unsigned>(px - (x.xyt & 0x3fff));
-                const unsigned dy = static_cast<unsigned>(py - ((x.xyt >> 14) & 0x3fff));
-                if (dx >= static_cast<unsigned>(P) || dy >= static_cast<unsigned>(P)) continue;
-                const int slot0 = static_cast<int>(static_cast<unsigned>(x.xyt) >> 28) - (kLayers ? 8 : 0);
-                const int t_end = kLayers ? min(L.Pt, L.slots - slot0) : 1;
-                for (int t = kLayers ? max(0, -slot0) : 0; t < t_end; ++t) {
-                    const int slot = slot0 + t;
-                    const int pos = (t * P + static_cast<int>(dy)) * P + static_cast<int>(dx);
-                    const float* f = L.filtered + static_cast<size_t>(x.r) * L.dim + pos;
-                    float val[4];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) val[c] = c < C ? __ldg(f + c * L.patch_dim) : 0.0f;
-                    if (L.coupled && !L.windowed) {
-                        const bool fused = static_cast<int>(dx) < fused_cols;
-#pragma unroll
-                        for (int s = 0; s < kMaxTileSlots; ++s) {
-                            if (s != slot) continue;
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) {
-                                if (c >= C) break;
-                                num[s][c] = fused ? __fmaf_rn(x.w, val[c], num[s][c])
-                                                  : __fadd_rn(num[s][c], __fmul_rn(x.w, val[c]));
-                            }
-                            wt[s] = __fadd_rn(wt[s], x.w);
-                        }
-                    } else {
-                        const float cw = __fmul_rn(x.w, window[dy * P + dx]);
-#pragma unroll
-                        for (int s = 0; s < kMaxTileSlots; ++s) {
-                            if (s != slot) continue;
-#pragma unroll
-                            for (int c = 0; c < 4; ++c) {
-                                if (c >= C) break;
-                                num[s][c] = __fadd_rn(num[s][c], __fmul_rn(cw, val[c]));
-                            }
-                            wt[s] = __fadd_rn(wt[s], cw);
-                        }
-                    }
-                }
+            parity ^= 1;
+            if (hit) entries[at + __popc(ballot & ((1u << lane) - 1u))] = en;
+            if (held > kTileEntries - kTileThreads) {
+                __syncthreads();
+                apply(held);
+                __syncthreads();
+                held = 0;
             }
-            __syncthreads();
         }
     }
+    __syncthreads();
+    apply(held);
+    // every pixel, so the stack needs no clearing
     if (px < L.width && py < L.height) {
         const size_t plane = static_cast<size_t>(L.width) * L.height;
 #pragma unroll
-        for (int s = 0; s < kMaxTileSlots; ++s) {
-            if (s >= L.slots) break;
-            float* base = L.stack + static_cast<size_t>(s) * (C + 1) * plane + static_cast<size_t>(py) * L.width + px;
+        for (int s = 0; s < kTileSlots; ++s) {
+            if (s >= slots) break;
+            float* base = L.stack + static_cast<size_t>(first_slot + s) * (kChannels + 1) * plane +
+                          static_cast<size_t>(py) * L.width + px;
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (c < C) base[c * plane] = num[s][c];
-            base[C * plane] = wt[s];
+            for (int c = 0; c < kChannels; ++c) base[c * plane] = num[s][c];
+            base[kChannels * plane] = wt[s];
         }
     }
 }
@@ -415,15 +335,12 @@ cudaError_t launch_aggregate_stacks(const AggregateLaunch& L, cudaStream_t strea
 }
 
 cudaError_t launch_tiles(const TileLaunch& L, cudaStream_t stream) {
-    if (L.channels > 4 || L.width >= (1 << 14) || L.height >= (1 << 14) || L.Pt > 7) return cudaErrorInvalidValue;
+    if ((L.channels != 1 && L.channels != 3) || L.width >= (1 << 14) || L.height >= (1 << 14) || L.Pt > 7)
+        return cudaErrorInvalidValue;
     const size_t smem = static_cast<size_t>(L.P) * L.P * sizeof(float);
-    if (L.slots <= kMaxTileSlots) {
-        if (L.Pt == 1) tile_slots_kernel<false><<<dim3(L.tiles_x, L.tiles_y, 1), kTileThreads, smem, stream>>>(L);
-        else tile_slots_kernel<true><<<dim3(L.tiles_x, L.tiles_y, 1), kTileThreads, smem, stream>>>(L);
-    } else {
-        const dim3 grid(L.tiles_x, L.tiles_y, L.slots);
-        tile_kernel<<<grid, kTileThreads, smem, stream>>>(L);
-    }
+    const dim3 grid(L.tiles_x, L.tiles_y, (L.slots + kTileSlots - 1) / kTileSlots);
+    if (L.channels == 1) tile_kernel<1><<<grid, kTileThreads, smem, stream>>>(L);
+    else tile_kernel<3><<<grid, kTileThreads, smem, stream>>>(L);
     return cudaGetLastError();
 }
 
