@@ -53,6 +53,7 @@ struct vnlbgpu_mlp {
     float* logits = nullptr;
     float* loss = nullptr;
     int* status = nullptr;  // the inference kernels' status word
+    float* workspace = nullptr;  // partial products of the backward GEMMs' splits
 
     int fan_in(int l) const { return l == 0 ? inputs : hidden; }
     int fan_out(int l) const { return l == layers ? outputs : hidden; }
@@ -77,6 +78,7 @@ struct vnlbgpu_mlp {
         if (logits) cudaFree(logits);
         if (loss) cudaFree(loss);
         if (status) cudaFree(status);
+        if (workspace) cudaFree(workspace);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -89,7 +91,8 @@ struct vnlbgpu_mlp {
     float gradients(const float* x, const int* targets, int batch, int tk) {
         check_batch(batch);
         vnlbgpu::check(vnlbgpu::mlp_forward(net, x, batch, acts, logits, stream), "MLP forward");
-        vnlbgpu::check(vnlbgpu::mlp_backward(net, x, batch, acts, logits, targets, tk, loss, dacts, gw, gb, stream),
+        vnlbgpu::check(vnlbgpu::mlp_backward(net, x, batch, acts, logits, targets, tk, loss, dacts, gw, gb,
+                                              workspace, stream),
                        "MLP backward");
         std::vector<float> l(static_cast<size_t>(batch));
         vnlbgpu::check(cudaMemcpyAsync(l.data(), loss, l.size() * sizeof(float), cudaMemcpyDeviceToHost, stream),
@@ -172,6 +175,7 @@ int vnlbgpu_mlp_create(int inputs, int hidden, int layers, int outputs, int max_
         }
         m->logits = vnlbgpu::device_alloc<float>(static_cast<size_t>(max_batch) * outputs, "cudaMalloc(MLP logits)");
         m->status = vnlbgpu::device_alloc<int>(1, "cudaMalloc(MLP status)");
+        m->workspace = vnlbgpu::device_alloc<float>(vnlbgpu::mlp_workspace_floats(), "cudaMalloc(MLP workspace)");
         vnlbgpu::check(cudaMemset(m->status, 0, sizeof(int)), "cudaMemset(MLP status)");
         m->loss = vnlbgpu::device_alloc<float>(static_cast<size_t>(max_batch), "cudaMalloc(MLP loss)");
         vnlbgpu::check(cudaStreamSynchronize(m->stream), "cudaStreamSynchronize(MLP)");
