@@ -14,6 +14,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -39,7 +40,6 @@ def build(verbose: bool = False, ptxas_info: bool = False, out: Path | None = No
     lib = Path(out) if out else LIB
     lib.parent.mkdir(parents=True, exist_ok=True)
     LIB_DIR.mkdir(exist_ok=True)
-    objs = []
     common = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--fmad=false", "-Xcompiler", "-fPIC,-ffp-contract=off",
                      "-I", str(PKG.parent / "include")]
     if ptxas_info:
@@ -47,7 +47,8 @@ def build(verbose: bool = False, ptxas_info: bool = False, out: Path | None = No
     common += [f"-D{d}" for d in defines]
     build_dir = PKG / "_build" / ("variant_" + lib.stem if out else "default")
     build_dir.mkdir(parents=True, exist_ok=True)
-    for src in SOURCES:
+
+    def compile_one(src: str) -> str:
         obj = build_dir / (Path(src).stem + ".o")
         cmd = [nvcc(), "-c", str(CSRC / src), "-o", str(obj)] + common
         if src.endswith(".cpp"):
@@ -55,7 +56,11 @@ def build(verbose: bool = False, ptxas_info: bool = False, out: Path | None = No
         if verbose:
             print(" ".join(cmd), flush=True)
         subprocess.run(cmd, check=True)
-        objs.append(str(obj))
+        return str(obj)
+
+    # the matcher's and the filter's kernels take most of the time: sources compile side by side
+    with ThreadPoolExecutor(min(len(SOURCES), os.cpu_count() or 1)) as pool:
+        objs = list(pool.map(compile_one, SOURCES))
     cmd = [nvcc(), "-shared", "-o", str(lib)] + ARCH + [*objs, "-cudart", "static"]
     subprocess.run(cmd, check=True)
     return lib

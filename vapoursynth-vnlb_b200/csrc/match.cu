@@ -22,6 +22,8 @@
 // Outputs per anchor g: the retained rows in the CPU's row order (the order
 // std::partial_sort leaves them in), their count, and the later grid anchors
 // whose paste-mask position one of its anchor-frame matches clears.
+#include <type_traits>
+
 #include "vnlb_kernels.h"
 
 namespace vnlbgpu {
@@ -123,51 +125,73 @@ __device__ void partial_sort_pairs(float* d, int* id, int middle, int last) {
 }
 
 
-// Distances of one lane task (candidate column cx_rel, rows gy*KY .. +KY-1)
-// against the warp's reference patch, for every plane of scheduled frame k.
-// Planes in shared memory are ordered (channel, t); region row stride `rs`.
+// Row stride of the reference patch in shared memory: whole 16-byte units, so
+// that a warp reads a row with one broadcast load per four samples.
+__host__ __device__ constexpr int ref_stride(int P) { return (P + 3) & ~3; }
+
+// Distance plus the SSD of one patch row held in registers.
+template <int P>
+__device__ __forceinline__ float add_row_ssd(float d, const float (&ref)[ref_stride(P)], const float (&cand)[P]) {
+    if constexpr (P >= kLanes && P < 2 * kLanes) {
+        // one full chunk of 8 (packed pairs: the same bits in half the
+        // instructions), then the unfused tail
+        float2 a[kLanes / 2], b[kLanes / 2];
+#pragma unroll
+        for (int i = 0; i < kLanes / 2; ++i) {
+            a[i] = make_float2(ref[2 * i], ref[2 * i + 1]);
+            b[i] = make_float2(cand[2 * i], cand[2 * i + 1]);
+        }
+        d = row_ssd8_x2(d, a, b);
+#pragma unroll
+        for (int i = kLanes; i < P; ++i) {
+            const float x = __fsub_rn(ref[i], cand[i]);
+            d = __fadd_rn(d, __fmul_rn(x, x));
+        }
+        return d;
+    } else {
+        return row_ssd<P>(d, [&](int i) { return ref[i]; }, [&](int i) { return cand[i]; });
+    }
+}
+
+template <int P>
+__device__ __forceinline__ void load_ref_row(float (&row)[ref_stride(P)], const float* ref) {
+#pragma unroll
+    for (int i = 0; i < ref_stride(P); i += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(ref + i);
+        row[i] = v.x;
+        row[i + 1] = v.y;
+        row[i + 2] = v.z;
+        row[i + 3] = v.w;
+    }
+}
+
+// Distances of one lane task (candidate column col0, rows row0 .. row0 + KY-1)
+// against the warp's reference patch, over planes [q0, q1) of scheduled frame
+// k, added to dist.  Planes in shared memory are ordered (channel, t); region
+// row stride `rs`.  A region row is loaded once for the KY candidates it
+// belongs to; the KY reference rows they compare it with slide along in
+// registers.
 template <int P>
 __device__ __forceinline__ void task_distances(const float* planes, int plane_values, int rs, int col0,
-                                               int row0, const float* ref, int planes_n, int p_dyn,
-                                               float dist[kKY]) {
+                                               int row0, const float* ref, int q0, int q1, int p_dyn,
+                                               float (&dist)[kKY]) {
     const int PP = P > 0 ? P : p_dyn;
-#pragma unroll
-    for (int j = 0; j < kKY; ++j) dist[j] = 0.0f;
-    for (int q = 0; q < planes_n; ++q) {
+    const int RS = ref_stride(PP);
+    for (int q = q0; q < q1; ++q) {
         const float* plane = planes + q * plane_values + row0 * rs + col0;
-        const float* ref_plane = ref + q * PP * PP;
-        if constexpr (P == kLanes) {
-            // packed pairs: half the FP32 instructions, the same bits
-            float2 rv[P * P / 2];
-#pragma unroll
-            for (int i = 0; i < P * P / 2; ++i) rv[i] = make_float2(ref_plane[2 * i], ref_plane[2 * i + 1]);
+        const float* ref_plane = ref + q * PP * RS;
+        if constexpr (P > 0) {
+            float rv[kKY][ref_stride(P)];
 #pragma unroll
             for (int r = 0; r < kKY + P - 1; ++r) {
-                float2 cv[P / 2];
-#pragma unroll
-                for (int i = 0; i < P / 2; ++i) cv[i] = make_float2(plane[r * rs + 2 * i], plane[r * rs + 2 * i + 1]);
-#pragma unroll
-                for (int j = 0; j < kKY; ++j) {
-                    const int y = r - j;
-                    if (y >= 0 && y < P) dist[j] = row_ssd8_x2(dist[j], rv + y * (P / 2), cv);
-                }
-            }
-        } else if constexpr (P > 0) {
-            float rv[P * P];
-#pragma unroll
-            for (int i = 0; i < P * P; ++i) rv[i] = ref_plane[i];
-#pragma unroll
-            for (int r = 0; r < kKY + P - 1; ++r) {
+                if (r < P) load_ref_row<P>(rv[r % kKY], ref_plane + r * RS);
                 float cv[P];
 #pragma unroll
                 for (int i = 0; i < P; ++i) cv[i] = plane[r * rs + i];
 #pragma unroll
                 for (int j = 0; j < kKY; ++j) {
                     const int y = r - j;
-                    if (y >= 0 && y < P) {
-                        dist[j] = row_ssd<P>(dist[j], [&](int i) { return rv[y * P + i]; },
-                                             [&](int i) { return cv[i]; });
-                    }
+                    if (y >= 0 && y < P) dist[j] = add_row_ssd<P>(dist[j], rv[y % kKY], cv);
                 }
             }
         } else {
@@ -176,11 +200,31 @@ __device__ __forceinline__ void task_distances(const float* planes, int plane_va
                 for (int j = 0; j < kKY; ++j) {
                     const int y = r - j;
                     if (y >= 0 && y < PP)
-                        dist[j] = row_ssd_dyn(dist[j], ref_plane + y * PP, plane + r * rs, PP);
+                        dist[j] = row_ssd_dyn(dist[j], ref_plane + y * RS, plane + r * rs, PP);
                 }
             }
         }
     }
+}
+
+// One candidate's distance over one more plane.
+template <int P>
+__device__ __forceinline__ float plane_distance(float d, const float* plane, int rs, const float* ref_plane,
+                                                int p_dyn) {
+    if constexpr (P > 0) {
+#pragma unroll
+        for (int y = 0; y < P; ++y) {
+            float rv[ref_stride(P)], cv[P];
+            load_ref_row<P>(rv, ref_plane + y * ref_stride(P));
+#pragma unroll
+            for (int i = 0; i < P; ++i) cv[i] = plane[y * rs + i];
+            d = add_row_ssd<P>(d, rv, cv);
+        }
+    } else {
+        for (int y = 0; y < p_dyn; ++y)
+            d = row_ssd_dyn(d, ref_plane + y * ref_stride(p_dyn), plane + y * rs, p_dyn);
+    }
+    return d;
 }
 
 // Approximate distances of one lane task for 8x8 patches (chosen form):
@@ -276,7 +320,18 @@ __device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* m
         : "memory");
 }
 
-template <int P, bool kApprox, bool kFlow>  // kFlow: search centres from L.centers
+// kFlow: search centres from L.centers.  kWords: the capped buffer and the
+// K-smallest front live in registers, slot i of the buffer in word i / 32 of
+// lane i % 32 (buffers of up to 32 kWords entries and K <= 32); 0: any size,
+// the buffer in shared memory and the front in up to four registers.  Buffers
+// of 64 in shared memory, with one lane running the final partial sort, took
+// half of the kernel: 57k anchors at 960x540 YUV (block 7, a 27 x 27 window,
+// two frames) 3.08 ms for the two planes of Basic and 5.98 ms for the six of
+// Final, now 1.66 and 3.45 ms (FP32 issue alone: 0.7 and 2.0 ms).  Blocks of
+// 10 took 9.2 ms for 83k anchors in the run-time loop, now 2.0 ms.  kPrune:
+// the later planes of candidates that can still pass only (MatchLaunch::
+// prune_cap > 0); its state costs registers, so the others do without.
+template <int P, bool kApprox, bool kFlow, int kWords, bool kPrune>
 __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __grid_constant__ CUtensorMap tmap) {
     extern __shared__ __align__(128) float smem[];
     __shared__ __align__(8) unsigned long long stage_bar;
@@ -304,9 +359,10 @@ __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __gr
     float* rowsq = norms + (kApprox ? plane_values : 0);
     float* warp_base = planes + planes_n * plane_values + (kApprox ? 2 * plane_values : 0) + warp * L.warp_floats;
     float* dist = warp_base;                                  // window_cells
-    float* ref = dist + L.window_cells;                        // planes_n * P * P
-    float* buf_d = ref + planes_n * Pd * Pd;                   // buffer_cap
+    float* ref = dist + ((L.window_cells + 3) & ~3);           // planes_n * P rows of ref_stride(P)
+    float* buf_d = ref + planes_n * Pd * ref_stride(Pd);       // buffer_cap
     int* buf_i = reinterpret_cast<int*>(buf_d + L.buffer_cap); // buffer_cap
+    unsigned short* survivors = reinterpret_cast<unsigned short*>(buf_i + L.buffer_cap);  // prune_cap
 
     const bool active_warp = warp < strip.count;
     const int g = strip.first + warp;
@@ -332,16 +388,47 @@ __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __gr
     s.worst = kInf;
     s.top_count = 0;
     s.top_front = kInf;
-    float my_top[kMaxTopPerLane];
-#pragma unroll
-    for (int i = 0; i < kMaxTopPerLane; ++i) my_top[i] = -kInf;
     const int K = L.K;
-    // register-resident buffer and heap when both fit in a warp
-    const bool fast = s.cap <= 32 && K <= 32;
-    unsigned reg_d = 0u, reg_top = 0u;  // bits of non-negative distances (0 = empty)
-    int reg_id = 0;
+    constexpr int kRegWords = kWords > 0 ? kWords : 1;
+    unsigned reg_d[kRegWords], reg_top = 0u;  // bits of non-negative distances (0 = empty)
+    int reg_id[kRegWords];
+#pragma unroll
+    for (int w = 0; w < kRegWords; ++w) {
+        reg_d[w] = 0u;
+        reg_id[w] = 0;
+    }
+    constexpr int kTopWords = kWords > 0 ? 1 : kMaxTopPerLane;
+    float my_top[kTopWords];
+#pragma unroll
+    for (int i = 0; i < kTopWords; ++i) my_top[i] = -kInf;
     float ref_norm = 0.0f;   // chosen form: ||reference||^2
     float reg_exact = 0.0f;  // chosen form: exact distance of this lane's buffer slot
+    const auto current_limit = [&] {
+        const float limit = s.top_count >= K ? std_max(L.tau, s.top_front) : kInf;
+        return s.count >= s.cap ? std_min(limit, s.worst) : limit;
+    };
+    // the buffer's largest distance and its first slot (std::max_element):
+    // non-negative floats order like their bit patterns
+    const auto find_worst = [&] {
+        unsigned m = reg_d[0];
+#pragma unroll
+        for (int w = 1; w < kRegWords; ++w) m = max(m, reg_d[w]);
+        m = __reduce_max_sync(0xffffffffu, m);
+        s.worst = __uint_as_float(m);
+#pragma unroll
+        for (int w = kRegWords - 1; w >= 0; --w) {
+            const unsigned hit = __ballot_sync(0xffffffffu, reg_d[w] == m);
+            if (hit) s.worst_idx = 32 * w + __ffs(hit) - 1;
+        }
+    };
+    const auto put = [&](int slot, float d, int id) {
+#pragma unroll
+        for (int w = 0; w < kRegWords; ++w)
+            if (32 * w + lane == slot) {
+                reg_d[w] = __float_as_uint(d);
+                reg_id[w] = id;
+            }
+    };
 
     // Flow-guided search: every warp's window of frame k lies around its
     // anchor's search centre there (same size as the anchor-centred one).  The
@@ -470,7 +557,8 @@ __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __gr
                 const int rem = i - q * Pd * Pd;
                 const int py = rem / Pd;
                 const int px = rem - py * Pd;
-                ref[i] = planes[q * plane_values + (ay - ry0 + py) * L.region_stride + (ax - rx0 + px)];
+                ref[(q * Pd + py) * ref_stride(Pd) + px] =
+                    planes[q * plane_values + (ay - ry0 + py) * L.region_stride + (ax - rx0 + px)];
             }
             __syncwarp();
             if constexpr (kApprox) {
@@ -481,63 +569,102 @@ __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __gr
                 ref_norm = acc;
             }
         }
-        // Distances of all candidates of frame k.
-        for (int task = lane; task < tasks; task += 32) {
-            const int cx = task % Wx;
-            const int gy = task / Wx;
-            float d[kKY];
-            if constexpr (kApprox)
-                task_distances_approx(planes, plane_values, L.region_stride, xl - rx0 + cx, yl - ry0 + gy * kKY, ref,
-                                      planes_n, ref_norm, norms, d);
-            else
-                task_distances<P>(planes, plane_values, L.region_stride, xl - rx0 + cx, yl - ry0 + gy * kKY, ref,
-                                  planes_n, Pd, d);
+        // Distances of all candidates of frame k.  With kPrune, those planes
+        // [0, 1) first: an SSD only grows plane by plane, so a candidate whose
+        // first plane exceeds the limit the frame starts with cannot pass the
+        // replay, whose limit only shrinks.  It keeps its partial distance,
+        // and the later planes run on the packed list of the others, if the
+        // list holds them (prune_cap, half of the window: a listed candidate
+        // costs about 1.3 times one of a task, which shares its region rows
+        // with three others).
+        const int rs = L.region_stride;
+        const float frame_limit = current_limit();
+        const auto dense = [&](int q0, int q1) {
+            for (int task = lane; task < tasks; task += 32) {
+                const int cx = task % Wx;
+                const int gy = task / Wx;
+                float d[kKY];
+                if constexpr (kApprox) {
+                    task_distances_approx(planes, plane_values, rs, xl - rx0 + cx, yl - ry0 + gy * kKY, ref, planes_n,
+                                          ref_norm, norms, d);
+                } else {
 #pragma unroll
-            for (int j = 0; j < kKY; ++j) {
-                const int cy = gy * kKY + j;
-                if (cy < Wy) dist[cy * Wx + cx] = d[j];
+                    for (int j = 0; j < kKY; ++j) {
+                        const int cy = gy * kKY + j;
+                        d[j] = kPrune && q0 > 0 && cy < Wy ? dist[cy * Wx + cx] : 0.0f;
+                    }
+                    task_distances<P>(planes, plane_values, rs, xl - rx0 + cx, yl - ry0 + gy * kKY, ref, q0, q1, Pd, d);
+                }
+#pragma unroll
+                for (int j = 0; j < kKY; ++j) {
+                    const int cy = gy * kKY + j;
+                    if (cy < Wy) dist[cy * Wx + cx] = d[j];
+                }
+            }
+            __syncwarp();
+        };
+        if (!kPrune || !(frame_limit < kInf)) {
+            dense(0, planes_n);
+        } else {
+            dense(0, 1);
+            int n = 0;
+            for (int base = 0; base < cells && n <= L.prune_cap; base += 32) {
+                const int idx = base + lane;
+                const bool in = idx < cells && dist[idx] <= frame_limit;
+                const unsigned mask = __ballot_sync(0xffffffffu, in);
+                const int at = n + __popc(mask & ((1u << lane) - 1u));
+                if (in && at < L.prune_cap) survivors[at] = static_cast<unsigned short>(idx);
+                n += __popc(mask);
+            }
+            if (n > L.prune_cap) {
+                dense(1, planes_n);
+            } else {
+                for (int q = 1; q < planes_n; ++q) {
+                    __syncwarp();
+                    int kept = 0;
+                    for (int base = 0; base < n; base += 32) {
+                        const int i = base + lane;
+                        int cell = 0;
+                        float d = kInf;
+                        if (i < n) {
+                            cell = survivors[i];
+                            const int cy = cell / Wx;
+                            const float* at = planes + q * plane_values + (yl - ry0 + cy) * rs + xl - rx0 + cell - cy * Wx;
+                            d = plane_distance<P>(dist[cell], at, rs, ref + q * Pd * ref_stride(Pd), Pd);
+                            dist[cell] = d;
+                        }
+                        // the list shrinks in place (entries move down only)
+                        const bool in = d <= frame_limit;
+                        const unsigned mask = __ballot_sync(0xffffffffu, in);
+                        if (in) survivors[kept + __popc(mask & ((1u << lane) - 1u))] = static_cast<unsigned short>(cell);
+                        kept += __popc(mask);
+                        __syncwarp();
+                    }
+                    n = kept;
+                }
+                __syncwarp();
             }
         }
-        __syncwarp();
         // Replay of the CPU's sequential selection over frame k, raster order.
-        if (fast) {
-            // buffer slot i and heap entry i live in lane i; non-negative float
-            // distances order like their bit patterns, so the first maximum
-            // (std::max_element) is a max-reduction and a ballot
+        if constexpr (kWords > 0) {
             for (int base = 0; base < cells; base += 32) {
                 const int idx = base + lane;
                 const float mine = idx < cells ? dist[idx] : kInf;
-                float limit = s.top_count >= K ? std_max(L.tau, s.top_front) : kInf;
-                if (s.count >= s.cap) limit = std_min(limit, s.worst);
-                unsigned pass = __ballot_sync(0xffffffffu, idx < cells && mine <= limit);
+                unsigned pass = __ballot_sync(0xffffffffu, idx < cells && mine <= current_limit());
                 while (pass) {
                     const int src_lane = __ffs(pass) - 1;
                     pass &= pass - 1;
                     const float d = __shfl_sync(0xffffffffu, mine, src_lane);
-                    limit = s.top_count >= K ? std_max(L.tau, s.top_front) : kInf;
-                    if (s.count >= s.cap) limit = std_min(limit, s.worst);
-                    if (!(d <= limit)) continue;
+                    if (!(d <= current_limit())) continue;
                     const int id = (k << 20) | (base + src_lane);
                     // record_candidate_match
                     if (s.count < s.cap) {
-                        if (lane == s.count) {
-                            reg_d = __float_as_uint(d);
-                            reg_id = id;
-                        }
+                        put(s.count, d, id);
                         s.count++;
-                        if (s.count == s.cap) {
-                            const unsigned w = __reduce_max_sync(0xffffffffu, reg_d);
-                            s.worst_idx = __ffs(__ballot_sync(0xffffffffu, reg_d == w)) - 1;
-                            s.worst = __uint_as_float(w);
-                        }
+                        if (s.count == s.cap) find_worst();
                     } else if (d < s.worst) {
-                        if (lane == s.worst_idx) {
-                            reg_d = __float_as_uint(d);
-                            reg_id = id;
-                        }
-                        const unsigned w = __reduce_max_sync(0xffffffffu, reg_d);
-                        s.worst_idx = __ffs(__ballot_sync(0xffffffffu, reg_d == w)) - 1;
-                        s.worst = __uint_as_float(w);
+                        put(s.worst_idx, d, id);
+                        find_worst();
                     }
                     // record_candidate_distance: the K smallest so far
                     if (s.top_count < K) {
@@ -555,75 +682,70 @@ __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __gr
             if constexpr (kApprox) {
                 // exact FP32 distance of the buffer slots frame k filled, while
                 // frame k is staged: each lane re-ranks its own slot
-                if (lane < s.count && (reg_id >> 20) == k) {
-                    const int cell = reg_id & 0xfffff;
+                if (lane < s.count && (reg_id[0] >> 20) == k) {
+                    const int cell = reg_id[0] & 0xfffff;
                     const int cy = cell / Wx;
                     reg_exact = exact_distance8(planes, plane_values, L.region_stride, xl - rx0 + (cell - cy * Wx),
                                                 yl - ry0 + cy, ref, planes_n);
                 }
             }
-            continue;
-        }
-        // Replay of the CPU's sequential selection over frame k, raster order.
-        for (int base = 0; base < cells; base += 32) {
-            const int idx = base + lane;
-            const float mine = idx < cells ? dist[idx] : kInf;
-            float limit = s.top_count >= K ? std_max(L.tau, s.top_front) : kInf;
-            if (s.count >= s.cap) limit = std_min(limit, s.worst);
-            unsigned pass = __ballot_sync(0xffffffffu, idx < cells && mine <= limit);
-            while (pass) {
-                const int src_lane = __ffs(pass) - 1;
-                pass &= pass - 1;
-                const float d = __shfl_sync(0xffffffffu, mine, src_lane);
-                limit = s.top_count >= K ? std_max(L.tau, s.top_front) : kInf;
-                if (s.count >= s.cap) limit = std_min(limit, s.worst);
-                if (!(d <= limit)) continue;
-                const int id = (k << 20) | (base + src_lane);
-                // record_candidate_match
-                if (s.count < s.cap) {
-                    if (lane == 0) {
-                        buf_d[s.count] = d;
-                        buf_i[s.count] = id;
+        } else {
+            for (int base = 0; base < cells; base += 32) {
+                const int idx = base + lane;
+                const float mine = idx < cells ? dist[idx] : kInf;
+                unsigned pass = __ballot_sync(0xffffffffu, idx < cells && mine <= current_limit());
+                while (pass) {
+                    const int src_lane = __ffs(pass) - 1;
+                    pass &= pass - 1;
+                    const float d = __shfl_sync(0xffffffffu, mine, src_lane);
+                    if (!(d <= current_limit())) continue;
+                    const int id = (k << 20) | (base + src_lane);
+                    // record_candidate_match
+                    if (s.count < s.cap) {
+                        if (lane == 0) {
+                            buf_d[s.count] = d;
+                            buf_i[s.count] = id;
+                        }
+                        s.count++;
+                        __syncwarp();
+                        if (s.count == s.cap) refresh_worst(buf_d, s.count, lane, s.worst_idx, s.worst);
+                    } else if (d < s.worst) {
+                        if (lane == 0) {
+                            buf_d[s.worst_idx] = d;
+                            buf_i[s.worst_idx] = id;
+                        }
+                        __syncwarp();
+                        refresh_worst(buf_d, s.count, lane, s.worst_idx, s.worst);
                     }
-                    s.count++;
-                    __syncwarp();
-                    if (s.count == s.cap) refresh_worst(buf_d, s.count, lane, s.worst_idx, s.worst);
-                } else if (d < s.worst) {
-                    if (lane == 0) {
-                        buf_d[s.worst_idx] = d;
-                        buf_i[s.worst_idx] = id;
-                    }
-                    __syncwarp();
-                    refresh_worst(buf_d, s.count, lane, s.worst_idx, s.worst);
-                }
-                // record_candidate_distance
-                if (s.top_count < K) {
-                    const int slot = s.top_count;
-#pragma unroll
-                    for (int i = 0; i < kMaxTopPerLane; ++i)
-                        if (i * 32 + lane == slot) my_top[i] = d;
-                    s.top_count++;
-                    if (s.top_count == K) {
+                    // record_candidate_distance
+                    if (s.top_count < K) {
+                        const int slot = s.top_count;
+    #pragma unroll
+                        for (int i = 0; i < kTopWords; ++i)
+                            if (i * 32 + lane == slot) my_top[i] = d;
+                        s.top_count++;
+                        if (s.top_count == K) {
+                            float m = -kInf;
+    #pragma unroll
+                            for (int i = 0; i < kTopWords; ++i) m = fmaxf(m, my_top[i]);
+                            s.top_front = warp_max(m);
+                        }
+                    } else if (d < s.top_front) {
+                        // replace one entry equal to the maximum
+                        int owner = 0x7fffffff;
+    #pragma unroll
+                        for (int i = 0; i < kTopWords; ++i)
+                            if (owner == 0x7fffffff && my_top[i] == s.top_front) owner = i * 32 + lane;
+    #pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) owner = min(owner, __shfl_xor_sync(0xffffffffu, owner, o));
+    #pragma unroll
+                        for (int i = 0; i < kTopWords; ++i)
+                            if (i * 32 + lane == owner) my_top[i] = d;
                         float m = -kInf;
-#pragma unroll
-                        for (int i = 0; i < kMaxTopPerLane; ++i) m = fmaxf(m, my_top[i]);
+    #pragma unroll
+                        for (int i = 0; i < kTopWords; ++i) m = fmaxf(m, my_top[i]);
                         s.top_front = warp_max(m);
                     }
-                } else if (d < s.top_front) {
-                    // replace one entry equal to the maximum
-                    int owner = 0x7fffffff;
-#pragma unroll
-                    for (int i = 0; i < kMaxTopPerLane; ++i)
-                        if (owner == 0x7fffffff && my_top[i] == s.top_front) owner = i * 32 + lane;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) owner = min(owner, __shfl_xor_sync(0xffffffffu, owner, o));
-#pragma unroll
-                    for (int i = 0; i < kMaxTopPerLane; ++i)
-                        if (i * 32 + lane == owner) my_top[i] = d;
-                    float m = -kInf;
-#pragma unroll
-                    for (int i = 0; i < kMaxTopPerLane; ++i) m = fmaxf(m, my_top[i]);
-                    s.top_front = warp_max(m);
                 }
             }
         }
@@ -632,20 +754,21 @@ __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __gr
     if (!active_warp) return;
     int S = 0;
     bool selected_in_warp = false;
-    if (kApprox && fast && K > 1) {
+    if (kApprox && K > 1) {
         // chosen form: select_similar_patches on the exact distances of the
         // buffer -- the K smallest, the threshold max(tau, d_K), the slots
         // within it, closest first (ties by candidate order), at most the cap
         const int n = s.count;
+        const int own_id = reg_id[0];
         int rank = 0;
         for (int j = 0; j < n; ++j) {
             const float dj = __shfl_sync(0xffffffffu, reg_exact, j);
-            const int ij = __shfl_sync(0xffffffffu, reg_id, j);
-            rank += (dj < reg_exact || (dj == reg_exact && ij < reg_id)) ? 1 : 0;
+            const int ij = __shfl_sync(0xffffffffu, own_id, j);
+            rank += (dj < reg_exact || (dj == reg_exact && ij < own_id)) ? 1 : 0;
         }
         if (lane < n) {
             buf_d[rank] = reg_exact;
-            buf_i[rank] = reg_id;
+            buf_i[rank] = own_id;
         }
         __syncwarp();
         const int M = min(K, n);
@@ -653,58 +776,107 @@ __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __gr
         const int within = __popc(__ballot_sync(0xffffffffu, lane < n && buf_d[lane] <= threshold));
         S = min(within, min(L.soft_cap, n));
         selected_in_warp = true;
-    } else if (fast) {
-        // select_similar_patches with pairwise distinct buffered distances:
-        // the heap replay below has a unique outcome, computed warp-wide.
-        // partial_sort(first, first + M, first + n) keeps in [0, M) the M
-        // smallest in ascending order; tail slot i (M <= i < n) ends up with
-        // the heap's maximum at the time element i arrived when that element
-        // is smaller (it is swapped in), else with the element itself.
+    } else if constexpr (kWords > 0) {
+        // select_similar_patches where the slots within the threshold have
+        // pairwise distinct distances: the heap replay below then has a
+        // unique outcome, computed warp-wide.  The M = min(K, n) smallest come
+        // first, ascending; the front's maximum is d_M.
         const int n = s.count;
-        const unsigned key = lane < n ? reg_d : (0x80000000u | static_cast<unsigned>(lane));
-        const bool tie = __any_sync(0xffffffffu, __popc(__match_any_sync(0xffffffffu, key)) > 1);
-        if (K > 1 && !tie) {
-            const int M = min(K, n);
-            unsigned d = reg_d;
-            int id = reg_id;
-            unsigned cur_max = __reduce_max_sync(0xffffffffu, lane < M ? d : 0u);
-            for (int i = M; i < n; ++i) {
-                const unsigned di = __shfl_sync(0xffffffffu, d, i);
-                const int ii = __shfl_sync(0xffffffffu, id, i);
-                if (di < cur_max) {
-                    const int o = __ffs(__ballot_sync(0xffffffffu, lane < M && d == cur_max)) - 1;
-                    const int oi = __shfl_sync(0xffffffffu, id, o);
-                    if (lane == o) {
-                        d = di;
-                        id = ii;
+        const int M = min(K, n);
+        const float d_m = __uint_as_float(__reduce_max_sync(0xffffffffu, reg_top));
+        const float threshold = std_max(L.tau, d_m);
+        // ranks among the slots within the threshold, and equal ones
+        unsigned within[kRegWords];
+        int total = 0;
+        bool tie = false;
+#pragma unroll
+        for (int w = 0; w < kRegWords; ++w) {
+            within[w] = __ballot_sync(0xffffffffu, 32 * w + lane < n && __uint_as_float(reg_d[w]) <= threshold);
+            total += __popc(within[w]);
+        }
+        if (K > 1) {
+            int rank[kRegWords];
+#pragma unroll
+            for (int w = 0; w < kRegWords; ++w) rank[w] = 0;
+            int equal = 0;
+#pragma unroll
+            for (int v = 0; v < kRegWords; ++v) {
+                for (unsigned m = within[v]; m; m &= m - 1) {
+                    const unsigned dj = __shfl_sync(0xffffffffu, reg_d[v], __ffs(m) - 1);
+#pragma unroll
+                    for (int w = 0; w < kRegWords; ++w) {
+                        rank[w] += dj < reg_d[w] ? 1 : 0;
+                        equal += (within[w] >> lane & 1u) && dj == reg_d[w] ? 1 : 0;
                     }
-                    if (lane == i) {
-                        d = cur_max;
-                        id = oi;
-                    }
-                    cur_max = __reduce_max_sync(0xffffffffu, lane < M ? d : 0u);
                 }
             }
-            // the kept M ascending (distinct: rank = number of smaller ones),
-            // then the tail slots within the threshold, in slot order
-            const float threshold = std_max(L.tau, __uint_as_float(cur_max));
-            int rank = 0;
-            for (int j = 0; j < M; ++j) rank += __shfl_sync(0xffffffffu, d, j) < d ? 1 : 0;
-            const bool keep_tail = lane >= M && lane < n && __uint_as_float(d) <= threshold;
-            const unsigned tail_mask = __ballot_sync(0xffffffffu, keep_tail);
-            if (lane < M) {
-                buf_d[rank] = __uint_as_float(d);
-                buf_i[rank] = id;
-            } else if (keep_tail) {
-                const int pos = M + __popc(tail_mask & ((1u << lane) - 1u));
-                buf_d[pos] = __uint_as_float(d);
-                buf_i[pos] = id;
+            int mine = 0;
+#pragma unroll
+            for (int w = 0; w < kRegWords; ++w) mine += within[w] >> lane & 1u;
+            tie = __any_sync(0xffffffffu, equal != mine);
+            if (!tie) {
+                // the M smallest in order; past them the others within the
+                // threshold, in the order of the slots they end up in
+                if (total > M) {
+                    // partial_sort(first, first + M, first + n): slots [0, M)
+                    // are the heap; tail slot i ends up with the heap's
+                    // maximum at the time element i arrived when that element
+                    // is smaller (it is swapped in), else with the element
+                    // itself.  M <= 32: the heap lies in word 0.
+                    unsigned cur_max = __reduce_max_sync(0xffffffffu, lane < M ? reg_d[0] : 0u);
+#pragma unroll
+                    for (int w = 0; w < kRegWords; ++w) {
+                        for (int i = max(M, 32 * w); i < min(n, 32 * w + 32); ++i) {
+                            const unsigned di = __shfl_sync(0xffffffffu, reg_d[w], i & 31);
+                            if (di >= cur_max) continue;
+                            const int ii = __shfl_sync(0xffffffffu, reg_id[w], i & 31);
+                            const int o = __ffs(__ballot_sync(0xffffffffu, lane < M && reg_d[0] == cur_max)) - 1;
+                            const int oi = __shfl_sync(0xffffffffu, reg_id[0], o);
+                            if (lane == o) {
+                                reg_d[0] = di;
+                                reg_id[0] = ii;
+                            }
+                            if (lane == (i & 31)) {
+                                reg_d[w] = cur_max;
+                                reg_id[w] = oi;
+                            }
+                            cur_max = __reduce_max_sync(0xffffffffu, lane < M ? reg_d[0] : 0u);
+                        }
+                    }
+                    int r0 = 0;
+                    for (int j = 0; j < M; ++j) r0 += __shfl_sync(0xffffffffu, reg_d[0], j) < reg_d[0] ? 1 : 0;
+                    int at = M;
+#pragma unroll
+                    for (int w = 0; w < kRegWords; ++w) {
+                        const int slot = 32 * w + lane;
+                        const bool keep = slot >= M && slot < n && __uint_as_float(reg_d[w]) <= threshold;
+                        const unsigned mask = __ballot_sync(0xffffffffu, keep);
+                        const int pos = slot < M ? r0 : at + __popc(mask & ((1u << lane) - 1u));
+                        if (slot < M || keep) {
+                            buf_d[pos] = __uint_as_float(reg_d[w]);
+                            buf_i[pos] = reg_id[w];
+                        }
+                        at += __popc(mask);
+                    }
+                } else {
+#pragma unroll
+                    for (int w = 0; w < kRegWords; ++w)
+                        if (within[w] >> lane & 1u) {
+                            buf_d[rank[w]] = __uint_as_float(reg_d[w]);
+                            buf_i[rank[w]] = reg_id[w];
+                        }
+                }
+                S = total;
+                selected_in_warp = true;
             }
-            S = M + __popc(tail_mask);
-            selected_in_warp = true;
-        } else if (lane < n) {
-            buf_d[lane] = __uint_as_float(reg_d);
-            buf_i[lane] = reg_id;
+        }
+        if (!selected_in_warp) {
+#pragma unroll
+            for (int w = 0; w < kRegWords; ++w)
+                if (32 * w + lane < n) {
+                    buf_d[32 * w + lane] = __uint_as_float(reg_d[w]);
+                    buf_i[32 * w + lane] = reg_id[w];
+                }
         }
         __syncwarp();
     }
@@ -871,8 +1043,8 @@ size_t match_shared_bytes(const MatchLaunch& L, int warps) {
     return (planes + static_cast<size_t>(warps) * L.warp_floats) * sizeof(float);
 }
 
-int match_warp_floats(int window_cells, int planes_n, int P, int buffer_cap) {
-    int f = window_cells + planes_n * P * P + 2 * buffer_cap;
+int match_warp_floats(int window_cells, int planes_n, int P, int buffer_cap, int prune_cap) {
+    const int f = ((window_cells + 3) & ~3) + planes_n * P * ref_stride(P) + 2 * buffer_cap + (prune_cap + 1) / 2;
     return (f + 3) & ~3;
 }
 
@@ -917,31 +1089,55 @@ cudaError_t launch_match(const MatchLaunch& L, int strips, int warps, const CUte
         kernel<<<strips, block, smem, stream>>>(L, map);
         err = cudaGetLastError();
     };
-    if (L.centers) {  // flow-guided search: windows around per-frame search centres
-        if (L.approx || warps > 8) return cudaErrorInvalidValue;
+    // words per lane of the register-resident buffer: the entries it can hold
+    // at once (its cap, or every candidate when there are fewer)
+    const long long candidates = static_cast<long long>(L.window_cells) * L.schedule_len;
+    const long long entries = L.soft_cap < candidates ? L.soft_cap : candidates;
+    const int words = L.K > 32 || entries > 128 ? 0 : entries <= 32 ? 1 : entries <= 64 ? 2 : 4;
+    // the patch sizes with kernels of their own; 0 takes any
+    const auto with_patch = [&](auto run) {
         switch (L.P) {
-            case 4: launch(match_kernel<4, false, true>); break;
-            case 5: launch(match_kernel<5, false, true>); break;
-            case 6: launch(match_kernel<6, false, true>); break;
-            case 7: launch(match_kernel<7, false, true>); break;
-            case 8: launch(match_kernel<8, false, true>); break;
-            default: launch(match_kernel<0, false, true>); break;
+            case 4: run(std::integral_constant<int, 4>{}); break;
+            case 5: run(std::integral_constant<int, 5>{}); break;
+            case 6: run(std::integral_constant<int, 6>{}); break;
+            case 7: run(std::integral_constant<int, 7>{}); break;
+            case 8: run(std::integral_constant<int, 8>{}); break;
+            case 10: run(std::integral_constant<int, 10>{}); break;
+            default: run(std::integral_constant<int, 0>{}); break;
         }
+    };
+    if (L.centers) {  // flow-guided search: windows around per-frame search centres
+        if (L.approx || warps > 8 || L.prune_cap > 0) return cudaErrorInvalidValue;
+        const auto flow = [&](auto patch) {
+            constexpr int P = decltype(patch)::value;
+            if (words == 0) launch(match_kernel<P, false, true, 0, false>);
+            else if (words == 1) launch(match_kernel<P, false, true, 1, false>);
+            else launch(match_kernel<P, false, true, 4, false>);
+        };
+        with_patch(flow);
         return err;
     }
     if (L.approx) {
-        if (L.P != kLanes) return cudaErrorInvalidValue;
-        launch(match_kernel<8, true, false>);
+        if (L.P != kLanes || words != 1) return cudaErrorInvalidValue;
+        launch(match_kernel<8, true, false, 1, false>);
         return err;
     }
-    switch (L.P) {
-        case 4: launch(match_kernel<4, false, false>); break;
-        case 5: launch(match_kernel<5, false, false>); break;
-        case 6: launch(match_kernel<6, false, false>); break;
-        case 7: launch(match_kernel<7, false, false>); break;
-        case 8: launch(match_kernel<8, false, false>); break;
-        default: launch(match_kernel<0, false, false>); break;
-    }
+    const auto plain = [&](auto patch) {
+        constexpr int P = decltype(patch)::value;
+        constexpr int kTwo = P >= 4 && P <= 6 ? 4 : 2;  // two words for the usual block sizes only
+        if (L.prune_cap > 0 && words > 0) {
+            if (words <= 2) launch(match_kernel<P, false, false, kTwo, true>);
+            else launch(match_kernel<P, false, false, 4, true>);
+            return;
+        }
+        switch (words) {
+            case 1: launch(match_kernel<P, false, false, 1, false>); break;
+            case 2: launch(match_kernel<P, false, false, kTwo, false>); break;
+            case 4: launch(match_kernel<P, false, false, 4, false>); break;
+            default: launch(match_kernel<P, false, false, 0, false>); break;
+        }
+    };
+    with_patch(plain);
     return err;
 }
 

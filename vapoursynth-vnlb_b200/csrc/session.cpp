@@ -532,9 +532,27 @@ struct Session {
         probe.region_stride = region_stride;
         probe.plane_floats = plane_floats_of(region_rows, region_stride);
         probe.approx = approx ? 1 : 0;
-        probe.warp_floats = match_warp_floats(cw0 * ch0, search_channels * Pt, P, buffer_cap);
-        return match_shared_bytes(probe, w) <= 200 * 1024;
+        const int planes_n = search_channels * Pt;
+        const auto bytes = [&](int cap) {
+            probe.warp_floats = match_warp_floats(cw0 * ch0, planes_n, P, buffer_cap, cap);
+            return match_shared_bytes(probe, w);
+        };
+        // the list of candidates whose later planes are worth computing
+        // (MatchLaunch::prune_cap): half of the window, from four planes up (57k
+        // anchors of 6 planes 3.64 -> 3.34 ms; with 2 and 3 planes the first
+        // plane's pass over the window costs more than it saves: 2.00 -> 2.13,
+        // 0.97 -> 1.01 ms), where it leaves as many blocks on a multiprocessor
+        // (the kernel is compiled for three)
+        const auto resident = [](size_t b) { return std::min<size_t>(3, (227 * 1024) / (b + 1024)); };
+        const int half = cw0 * ch0 / 2;
+        prune_cap = 0;
+        if (planes_n >= 4 && !approx && half >= 32 && half <= 0x7fff && resident(bytes(half)) == resident(bytes(0)))
+            prune_cap = half;
+        // one anchor per block fits whatever fits without the rows' padding
+        const size_t padding = w > 1 ? 0 : 4 * static_cast<size_t>(planes_n * P * ((4 - P % 4) % 4) + 3 + prune_cap);
+        return bytes(prune_cap) <= 200 * 1024 + padding;
     }
+    int prune_cap = 0;
     // flow-guided search: the strips' reservation widened by up to 16 columns
     // and 8 rows while the shared memory allows
     void set_flow_region() {
@@ -551,7 +569,7 @@ struct Session {
             probe.region_rows = flow_region_rows;
             probe.region_stride = flow_region_stride;
             probe.plane_floats = plane_floats_of(flow_region_rows, flow_region_stride);
-            probe.warp_floats = match_warp_floats(cw0 * ch0, search_channels * Pt, P, buffer_cap);
+            probe.warp_floats = match_warp_floats(cw0 * ch0, search_channels * Pt, P, buffer_cap, 0);
             if (match_shared_bytes(probe, warps) <= 200 * 1024) break;
         }
     }
@@ -1373,7 +1391,8 @@ struct Session {
         m.window_cells = cw * chh;
         m.buffer_cap = buffer_cap;
         m.approx = approx ? 1 : 0;
-        m.warp_floats = match_warp_floats(m.window_cells, search_channels * Pt, P, buffer_cap);
+        m.prune_cap = flow_on() ? 0 : prune_cap;
+        m.warp_floats = match_warp_floats(m.window_cells, search_channels * Pt, P, buffer_cap, m.prune_cap);
         m.rows = lane.rows.ptr;
         m.row_counts = lane.row_counts.ptr;
         m.victims = lane.victims.ptr;

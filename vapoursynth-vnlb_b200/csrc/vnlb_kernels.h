@@ -73,6 +73,8 @@ struct MatchLaunch {
     int window_cells;     // max Wx*Wy
     int buffer_cap;       // match buffer capacity per warp
     int warp_floats;      // shared floats per warp
+    int prune_cap;        // plain matcher, several planes: candidates (at most) whose later planes are computed
+                          // from a list instead of for the whole window; 0: no list (see match_prune_cap)
     int approx;           // chosen form in this matcher: approximate distances, exact re-rank
     // tensor-core form (match_chosen.cu)
     int tiles_x;          // 8-column candidate blocks per strip
@@ -150,7 +152,7 @@ struct CentersLaunch {
 cudaError_t launch_centers(const CentersLaunch& L, cudaStream_t stream);
 
 size_t match_shared_bytes(const MatchLaunch& L, int warps);
-int match_warp_floats(int window_cells, int planes_n, int P, int buffer_cap);
+int match_warp_floats(int window_cells, int planes_n, int P, int buffer_cap, int prune_cap);
 // tmap: the search source store as a 2-D float tensor (width x rows of every
 // plane of every slot), box (region_stride, region_rows); used when L.tma.
 cudaError_t launch_match(const MatchLaunch& L, int strips, int warps, const CUtensorMap* tmap,
