@@ -1622,56 +1622,48 @@ __global__ void __launch_bounds__(32 * kTileWarps, kQ == 1 ? 4 : 2) apply_tile_k
 // for D % 32 == 0, rank <= 8 and at most 8 model rows (the shapes of the
 // default parameter sets: 8x8 patches, one or three planes, rank 8, group 8).
 //
-// A lane owns columns lane + 32 jj for the elementwise work (centred model
-// rows in registers, basis columns, the reconstruction and its store); for
-// the dot products octet k = lane / 8 runs the pinned 8-lane chains j = lane
-// % 8 over elements j + 8 m of components k and k + 4 at once, on packed
-// pairs: the basis sits in shared memory as float2 (component p, p + 4), so
-// one 8-byte load and one packed fused multiply-add advance both chains.
-// Per warp (floats): basis [4][D] float2, u[D], v[D], dual [8][8],
-// per-component scalars [5][8], scores[max_rows], row bases[max_rows] (size_t).
+// A lane owns columns lane + 32 jj for the elementwise work (the centred model
+// rows and all components' basis values of a block of columns in registers, the
+// reconstruction and its store).  The rows go in tiles of four, [column][row]
+// beside a basis [column][component]: for the dot products lane (j, q, h) runs
+// the pinned chain j (columns j + 8 m) of rows 2 h, 2 h + 1 against components
+// 4 q .. 4 q + 3, so an 8-byte and a 16-byte load feed eight multiply-adds, and
+// the halving folds leave every lane with one row's dot of one component.  (A
+// row at a time with a component pair per octet, it took 490 / 548 us for 32k
+// groups at D = 192, Basic / Final, now 255 / 407 us.)
+// Per warp (floats): basis [D][12], U [D][4], V [D][4] (Final), dual [8][8],
+// per-component scalars [5][8], projections [8][4], quotients and squares
+// [4][8], norms [4], scores[max_rows], row bases[max_rows] (size_t).
 constexpr int kWarpApplyWarps = 4;
+constexpr int kWarpLdb = 12;  // floats per basis column: 8 columns start 3 bank quads apart
 
 struct WarpApplyLayout {
-    int basis, u, v, dual, scal, scores, recon, rw, bases, per_warp;
+    int basis, u, v, dual, scal, proj, quot, square, norms, scores, recon, rw, bases, per_warp;
 };
 
 // scatter: also the rows' scaled projections [max_rows][8] and weights
 // [max_rows], kept for the second pass that adds the rows into the stack
-__host__ __device__ inline WarpApplyLayout warp_apply_layout(int D, int max_rows, bool scatter = false) {
+__host__ __device__ inline WarpApplyLayout warp_apply_layout(int D, int max_rows, bool final_stage,
+                                                             bool scatter) {
     WarpApplyLayout w{};
     int off = 0;
-    w.basis = off;  off += 8 * D;
-    w.u = off;      off += D;
-    w.v = off;      off += D;
+    w.basis = off;  off += kWarpLdb * D;
+    w.u = off;      off += 4 * D;
+    w.v = off;      off += final_stage ? 4 * D : 0;
     w.dual = off;   off += 64;
     w.scal = off;   off += 5 * 8;
+    w.proj = off;   off += 32;
+    w.quot = off;   off += 32;
+    w.square = off; off += 32;
+    w.norms = off;  off += 4;
+    w.recon = off;  off += scatter ? 8 * ((max_rows + 3) & ~3) : 0;
     w.scores = off; off += max_rows;
-    w.recon = off;  off += scatter ? 8 * max_rows : 0;
     w.rw = off;     off += scatter ? max_rows : 0;
     off = (off + 1) & ~1;
     w.bases = off;  off += 2 * max_rows;
     off = (off + 3) & ~3;
     w.per_warp = off;
     return w;
-}
-
-__device__ __forceinline__ float2 octet_reduce2(float2 v) {
-    // the reduce8 fold of lanes 8k .. 8k+7 into lane 8k, for both halves
-    v.x = __fadd_rn(v.x, __shfl_down_sync(0xffffffffu, v.x, 4, 8));
-    v.y = __fadd_rn(v.y, __shfl_down_sync(0xffffffffu, v.y, 4, 8));
-    v.x = __fadd_rn(v.x, __shfl_down_sync(0xffffffffu, v.x, 2, 8));
-    v.y = __fadd_rn(v.y, __shfl_down_sync(0xffffffffu, v.y, 2, 8));
-    v.x = __fadd_rn(v.x, __shfl_down_sync(0xffffffffu, v.x, 1, 8));
-    v.y = __fadd_rn(v.y, __shfl_down_sync(0xffffffffu, v.y, 1, 8));
-    return v;
-}
-
-__device__ __forceinline__ float octet_reduce(float v) {
-    v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, 4, 8));
-    v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, 2, 8));
-    v = __fadd_rn(v, __shfl_down_sync(0xffffffffu, v, 1, 8));
-    return v;
 }
 
 // resident blocks per SM the warp-per-group apply is compiled for (a register
@@ -1755,7 +1747,48 @@ __device__ __forceinline__ void scatter_row(const FilterLaunch& L, const MatchRo
     }
 }
 
-template <int D, bool kScatter>
+// A tile's reconstruction (project_bayes_estimate) of this lane's columns, the
+// components in order: o[row][jj].
+template <int kCols>
+__device__ __forceinline__ void warp_reconstruct(const float* basis, const float* sc, const float* coef, int R, int lane,
+                                                 const float (&cc)[kCols], float (&o)[4][kCols]) {
+    float2 acc[kCols][2];
+#pragma unroll
+    for (int jj = 0; jj < kCols; ++jj) acc[jj][0] = acc[jj][1] = make_float2(0.0f, 0.0f);
+#pragma unroll
+    for (int c0 = 0; c0 < 8; c0 += 4) {
+        if (c0 >= R) break;
+        float b[kCols][4];
+#pragma unroll
+        for (int jj = 0; jj < kCols; ++jj) {
+            const float4 t = *reinterpret_cast<const float4*>(basis + (lane + 32 * jj) * kWarpLdb + c0);
+            b[jj][0] = t.x;
+            b[jj][1] = t.y;
+            b[jj][2] = t.z;
+            b[jj][3] = t.w;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c0 + c >= R || coef[c0 + c] == 0.0f) continue;
+            const float4 s = *reinterpret_cast<const float4*>(sc + 4 * (c0 + c));
+            const float2 s01 = make_float2(s.x, s.y), s23 = make_float2(s.z, s.w);
+#pragma unroll
+            for (int jj = 0; jj < kCols; ++jj) {
+                acc[jj][0] = fma2_rn(s01, dup2(b[jj][c]), acc[jj][0]);
+                acc[jj][1] = fma2_rn(s23, dup2(b[jj][c]), acc[jj][1]);
+            }
+        }
+    }
+#pragma unroll
+    for (int jj = 0; jj < kCols; ++jj) {
+        o[0][jj] = __fadd_rn(acc[jj][0].x, cc[jj]);
+        o[1][jj] = __fadd_rn(acc[jj][0].y, cc[jj]);
+        o[2][jj] = __fadd_rn(acc[jj][1].x, cc[jj]);
+        o[3][jj] = __fadd_rn(acc[jj][1].y, cc[jj]);
+    }
+}
+
+template <int D, bool kFinal, bool kScatter>
 __global__ void __launch_bounds__(32 * kWarpApplyWarps, VNLB_APPLY_MIN_BLOCKS) apply_warp_kernel(FilterLaunch L) {
     static_assert(D % 32 == 0, "columns are owned in blocks of 32");
     constexpr int kCols = D / 32;
@@ -1765,19 +1798,21 @@ __global__ void __launch_bounds__(32 * kWarpApplyWarps, VNLB_APPLY_MIN_BLOCKS) a
     const int warp = threadIdx.x >> 5;
     const int j8 = lane & 7;
     const int oct = lane >> 3;
-    const WarpApplyLayout lay = warp_apply_layout(D, L.max_rows, kScatter);
+    const WarpApplyLayout lay = warp_apply_layout(D, L.max_rows, kFinal, kScatter);
     int* coloff = reinterpret_cast<int*>(sm);
     float* wr = sm + D + warp * lay.per_warp;
-    float2* basis2 = reinterpret_cast<float2*>(wr + lay.basis);
-    const float* basis_f = wr + lay.basis;  // component c, column col at ((c & 3) * D + col) * 2 + (c >> 2)
-    float* u = wr + lay.u;
-    float* v = wr + lay.v;
-    float* dual = wr + lay.dual;
+    float* basis = wr + lay.basis;  // component c, column col at col * kWarpLdb + c
+    float* U = wr + lay.u;
+    float* V = wr + lay.v;
+    float* dual = wr + lay.dual;    // [sample][component]
     float* eig = wr + lay.scal;
     float* coef = eig + 8;
     float* denom = coef + 8;
     float* inv_sqrt = denom + 8;
     float* terms = inv_sqrt + 8;
+    float* quot = wr + lay.quot;
+    float* square = wr + lay.square;
+    float* norms = wr + lay.norms;
     float* scores = wr + lay.scores;
     size_t* bases = reinterpret_cast<size_t*>(wr + lay.bases);
     for (int col = threadIdx.x; col < D; col += blockDim.x) coloff[col] = column_offset(L, col);
@@ -1785,21 +1820,25 @@ __global__ void __launch_bounds__(32 * kWarpApplyWarps, VNLB_APPLY_MIN_BLOCKS) a
     const int Bmax = bmax_of(L);
     const int R = L.rank;
     const StageConfig& P = L.cfg;
-    const bool final_stage = L.stage == 1;
-    const float* model_video = final_stage ? L.basic : L.noisy;
+    const float* model_video = kFinal ? L.basic : L.noisy;
     const bool weights_enabled = P.weight_alpha != 0.0f || P.weight_beta != 0.0f || P.weight_gamma != 0.0f;
     const float sigma2 = __fmul_rn(__fmul_rn(P.beta, P.sigma), P.sigma);
-    const float model_noise2 = final_stage ? __fmul_rn(__fmul_rn(P.beta, P.sigma_basic), P.sigma_basic) : sigma2;
-    const float match_sigma = final_stage ? P.sigma_basic : P.sigma;
+    const float model_noise2 = kFinal ? __fmul_rn(__fmul_rn(P.beta, P.sigma_basic), P.sigma_basic) : sigma2;
+    const float match_sigma = kFinal ? P.sigma_basic : P.sigma;
     const float mem2 = std_max(__fmul_rn(match_sigma, match_sigma),
                                __fmul_rn(__fmul_rn(P.membership_noise_floor, P.sigma), P.sigma));
     const bool membership_on = P.weight_beta != 0.0f;
-    const bool need_dm = membership_on || !final_stage;
     const float score_scale = __fsqrt_rn(__fmul_rn(2.0f, static_cast<float>(D)));
     const int active_count = L.counters->active;
     const int models = L.models;  // models per group (planes when uncoupled)
     const size_t hw = static_cast<size_t>(L.height) * L.width;
+    const int q4 = 4 * (oct & 1), h = oct >> 1;          // this lane's component quad and row pair
+    const int row_l = 2 * h + (j8 >> 2);                 // ... and its row and component after the folds
+    const int comp_l = q4 + (j8 & 3);
     __syncthreads();
+    int off[kCols];
+#pragma unroll
+    for (int jj = 0; jj < kCols; ++jj) off[jj] = coloff[lane + 32 * jj];
 
     for (int mi = blockIdx.x * kWarpApplyWarps + warp; mi < active_count * models;
          mi += gridDim.x * kWarpApplyWarps) {
@@ -1837,101 +1876,96 @@ __global__ void __launch_bounds__(32 * kWarpApplyWarps, VNLB_APPLY_MIN_BLOCKS) a
             cc[jj] = __ldg(gm + D + lane + 32 * jj);
         }
         for (int i = lane; i < S; i += 32) bases[i] = row_base(L, rows[i]) + mc * hw;  // this model's plane
-        for (int i = lane; i < R * Bmax; i += 32) {
-            const int b = i / Bmax, s = i - b * Bmax;
-            dual[b * 8 + s] = L.dual[static_cast<size_t>(mi) * R * Bmax + i];
+        for (int i = lane; i < 64; i += 32) {
+            const int s = i >> 3, b = i & 7;
+            dual[i] = s < B && b < R ? L.dual[static_cast<size_t>(mi) * R * Bmax + b * Bmax + s] : 0.0f;
         }
-        if (lane < R) {
+        if (lane < 8) {
             const int c = lane;
-            const float lambda = L.eig[static_cast<size_t>(mi) * R + c];
+            const float lambda = c < R ? L.eig[static_cast<size_t>(mi) * R + c] : 0.0f;
             eig[c] = lambda;
             const float diff = __fsub_rn(lambda, model_noise2);
             const float signal = diff > 0.0f ? diff : 0.0f;
             denom[c] = __fadd_rn(signal, mem2);
             inv_sqrt[c] = lambda > kEigenFloor ? __fdiv_rn(1.0f, __fsqrt_rn(lambda)) : 0.0f;
             terms[c] = (membership_on && signal > 0.0f) ? cr_log1pf(__fdiv_rn(signal, mem2)) : 0.0f;
-            const float sigma_basic2 = final_stage ? model_noise2 : sigma2;
+            const float sigma_basic2 = kFinal ? model_noise2 : sigma2;
             const float threshold = __fmul_rn(P.variance_threshold, sigma2);
             float variance = lambda;
             if (sigma_basic2 > 0.0f) variance = __fsub_rn(variance, std_min(variance, sigma_basic2));
-            coef[c] = variance > threshold ? __fdiv_rn(1.0f, __fadd_rn(1.0f, __fdiv_rn(sigma2, variance))) : 0.0f;
+            coef[c] = c < R && variance > threshold ? __fdiv_rn(1.0f, __fadd_rn(1.0f, __fdiv_rn(sigma2, variance)))
+                                                    : 0.0f;
         }
         __syncwarp();
 
-        if (R > 0) {
-            // dual -> primal basis over blocks of this lane's columns: the
-            // centred model rows of the block in registers, then every
-            // component's samples accumulated in order (all columns fused)
-            float* bf = wr + lay.basis;
+        // dual -> primal basis over blocks of this lane's columns: the centred
+        // model rows of the block in registers, then every component's samples
+        // accumulated in order (all columns fused); components at or below the
+        // floor are zero
+        {
             constexpr int kBlk = kCols % 3 == 0 ? 3 : (kCols % 2 == 0 ? 2 : 1);
 #pragma unroll
             for (int j0 = 0; j0 < kCols; j0 += kBlk) {
-                float xr[8][kBlk];
+                float2 acc[kBlk][4];
 #pragma unroll
-                for (int s = 0; s < 8; ++s) {
-                    if (s < B) {
-                        const float* src = model_video + bases[s];
+                for (int jj = 0; jj < kBlk; ++jj)
 #pragma unroll
-                        for (int jj = 0; jj < kBlk; ++jj)
-                            xr[s][jj] = __fsub_rn(__ldg(src + coloff[lane + 32 * (j0 + jj)]), mm[j0 + jj]);
-                    } else {
+                    for (int p = 0; p < 4; ++p) acc[jj][p] = make_float2(0.0f, 0.0f);
+                float x[8][kBlk];
 #pragma unroll
-                        for (int jj = 0; jj < kBlk; ++jj) xr[s][jj] = 0.0f;
-                    }
-                }
-#pragma unroll
-                for (int b = 0; b < 8; ++b) {
-                    if (b >= R) break;
-                    const bool live = eig[b] > kEigenFloor;
-                    float acc[kBlk];
-#pragma unroll
-                    for (int jj = 0; jj < kBlk; ++jj) acc[jj] = 0.0f;
-                    if (live) {
-#pragma unroll
-                        for (int s = 0; s < 8; ++s) {
-                            if (s >= B) break;
-                            const float w = dual[b * 8 + s];
-#pragma unroll
-                            for (int jj = 0; jj < kBlk; ++jj) acc[jj] = __fmaf_rn(w, xr[s][jj], acc[jj]);
-                        }
-                        const float is = inv_sqrt[b];
-#pragma unroll
-                        for (int jj = 0; jj < kBlk; ++jj) acc[jj] = __fmul_rn(acc[jj], is);
-                    }
+                for (int s = 0; s < 8; ++s)
 #pragma unroll
                     for (int jj = 0; jj < kBlk; ++jj)
-                        bf[((b & 3) * D + lane + 32 * (j0 + jj)) * 2 + (b >> 2)] = acc[jj];
+                        x[s][jj] = s < B ? __ldg(model_video + bases[s] + off[j0 + jj]) : mm[j0 + jj];
+#pragma unroll
+                for (int s = 0; s < 8; ++s) {
+                    if (s >= B) break;
+                    const float4 w0 = *reinterpret_cast<const float4*>(dual + 8 * s);
+                    const float4 w1 = *reinterpret_cast<const float4*>(dual + 8 * s + 4);
+#pragma unroll
+                    for (int jj = 0; jj < kBlk; ++jj) {
+                        const float2 xx = dup2(__fsub_rn(x[s][jj], mm[j0 + jj]));
+                        acc[jj][0] = fma2_rn(make_float2(w0.x, w0.y), xx, acc[jj][0]);
+                        acc[jj][1] = fma2_rn(make_float2(w0.z, w0.w), xx, acc[jj][1]);
+                        acc[jj][2] = fma2_rn(make_float2(w1.x, w1.y), xx, acc[jj][2]);
+                        acc[jj][3] = fma2_rn(make_float2(w1.z, w1.w), xx, acc[jj][3]);
+                    }
+                }
+#pragma unroll
+                for (int jj = 0; jj < kBlk; ++jj) {
+                    float4* out = reinterpret_cast<float4*>(basis + (lane + 32 * (j0 + jj)) * kWarpLdb);
+#pragma unroll
+                    for (int p = 0; p < 2; ++p)
+                        out[p] = make_float4(__fmul_rn(acc[jj][2 * p].x, inv_sqrt[4 * p]),
+                                             __fmul_rn(acc[jj][2 * p].y, inv_sqrt[4 * p + 1]),
+                                             __fmul_rn(acc[jj][2 * p + 1].x, inv_sqrt[4 * p + 2]),
+                                             __fmul_rn(acc[jj][2 * p + 1].y, inv_sqrt[4 * p + 3]));
                 }
             }
-            __syncwarp();
-            // unit norm: octet k normalises components k and k + 4
-            {
-                float2 nv = make_float2(0.0f, 0.0f);
-                const float2* row = basis2 + oct * D;
-#pragma unroll
-                for (int m = 0; m < kChain; ++m) {
-                    const float2 x = row[j8 + 8 * m];
-                    nv = fma2_rn(x, x, nv);
-                }
-                nv = octet_reduce2(nv);
-                const float n0 = __shfl_sync(0xffffffffu, nv.x, oct * 8);
-                const float n1 = __shfl_sync(0xffffffffu, nv.y, oct * 8);
-                const int c0 = oct, c1 = oct + 4;
-                const bool live0 = c0 < R && eig[c0] > kEigenFloor;
-                const bool live1 = c1 < R && eig[c1] > kEigenFloor;
-                const float s0 = live0 && !(n0 <= kEigenFloor) ? __fdiv_rn(1.0f, __fsqrt_rn(n0)) : 0.0f;
-                const float s1 = live1 && !(n1 <= kEigenFloor) ? __fdiv_rn(1.0f, __fsqrt_rn(n1)) : 0.0f;
-                float2* wrow = basis2 + oct * D;
-#pragma unroll
-                for (int m = 0; m < kChain; ++m) {
-                    float2 x = wrow[j8 + 8 * m];
-                    if (live0) x.x = n0 <= kEigenFloor ? 0.0f : __fmul_rn(x.x, s0);
-                    if (live1) x.y = n1 <= kEigenFloor ? 0.0f : __fmul_rn(x.y, s1);
-                    wrow[j8 + 8 * m] = x;
-                }
-            }
-            __syncwarp();
         }
+        __syncwarp();
+        // unit norm: octet k normalises components k and k + 4
+        {
+            float2 nv = make_float2(0.0f, 0.0f);
+            float* col = basis + j8 * kWarpLdb + oct;
+#pragma unroll 8
+            for (int m = 0; m < kChain; ++m) {
+                const float2 x = make_float2(col[m * 8 * kWarpLdb], col[m * 8 * kWarpLdb + 4]);
+                nv = fma2_rn(x, x, nv);
+            }
+            const float n0 = octet_fold(nv.x), n1 = octet_fold(nv.y);
+            const bool none0 = !(oct < R && eig[oct] > kEigenFloor) || n0 <= kEigenFloor;
+            const bool none1 = !(oct + 4 < R && eig[oct + 4] > kEigenFloor) || n1 <= kEigenFloor;
+            const float s0 = none0 ? 0.0f : __fdiv_rn(1.0f, __fsqrt_rn(n0));
+            const float s1 = none1 ? 0.0f : __fdiv_rn(1.0f, __fsqrt_rn(n1));
+#pragma unroll 8
+            for (int m = 0; m < kChain; ++m) {
+                float* at = col + m * 8 * kWarpLdb;
+                at[0] = none0 ? 0.0f : __fmul_rn(at[0], s0);
+                at[4] = none1 ? 0.0f : __fmul_rn(at[4], s1);
+            }
+        }
+        __syncwarp();
         // group precision and volume, component order (every lane, uniform)
         float lgw, volume;
         {
@@ -1950,135 +1984,133 @@ __global__ void __launch_bounds__(32 * kWarpApplyWarps, VNLB_APPLY_MIN_BLOCKS) a
             volume = __fdiv_rn(vol, static_cast<float>(D));
         }
 
-        // rows: membership score and reconstruction; the next row's samples are
-        // loaded while the current one is reduced
+        // rows in tiles of four: membership scores and reconstruction
         float min_score = kInf;
-        float nx[kCols], nb[kCols];
-        if (S > 0) {
-#pragma unroll
-            for (int jj = 0; jj < kCols; ++jj) {
-                const size_t off = bases[0] + coloff[lane + 32 * jj];
-                nx[jj] = __ldg(L.noisy + off);
-                nb[jj] = final_stage ? __ldg(L.basic + off) : 0.0f;
-            }
-        }
-        for (int i = 0; i < S; ++i) {
-#pragma unroll
-            for (int jj = 0; jj < kCols; ++jj) {
-                const int col = lane + 32 * jj;
-                if (final_stage) {
-                    u[col] = __fsub_rn(nb[jj], mm[jj]);
-                    v[col] = __fsub_rn(nx[jj], cc[jj]);
-                } else {
-                    u[col] = __fsub_rn(nx[jj], mm[jj]);
-                }
-            }
-            if (i + 1 < S) {
+        for (int t0 = 0; t0 < S; t0 += 4) {
+            const int nrows = min(4, S - t0);
+            {
+                // a missing row repeats the first
+                const size_t b0 = bases[t0], b1 = bases[t0 + (nrows > 1 ? 1 : 0)];
+                const size_t b2 = bases[t0 + (nrows > 2 ? 2 : 0)], b3 = bases[t0 + (nrows > 3 ? 3 : 0)];
 #pragma unroll
                 for (int jj = 0; jj < kCols; ++jj) {
-                    const size_t off = bases[i + 1] + coloff[lane + 32 * jj];
-                    nx[jj] = __ldg(L.noisy + off);
-                    nb[jj] = final_stage ? __ldg(L.basic + off) : 0.0f;
-                }
-            }
-            __syncwarp();
-            // octet chains: norm of u, u . basis and (Final) v . basis for
-            // components oct and oct + 4
-            float nrm = 0.0f;
-            float2 pm = make_float2(0.0f, 0.0f), pr = make_float2(0.0f, 0.0f);
-            const float2* brow = basis2 + oct * D;
-#pragma unroll 8
-            for (int m = 0; m < kChain; ++m) {
-                const int e = j8 + 8 * m;
-                const float ue = u[e];
-                if (membership_on) nrm = __fmaf_rn(ue, ue, nrm);
-                if (R > 0) {
-                    const float2 bb = brow[e];
-                    if (need_dm) pm = fma2_rn(make_float2(ue, ue), bb, pm);
-                    if (final_stage) {
-                        const float ve = v[e];
-                        pr = fma2_rn(make_float2(ve, ve), bb, pr);
+                    const float* nz = L.noisy + off[jj];
+                    const float x0 = __ldg(nz + b0), x1 = __ldg(nz + b1), x2 = __ldg(nz + b2), x3 = __ldg(nz + b3);
+                    float4* u4 = reinterpret_cast<float4*>(U) + lane + 32 * jj;
+                    if constexpr (kFinal) {
+                        const float* bs = L.basic + off[jj];
+                        const float y0 = __ldg(bs + b0), y1 = __ldg(bs + b1), y2 = __ldg(bs + b2), y3 = __ldg(bs + b3);
+                        *u4 = make_float4(__fsub_rn(y0, mm[jj]), __fsub_rn(y1, mm[jj]), __fsub_rn(y2, mm[jj]),
+                                          __fsub_rn(y3, mm[jj]));
+                        reinterpret_cast<float4*>(V)[lane + 32 * jj] =
+                            make_float4(__fsub_rn(x0, cc[jj]), __fsub_rn(x1, cc[jj]), __fsub_rn(x2, cc[jj]),
+                                        __fsub_rn(x3, cc[jj]));
+                    } else {
+                        *u4 = make_float4(__fsub_rn(x0, mm[jj]), __fsub_rn(x1, mm[jj]), __fsub_rn(x2, mm[jj]),
+                                          __fsub_rn(x3, mm[jj]));
                     }
                 }
             }
-            if (membership_on) nrm = octet_reduce(nrm);
-            if (need_dm) pm = octet_reduce2(pm);
-            if (final_stage) pr = octet_reduce2(pr);
-            // lane c < R gathers component c from its octet leader
-            const int src = 8 * (lane & 3);
-            const bool hi = (lane & 4) != 0;
-            float mk = 0.0f, rk = 0.0f;
-            {
-                const float tx = __shfl_sync(0xffffffffu, pm.x, src);
-                const float ty = __shfl_sync(0xffffffffu, pm.y, src);
-                mk = hi ? ty : tx;
-                if (final_stage) {
-                    const float qx = __shfl_sync(0xffffffffu, pr.x, src);
-                    const float qy = __shfl_sync(0xffffffffu, pr.y, src);
-                    rk = hi ? qy : qx;
-                } else {
-                    rk = mk;
-                }
-            }
-            if (membership_on) {
-                const float norm2 = __shfl_sync(0xffffffffu, nrm, 0);
-                const float proj2 = __fmul_rn(mk, mk);
-                const float q = lane < R ? __fdiv_rn(proj2, denom[lane]) : 0.0f;
-                float distance = 0.0f, projected = 0.0f;
-                for (int c = 0; c < R; ++c) {
-                    distance = __fadd_rn(distance, __shfl_sync(0xffffffffu, q, c));
-                    projected = __fadd_rn(projected, __shfl_sync(0xffffffffu, proj2, c));
-                }
-                const float res = __fsub_rn(norm2, projected);
-                distance = __fadd_rn(distance, __fdiv_rn(res > 0.0f ? res : 0.0f, mem2));
-                const float score = __fdiv_rn(__fsub_rn(distance, static_cast<float>(D)), score_scale);
-                if (lane == 0) scores[i] = score;
-                min_score = std_min(min_score, score);
-            }
-            // reconstruction (project_bayes_estimate), components in order
-            const float scaled = lane < R ? __fmul_rn(coef[lane], rk) : 0.0f;
-            if constexpr (kScatter) {
-                // kept for the pass after the weights
-                if (lane < 8) wr[lay.recon + i * 8 + lane] = scaled;
-                __syncwarp();
-            } else {
-            float o[kCols];
-#pragma unroll
-            for (int jj = 0; jj < kCols; ++jj) o[jj] = 0.0f;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                if (c >= R) break;
-                const float sc = __shfl_sync(0xffffffffu, scaled, c);
-                if (coef[c] == 0.0f) continue;
-#pragma unroll
-                for (int jj = 0; jj < kCols; ++jj)
-                    o[jj] = __fmaf_rn(sc, basis_f[((c & 3) * D + lane + 32 * jj) * 2 + (c >> 2)], o[jj]);
-            }
-            float* out = L.filtered + static_cast<size_t>(r0 + i) * L.row_dim + mc * D;
-#pragma unroll
-            for (int jj = 0; jj < kCols; ++jj) out[lane + 32 * jj] = __fadd_rn(o[jj], cc[jj]);
             __syncwarp();
+            // chains of rows 2 h, 2 h + 1 against components q4 .. q4 + 3
+            float2 am[2][2], ar[2][2], an = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int p = 0; p < 2; ++p) am[i][p] = ar[i][p] = make_float2(0.0f, 0.0f);
+            const float* bp = basis + j8 * kWarpLdb + q4;
+            const float* up = U + 4 * j8 + 2 * h;
+            const float* vp = V + 4 * j8 + 2 * h;
+#pragma unroll 8
+            for (int m = 0; m < kChain; ++m) {
+                const float4 b = *reinterpret_cast<const float4*>(bp + m * 8 * kWarpLdb);
+                const float2 b01 = make_float2(b.x, b.y), b23 = make_float2(b.z, b.w);
+                const float2 u = *reinterpret_cast<const float2*>(up + m * 32);
+                am[0][0] = fma2_rn(dup2(u.x), b01, am[0][0]);
+                am[0][1] = fma2_rn(dup2(u.x), b23, am[0][1]);
+                am[1][0] = fma2_rn(dup2(u.y), b01, am[1][0]);
+                am[1][1] = fma2_rn(dup2(u.y), b23, am[1][1]);
+                an = fma2_rn(u, u, an);
+                if constexpr (kFinal) {
+                    const float2 v = *reinterpret_cast<const float2*>(vp + m * 32);
+                    ar[0][0] = fma2_rn(dup2(v.x), b01, ar[0][0]);
+                    ar[0][1] = fma2_rn(dup2(v.x), b23, ar[0][1]);
+                    ar[1][0] = fma2_rn(dup2(v.y), b01, ar[1][0]);
+                    ar[1][1] = fma2_rn(dup2(v.y), b23, ar[1][1]);
+                }
+            }
+            // fold: row by bit 2 of j8, component by bits 1 and 0 (the
+            // additions of reduce8: xor 4, then 2, then 1)
+            const auto fold = [&](const float2 (&v)[2][2]) {
+                const bool hi = j8 & 4;
+                float2 r[2];
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    r[p].x = fold_half(hi ? v[1][p].x : v[0][p].x, hi ? v[0][p].x : v[1][p].x, 4);
+                    r[p].y = fold_half(hi ? v[1][p].y : v[0][p].y, hi ? v[0][p].y : v[1][p].y, 4);
+                }
+                const bool second = j8 & 2;
+                const float x = fold_half(second ? r[1].x : r[0].x, second ? r[0].x : r[1].x, 2);
+                const float y = fold_half(second ? r[1].y : r[0].y, second ? r[0].y : r[1].y, 2);
+                return fold_half((j8 & 1) ? y : x, (j8 & 1) ? x : y, 1);
+            };
+            const float mk = fold(am);
+            float rk = mk;
+            if constexpr (kFinal) rk = fold(ar);
+            float* sc = kScatter ? wr + lay.recon + 8 * t0 : wr + lay.proj;  // [component][row]
+            sc[comp_l * 4 + row_l] = __fmul_rn(coef[comp_l], rk);
+            if (membership_on) {
+                const float p2 = __fmul_rn(mk, mk);
+                square[8 * row_l + comp_l] = p2;
+                quot[8 * row_l + comp_l] = __fdiv_rn(p2, denom[comp_l]);
+                float n = fold_half((j8 & 4) ? an.y : an.x, (j8 & 4) ? an.x : an.y, 4);
+                n = __fadd_rn(n, __shfl_xor_sync(0xffffffffu, n, 2));
+                n = __fadd_rn(n, __shfl_xor_sync(0xffffffffu, n, 1));
+                if (q4 == 0 && (j8 & 3) == 0) norms[row_l] = n;
+                __syncwarp();
+                if (lane < nrows) {
+                    float distance = 0.0f, projected = 0.0f;
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        if (c >= R) break;
+                        distance = __fadd_rn(distance, quot[8 * lane + c]);
+                        projected = __fadd_rn(projected, square[8 * lane + c]);
+                    }
+                    const float res = __fsub_rn(norms[lane], projected);
+                    distance = __fadd_rn(distance, __fdiv_rn(res > 0.0f ? res : 0.0f, mem2));
+                    const float score = __fdiv_rn(__fsub_rn(distance, static_cast<float>(D)), score_scale);
+                    scores[t0 + lane] = score;
+                    min_score = std_min(min_score, score);
+                }
+            }
+            __syncwarp();
+            if constexpr (!kScatter) {
+                float o[4][kCols];
+                warp_reconstruct<kCols>(basis, sc, coef, R, lane, cc, o);
+                float* out = L.filtered + static_cast<size_t>(r0 + t0) * L.row_dim + mc * D + lane;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (i >= nrows) break;
+#pragma unroll
+                    for (int jj = 0; jj < kCols; ++jj) out[static_cast<size_t>(i) * L.row_dim + 32 * jj] = o[i][jj];
+                }
+                __syncwarp();
             }
         }
+        // each of lanes 0-3 holds the least score of its rows
+        min_score = std_min(min_score, __shfl_xor_sync(0xffffffffu, min_score, 1));
+        min_score = std_min(min_score, __shfl_xor_sync(0xffffffffu, min_score, 2));
+        min_score = __shfl_sync(0xffffffffu, min_score, 0);
         // aggregation weights (accumulate_aggregation_model + finalize)
         for (int i = lane; i < S; i += 32) {
+            const float lw0 = model_log_weight(P, membership_on, lgw, volume, scores[i], min_score);
             if (models > 1) {
-                L.logw[static_cast<size_t>(r0 + i) * models + mc] =
-                    model_log_weight(P, membership_on, lgw, volume, scores[i], min_score);
+                L.logw[static_cast<size_t>(r0 + i) * models + mc] = lw0;
                 continue;
             }
             float w = 1.0f;
             if (weights_enabled) {
-                float lw;
-                if (P.weight_alpha == 0.0f && P.weight_beta == 0.0f) {
-                    lw = 0.0f;
-                } else if (membership_on) {
-                    const float diff = __fsub_rn(scores[i], min_score);
-                    const float membership = __fadd_rn(diff > 0.0f ? diff : 0.0f, volume);
-                    lw = __fadd_rn(0.0f, __fsub_rn(lgw, __fmul_rn(P.weight_beta, membership)));
-                } else {
-                    lw = __fadd_rn(0.0f, lgw);
-                }
+                float lw = __fadd_rn(0.0f, lw0);
                 lw = lw < -80.0f ? -80.0f : (80.0f < lw ? 80.0f : lw);
                 w = cr_expf(lw);
             }
@@ -2089,23 +2121,14 @@ __global__ void __launch_bounds__(32 * kWarpApplyWarps, VNLB_APPLY_MIN_BLOCKS) a
         if constexpr (kScatter) {
             // each row rebuilt from its scaled projections and added into the
             // stack with its weight
-            for (int i = 0; i < S; ++i) {
-                const float* sc = wr + lay.recon + i * 8;
-                float o[kCols];
+            for (int t0 = 0; t0 < S; t0 += 4) {
+                float o[4][kCols];
+                warp_reconstruct<kCols>(basis, wr + lay.recon + 8 * t0, coef, R, lane, cc, o);
 #pragma unroll
-                for (int jj = 0; jj < kCols; ++jj) o[jj] = 0.0f;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    if (c >= R) break;
-                    if (coef[c] == 0.0f) continue;
-                    const float scv = sc[c];
-#pragma unroll
-                    for (int jj = 0; jj < kCols; ++jj)
-                        o[jj] = __fmaf_rn(scv, basis_f[((c & 3) * D + lane + 32 * jj) * 2 + (c >> 2)], o[jj]);
+                for (int i = 0; i < 4; ++i) {
+                    if (t0 + i >= S) break;
+                    scatter_row(L, rows[t0 + i], o[i], wr[lay.rw + t0 + i], lane);
                 }
-#pragma unroll
-                for (int jj = 0; jj < kCols; ++jj) o[jj] = __fadd_rn(o[jj], cc[jj]);
-                scatter_row(L, rows[i], o, wr[lay.rw + i], lane);
             }
             __syncwarp();
         }
@@ -2174,9 +2197,11 @@ cudaError_t launch_jacobi_small(const FilterLaunch& L, int max_groups, cudaStrea
 template <int D>
 cudaError_t launch_apply_warp(const FilterLaunch& L, int max_groups, cudaStream_t stream) {
     const bool scatter = L.scatter != nullptr;
-    const WarpApplyLayout lay = warp_apply_layout(D, L.max_rows, scatter);
+    const bool final_stage = L.stage == 1;
+    const WarpApplyLayout lay = warp_apply_layout(D, L.max_rows, final_stage, scatter);
     const size_t smem = (static_cast<size_t>(D) + static_cast<size_t>(kWarpApplyWarps) * lay.per_warp) * sizeof(float);
-    auto kernel = scatter ? apply_warp_kernel<D, true> : apply_warp_kernel<D, false>;
+    auto kernel = final_stage ? (scatter ? apply_warp_kernel<D, true, true> : apply_warp_kernel<D, true, false>)
+                              : (scatter ? apply_warp_kernel<D, false, true> : apply_warp_kernel<D, false, false>);
     cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(kernel), static_cast<int>(smem));
     if (err != cudaSuccess) return err;
     const int ctas = std::max(1, std::min((max_groups + kWarpApplyWarps - 1) / kWarpApplyWarps, 148 * 8));
@@ -2197,6 +2222,17 @@ int tile_apply_warps(const FilterLaunch& L) {
                                     .bytes) <= kFilterSharedLimit)
             return warps;
     return 0;
+}
+
+// The shapes of the warp-per-group apply, as far as its block's shared memory
+// goes (thousands of rows per group do not fit).
+bool warp_apply_shape(const FilterLaunch& L, bool scatter) {
+    const int D = L.dim;
+    const int Bmax = std::min(L.model_cap, L.max_rows);
+    if (L.rank > 8 || Bmax > 8 || L.nmax != Bmax || (D != 64 && D != 128 && D != 192 && D != 256)) return false;
+    const WarpApplyLayout lay = warp_apply_layout(D, L.max_rows, L.stage == 1, scatter);
+    return (static_cast<size_t>(D) + static_cast<size_t>(kWarpApplyWarps) * lay.per_warp) * sizeof(float) <=
+           kFilterSharedLimit;
 }
 
 }  // namespace
@@ -2233,12 +2269,7 @@ size_t filter_shared_bytes(const FilterLaunch& L) {
 
 size_t filter_shared_limit() { return kFilterSharedLimit; }
 
-bool filter_can_scatter(const FilterLaunch& L) {
-    const int D = L.dim;
-    const int Bmax = std::min(L.model_cap, L.max_rows);
-    return L.models == 1 && L.rank <= 8 && Bmax <= 8 && L.nmax == Bmax &&
-           (D == 64 || D == 128 || D == 192 || D == 256);
-}
+bool filter_can_scatter(const FilterLaunch& L) { return L.models == 1 && warp_apply_shape(L, true); }
 
 int filter_scatter_pack(const FilterLaunch& L) {
     if (!filter_can_scatter(L)) return 0;
@@ -2308,7 +2339,7 @@ cudaError_t launch_filter(const FilterLaunch& L, int max_groups_in, cudaStream_t
 #ifndef VNLB_APPLY_WARP
 #define VNLB_APPLY_WARP 1  // the warp-per-group apply for its shapes; a build parameter for comparisons
 #endif
-    const bool warp_shape = R <= 8 && Bmax <= 8 && L.nmax == Bmax && (D == 64 || D == 128 || D == 192 || D == 256);
+    const bool warp_shape = warp_apply_shape(L, L.scatter != nullptr);
     if (L.scatter && !(warp_shape && L.models == 1)) return cudaErrorInvalidValue;  // see filter_can_scatter
     if (L.scatter && L.scatter_pack != 0 &&
         (L.scatter_pack != filter_scatter_pack(L) ||
