@@ -125,9 +125,10 @@ typedef struct vnlbgpu_stats {
     long long active_groups;   /* groups filtered (after the paste mask) */
     long long rows;            /* retained rows filtered and aggregated */
     long long kernel_launches; /* kernels this session launched */
-    long long pipeline_lanes;  /* anchor frames the session keeps in flight (1-8, fewer
-                                  when their group buffers would exceed half of the free
-                                  device memory at create time) */
+    long long pipeline_lanes;  /* anchor frames the session keeps in flight (1-8, at most
+                                  the clip's anchor frames, and fewer when their group
+                                  buffers would exceed half of the free device memory at
+                                  create time) */
     long long source_slots;    /* frames each source store holds on the device */
     long long source_uploads;  /* source frames copied to the device */
     long long learned_tiles;   /* learned form: tiles checked against the full search */

@@ -55,20 +55,48 @@ void check(cudaError_t status, const char* what) {
 template <typename T> struct DeviceArray {
     T* ptr = nullptr;
     size_t count = 0;
+    bool owned = true;  // false: a part of an Arena
     DeviceArray() = default;
     DeviceArray(const DeviceArray&) = delete;
     DeviceArray& operator=(const DeviceArray&) = delete;
     ~DeviceArray() { release(); }
     void release() {
-        if (ptr) cudaFree(ptr);
+        if (ptr && owned) cudaFree(ptr);
         ptr = nullptr;
         count = 0;
+        owned = true;
     }
     void allocate(size_t n, const char* what) {
         release();
         if (n == 0) return;
         check(cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T)), what);
         count = n;
+    }
+};
+
+// Arrays that live and die together in one device allocation: `lay` names them
+// twice, first to add up their sizes, then to place them.  An allocation and a
+// free cost tens of microseconds each, and a lane has some twenty arrays.
+struct Arena {
+    DeviceArray<unsigned char> block;
+    size_t used = 0;
+    template <typename T> void take(DeviceArray<T>& array, size_t n) {
+        constexpr size_t kAlign = 256;
+        used = (used + kAlign - 1) / kAlign * kAlign;
+        if (block.ptr && n > 0) {
+            array.release();
+            array.ptr = reinterpret_cast<T*>(block.ptr + used);
+            array.count = n;
+            array.owned = false;
+        }
+        used += n * sizeof(T);
+    }
+    template <typename Fn> void lay(Fn&& fn, const char* what) {
+        used = 0;
+        fn();
+        block.allocate(used, what);
+        used = 0;
+        fn();
     }
 };
 
@@ -375,6 +403,7 @@ struct Session {
     // device memory, so that a Basic session leaves room for its Final.
     struct Lane {
         cudaStream_t stream = nullptr;
+        Arena arena;  // the arrays below, but for the search centres and the network's
         DeviceArray<MatchRow> rows, row_info;
         DeviceArray<int2> centers;  // flow-guided search: [anchor][scheduled frame]
         DeviceArray<int> row_counts, victims, victim_counts, active, row_offset, row_group, active_prefix, gflags;
@@ -716,7 +745,7 @@ struct Session {
         stream = own_stream;
 
         // largest grid over the anchor phases
-        for (int key = 0; key < step; ++key) max_groups = std::max(max_groups, static_cast<int>(build_anchor_list(key).size()));
+        for (int key = 0; key < step; ++key) max_groups = std::max(max_groups, anchor_count(key));
         victim_stride = std::max(8, max_rows * 5);
         // match region geometry
         const int KY = 4;
@@ -787,34 +816,37 @@ struct Session {
             R * (sizeof(MatchRow) + sizeof(int)) +
             M * (2 * static_cast<size_t>(dim) + N * N + rank1 + rank1 * N) * sizeof(float) + M * sizeof(int);
         lane_count = static_cast<int>(std::min<size_t>(kMaxLanes, free_bytes / 2 / std::max<size_t>(lane_bytes, 1)));
+        lane_count = std::min(lane_count, valid_anchor_frames);  // a lane holds an anchor frame
         if (lane_count < 1) fail("VNLB CUDA: the group buffers of one anchor frame do not fit in device memory");
         lanes_allocated = lane_count;
         for (int li = 0; li < lane_count; ++li) {
             Lane& l = lanes[li];
             check(cudaStreamCreateWithFlags(&l.stream, cudaStreamNonBlocking), "cudaStreamCreate(lane)");
-            l.rows.allocate(G * max_rows, "cudaMalloc(match rows)");
-            l.row_counts.allocate(G, "cudaMalloc(row counts)");
-            l.victims.allocate(G * victim_stride, "cudaMalloc(victims)");
-            l.victim_counts.allocate(G, "cudaMalloc(victim counts)");
-            l.active.allocate(G, "cudaMalloc(active groups)");
-            l.active_xy.allocate(G, "cudaMalloc(active positions)");
-            l.row_offset.allocate(G + 1, "cudaMalloc(row offsets)");
-            l.active_prefix.allocate(G + 1, "cudaMalloc(active prefix)");
-            l.counters.allocate(1, "cudaMalloc(counters)");
-            if (chosen) {
-                l.approx.allocate(G * approx_stride, "cudaMalloc(approximate distances)");
-                l.tc_mu.allocate(G * kChosenMaxPlanes, "cudaMalloc(strip offsets)");  // a strip has an anchor
-            }
-            l.filtered.allocate(R * row_dim, "cudaMalloc(filtered rows)");
-            l.gmeans.allocate(M * 2 * dim, "cudaMalloc(group means)");
-            l.gram.allocate(M * N * N, "cudaMalloc(group Gram)");
-            l.eig.allocate(M * std::max(1, p.rank), "cudaMalloc(group eigenvalues)");
-            l.dual.allocate(M * std::max(1, p.rank) * N, "cudaMalloc(group eigenvectors)");
-            l.gflags.allocate(M, "cudaMalloc(group flags)");
-            if (models > 1) l.logw.allocate(R * models, "cudaMalloc(row log weights)");
-            l.weights.allocate(R, "cudaMalloc(row weights)");
-            l.row_info.allocate(R, "cudaMalloc(row info)");
-            l.row_group.allocate(R, "cudaMalloc(row groups)");
+            l.arena.lay(
+                [&] {
+                    l.arena.take(l.rows, G * max_rows);
+                    l.arena.take(l.row_counts, G);
+                    l.arena.take(l.victims, G * victim_stride);
+                    l.arena.take(l.victim_counts, G);
+                    l.arena.take(l.active, G);
+                    l.arena.take(l.active_xy, G);
+                    l.arena.take(l.row_offset, G + 1);
+                    l.arena.take(l.active_prefix, G + 1);
+                    l.arena.take(l.counters, 1);
+                    l.arena.take(l.approx, chosen ? G * approx_stride : 0);
+                    l.arena.take(l.tc_mu, chosen ? G * kChosenMaxPlanes : 0);  // a strip has an anchor
+                    l.arena.take(l.filtered, R * row_dim);
+                    l.arena.take(l.gmeans, M * 2 * dim);
+                    l.arena.take(l.gram, M * N * N);
+                    l.arena.take(l.eig, M * std::max(1, p.rank));
+                    l.arena.take(l.dual, M * std::max(1, p.rank) * N);
+                    l.arena.take(l.gflags, M);
+                    l.arena.take(l.logw, models > 1 ? R * models : 0);
+                    l.arena.take(l.weights, R);
+                    l.arena.take(l.row_info, R);
+                    l.arena.take(l.row_group, R);
+                },
+                "cudaMalloc(lane buffers)");
         }
         // learned form: network shape and per-lane buffers (the network's own
         // activations follow once one is attached)
@@ -916,15 +948,16 @@ struct Session {
             while (k1 < rows_n && row_y[k1] <= hi) ++k1;
             tgr[ty] = make_int2(k0, k1);
         }
-        for (int k = 0; k < rows_n; ++k)
+        for (int k = 0; k < rows_n; ++k) {
+            int j0 = row_first[k], j1 = row_first[k];  // both only move right along a row
             for (int tx = 0; tx < tiles_x; ++tx) {
                 const int lo = tx * kTile - (P - 1) - reach_x, hi = tx * kTile + kTile - 1 + reach_x;
-                int j0 = row_first[k];
                 while (j0 < row_first[k + 1] && a[j0].x < lo) ++j0;
-                int j1 = j0;
+                j1 = std::max(j1, j0);
                 while (j1 < row_first[k + 1] && a[j1].x <= hi) ++j1;
                 tan[static_cast<size_t>(k) * tiles_x + tx] = make_int2(j0, j1);
             }
+        }
         d_rows.allocate(tgr.size(), "cudaMalloc(tile rows)");
         d_anchors.allocate(tan.size(), "cudaMalloc(tile anchors)");
         check(cudaMemcpy(d_rows.ptr, tgr.data(), tgr.size() * sizeof(int2), cudaMemcpyHostToDevice),
@@ -949,6 +982,20 @@ struct Session {
             }
         }
         return out;
+    }
+
+    // the length of build_anchor_list(phase_key)
+    int anchor_count(int phase_key) const {
+        const int max_x = width - P, max_y = height - P;
+        int count = 0;
+        for (int y = 0; y <= max_y; ++y) {
+            if (!(y == 0 || y == max_y || y % step == phase_key % step)) continue;
+            const int phase = (y == max_y ? 0 : phase_key + (y / step)) % step;
+            // x = phase, phase + step, ...; then the two ends where they are not among them
+            count += (max_x >= phase ? (max_x - phase) / step + 1 : 0) + (phase != 0 ? 1 : 0) +
+                     (max_x > 0 && max_x % step != phase ? 1 : 0);
+        }
+        return count;
     }
 
     int grid_key(int anchor) const {
