@@ -10,15 +10,15 @@
 // (src/linalg/linalg.cpp).
 //
 // Three kernels, each shaped to its parallelism:
-//   prepare  one warp per group: equality and flat-area tests, the means of
-//            the first B rows, the centred model rows (shared memory) and the
-//            B x B dual Gram, one pair per lane;
-//   jacobi   the cyclic Jacobi of many groups per warp, one lane per matrix
-//            row (a latency-bound chain of dependent rotations, so throughput
+//   prepare  a warp or a CTA per group: equality and flat-area tests, the
+//            means of the first B rows, the centred model rows (shared memory)
+//            and the B x B dual Gram, a 4 x 4 block of pairs per octet of lanes;
+//   jacobi   the cyclic Jacobi of many groups per warp, a few lanes per group
+//            (a latency-bound chain of dependent rotations, so throughput
 //            comes from the number of groups in flight);
-//   apply    a warp or a CTA per group: dual -> primal basis, Wiener coefficients,
-//            precision and volume, then every retained row streamed once per
-//            warp for its membership score and its shrunken reconstruction,
+//   apply    a warp or a CTA per group: dual -> primal basis, Wiener
+//            coefficients, precision and volume, then the retained rows in
+//            tiles for their membership scores and shrunken reconstructions,
 //            and finally the aggregation weights.
 // Samples are addressed through a per-launch table of column offsets
 // (channel, t, py, px) -> video offset, so a gather is one add and one load.
@@ -41,6 +41,7 @@ constexpr int kApplyWarps = kApplyThreads / 32;
 constexpr int kRecCols = 8;  // reconstruction columns held in registers per lane (blocks of 256)
 constexpr int kPrepareWarps = 4;
 constexpr float kEigenFloor = 128.0f * FLT_EPSILON;
+constexpr int kTileRows = 4;       // rows of a tile of dot products
 constexpr size_t kFilterSharedLimit = 227 * 1024;  // dynamic shared memory of one CTA on sm_100
 
 // dot_contiguous_highway (the pinned 8-lane order) computed by an octet of
@@ -91,6 +92,37 @@ __device__ __forceinline__ size_t row_base(const FilterLaunch& L, const MatchRow
 }
 
 __device__ __forceinline__ int bmax_of(const FilterLaunch& L) { return min(L.model_cap, L.max_rows); }
+
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+
+// One step of the halving fold: keeps `keep`, adds the partner's copy of it.
+__device__ __forceinline__ float fold_half(float keep, float send, int mask) {
+    return __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, mask));
+}
+
+// Folds the octet chains v[row][component]: lane j ends with row r =
+// (j & 4) / 2 + (j & 2) / 2 and components 2 (j & 1), 2 (j & 1) + 1.
+__device__ __forceinline__ float2 fold_tile(const float2 (&v)[kTileRows][2], int j) {
+    float2 a[2][2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const float2 lo = v[r][p], hi = v[r + 2][p];
+            a[r][p].x = fold_half((j & 4) ? hi.x : lo.x, (j & 4) ? lo.x : hi.x, 4);
+            a[r][p].y = fold_half((j & 4) ? hi.y : lo.y, (j & 4) ? lo.y : hi.y, 4);
+        }
+    float2 b[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        b[p].x = fold_half((j & 2) ? a[1][p].x : a[0][p].x, (j & 2) ? a[0][p].x : a[1][p].x, 2);
+        b[p].y = fold_half((j & 2) ? a[1][p].y : a[0][p].y, (j & 2) ? a[0][p].y : a[1][p].y, 2);
+    }
+    float2 c;
+    c.x = fold_half((j & 1) ? b[1].x : b[0].x, (j & 1) ? b[0].x : b[1].x, 1);
+    c.y = fold_half((j & 1) ? b[1].y : b[0].y, (j & 1) ? b[0].y : b[1].y, 1);
+    return c;
+}
 
 // One m16n8k8 TF32 tensor-core MMA with FP32 accumulation (row-major A,
 // column-major B): d += a * b.
@@ -158,10 +190,15 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
     const int Bmax = bmax_of(L);
     int* coloff = reinterpret_cast<int*>(sm);
     size_t* bases_all = reinterpret_cast<size_t*>(sm + ((D + 3) & ~3));  // kGroups * max_rows
-    const int ldx = D + 8;  // padded row stride: octets on different rows hit different banks
+    // model row s, column col at X[s * rs + col * cs]: rows at a padded stride
+    // (octets on different rows hit different banks), or, for the blocked dual
+    // Gram of a whole CTA, columns of ldc floats (PrepareColumns)
+    const int ldc = W > 1 ? L.gram_columns : 0;
+    const int rs = ldc > 0 ? 1 : D + 8, cs = ldc > 0 ? ldc : 1;
     const int slot = threadIdx.x / kT;          // this group's slot in the CTA
     const int t = threadIdx.x - slot * kT;      // thread within the group
-    float* X = reinterpret_cast<float*>(bases_all + kGroups * L.max_rows) + slot * Bmax * ldx;  // model rows
+    float* X = reinterpret_cast<float*>(bases_all + kGroups * L.max_rows + (ldc > 0 ? L.max_rows & 1 : 0)) +
+               slot * Bmax * (D + 8);  // model rows; columns start on 16 bytes
     size_t* bases = bases_all + slot * L.max_rows;
     for (int col = threadIdx.x; col < D; col += blockDim.x) coloff[col] = column_offset(L, col);
     __syncthreads();
@@ -311,10 +348,10 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
         for (int col = t; col < D; col += kT) {
             const float* src = model_video + cb + coloff[col];
 #pragma unroll 8
-            for (int s2 = 0; s2 < B; ++s2) X[s2 * ldx + col] = __ldg(src + bases[s2]);
+            for (int s2 = 0; s2 < B; ++s2) X[s2 * rs + col * cs] = __ldg(src + bases[s2]);
             float mm = 0.0f;
 #pragma unroll 8
-            for (int s2 = 0; s2 < B; ++s2) mm = __fadd_rn(mm, X[s2 * ldx + col]);
+            for (int s2 = 0; s2 < B; ++s2) mm = __fadd_rn(mm, X[s2 * rs + col * cs]);
             mm = __fmul_rn(mm, inv_b);
             float center = mm;  // Basic: noisy mean; Final flat: basic mean
             if (final_stage && !flat) {
@@ -327,7 +364,7 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
             means[col] = mm;
             means[D + col] = center;
 #pragma unroll 8
-            for (int s2 = 0; s2 < B; ++s2) X[s2 * ldx + col] = __fsub_rn(X[s2 * ldx + col], mm);
+            for (int s2 = 0; s2 < B; ++s2) X[s2 * rs + col * cs] = __fsub_rn(X[s2 * rs + col * cs], mm);
         }
         group_sync();
         if (L.rank > 0) {
@@ -335,7 +372,59 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
             float* gram = L.gram + static_cast<size_t>(v) * L.nmax * L.nmax;
             if (D >= 64 && B < D && L.mixed && W == 1 && B <= 16 && D % 8 == 0) {
                 // chosen forms: TF32 tensor-core Gram, FP32 accumulation
-                gram_tf32(X, ldx, B, D, scale, gram, lane);
+                gram_tf32(X, rs, B, D, scale, gram, lane);
+            } else if (W > 1 && ldc > 0) {
+                // dual Gram (compute_gram_centered) in blocks of 4 x 4 pairs, an
+                // octet per block: lane j runs the pinned chain j of the 16
+                // pairs on two 16-byte loads per step, and the folds leave it
+                // with row r and two columns of the block
+                const int quads = (B + 3) / 4;
+                const int blocks = quads * (quads + 1) / 2;
+                const int j = lane & 7;
+                const int full = D / kLanes;
+                const int r = ((j >> 2) << 1) | ((j >> 1) & 1), c2 = 2 * (j & 1);
+                for (int e0 = 0; e0 < blocks; e0 += kT / 8) {
+                    const int e = min(e0 + (t >> 3), blocks - 1);
+                    int qa = 0;
+                    while ((qa + 1) * (qa + 2) / 2 <= e) ++qa;
+                    const int qb = e - qa * (qa + 1) / 2;
+                    float2 acc[4][2];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = make_float2(0.0f, 0.0f);
+                    const float* xa = X + j * ldc + 4 * qa;
+                    const float* xb = X + j * ldc + 4 * qb;
+#pragma unroll 4
+                    for (int m = 0; m < full; ++m) {
+                        const float4 a4 = *reinterpret_cast<const float4*>(xa + m * kLanes * ldc);
+                        const float4 b4 = *reinterpret_cast<const float4*>(xb + m * kLanes * ldc);
+                        const float2 b01 = make_float2(b4.x, b4.y), b23 = make_float2(b4.z, b4.w);
+                        acc[0][0] = fma2_rn(dup2(a4.x), b01, acc[0][0]);
+                        acc[0][1] = fma2_rn(dup2(a4.x), b23, acc[0][1]);
+                        acc[1][0] = fma2_rn(dup2(a4.y), b01, acc[1][0]);
+                        acc[1][1] = fma2_rn(dup2(a4.y), b23, acc[1][1]);
+                        acc[2][0] = fma2_rn(dup2(a4.z), b01, acc[2][0]);
+                        acc[2][1] = fma2_rn(dup2(a4.z), b23, acc[2][1]);
+                        acc[3][0] = fma2_rn(dup2(a4.w), b01, acc[3][0]);
+                        acc[3][1] = fma2_rn(dup2(a4.w), b23, acc[3][1]);
+                    }
+                    float2 dot = fold_tile(acc, j);
+                    for (int idx = full * kLanes; idx < D; ++idx) {
+                        const float x = X[idx * ldc + 4 * qa + r];
+                        const float* y = X + idx * ldc + 4 * qb + c2;
+                        dot.x = __fadd_rn(dot.x, __fmul_rn(x, y[0]));
+                        dot.y = __fadd_rn(dot.y, __fmul_rn(x, y[1]));
+                    }
+                    const int row = 4 * qa + r;
+                    const float vals[2] = {__fmul_rn(scale, dot.x), __fmul_rn(scale, dot.y)};
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const int col = 4 * qb + c2 + q;
+                        if (row < B && col <= row && e0 + (t >> 3) < blocks) {
+                            gram[row * B + col] = vals[q];
+                            gram[col * B + row] = vals[q];
+                        }
+                    }
+                }
             } else if (D >= 64 && B < D) {
                 // dual Gram (compute_gram_centered): octet k takes pair e0 + k;
                 // lane j of the octet runs the pinned chain j (octet_dot8)
@@ -346,7 +435,7 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
                     int r = 0;
                     while ((r + 1) * (r + 2) / 2 <= e) ++r;
                     const int c = e - r * (r + 1) / 2;
-                    const float val = __fmul_rn(scale, octet_dot8(X + r * ldx, X + c * ldx, D, lane & 7));
+                    const float val = __fmul_rn(scale, octet_dot8(X + r * rs, X + c * rs, D, lane & 7));
                     if ((lane & 7) == 0 && e0 + oct < pairs) {
                         gram[r * B + c] = val;
                         gram[c * B + r] = val;
@@ -368,8 +457,8 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
                     const bool fused = fused_column(rem, D - r);
                     float acc = 0.0f;
                     for (int s2 = 0; s2 < B; ++s2) {
-                        const float left = X[s2 * ldx + r];
-                        const float x = X[s2 * ldx + c];
+                        const float left = X[s2 * rs + r];
+                        const float x = X[s2 * rs + c];
                         acc = fused ? __fmaf_rn(left, x, acc) : __fadd_rn(acc, __fmul_rn(left, x));
                     }
                     const float val = __fmul_rn(acc, scale);
@@ -1091,7 +1180,6 @@ __global__ void __launch_bounds__(kApplyThreads, 3) apply_kernel(FilterLaunch L)
 // components, and the unfused tail, the division by the component's
 // variance and the shrinkage follow there.  The reconstruction takes blocks of
 // 32 columns, one per lane and block, all components of a column in registers.
-constexpr int kTileRows = 4;
 constexpr int kTileWarps = 4;
 
 struct TileApplyLayout {
@@ -1120,8 +1208,6 @@ __host__ __device__ inline TileApplyLayout tile_apply_layout(int D, int Bmax, in
     a.bytes = off * static_cast<int>(sizeof(float));
     return a;
 }
-
-__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
 
 // Dual -> primal basis of kCols columns (tid + 128-strided) of one thread:
 // acc[c] += dual[c][s] * x_s[col], the samples in order, then the scale.
@@ -1256,35 +1342,6 @@ __device__ __forceinline__ void tile_reconstruct(const float* basis, int ldb, co
         if (nrows > 2) at[2 * row_stride] = __fadd_rn(o[k][1].x, mid);
         if (nrows > 3) at[3 * row_stride] = __fadd_rn(o[k][1].y, mid);
     }
-}
-
-// One step of the halving fold: keeps `keep`, adds the partner's copy of it.
-__device__ __forceinline__ float fold_half(float keep, float send, int mask) {
-    return __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, send, mask));
-}
-
-// Folds the octet chains v[row][component]: lane j ends with row r =
-// (j & 4) / 2 + (j & 2) / 2 and components 2 (j & 1), 2 (j & 1) + 1.
-__device__ __forceinline__ float2 fold_tile(const float2 (&v)[kTileRows][2], int j) {
-    float2 a[2][2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const float2 lo = v[r][p], hi = v[r + 2][p];
-            a[r][p].x = fold_half((j & 4) ? hi.x : lo.x, (j & 4) ? lo.x : hi.x, 4);
-            a[r][p].y = fold_half((j & 4) ? hi.y : lo.y, (j & 4) ? lo.y : hi.y, 4);
-        }
-    float2 b[2];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        b[p].x = fold_half((j & 2) ? a[1][p].x : a[0][p].x, (j & 2) ? a[0][p].x : a[1][p].x, 2);
-        b[p].y = fold_half((j & 2) ? a[1][p].y : a[0][p].y, (j & 2) ? a[0][p].y : a[1][p].y, 2);
-    }
-    float2 c;
-    c.x = fold_half((j & 1) ? b[1].x : b[0].x, (j & 1) ? b[0].x : b[1].x, 1);
-    c.y = fold_half((j & 1) ? b[1].y : b[0].y, (j & 1) ? b[0].y : b[1].y, 1);
-    return c;
 }
 
 template <int kQ, bool kFinal>
@@ -2291,14 +2348,30 @@ cudaError_t launch_filter(const FilterLaunch& L, int max_groups_in, cudaStream_t
         const size_t rows_bytes = static_cast<size_t>(Bmax) * (D + 8) * sizeof(float);
         const bool wide = rows_bytes > 8 * 1024;
         const int groups_per_cta = wide ? 1 : kPrepareWarps;
-        const size_t smem = (colpad + static_cast<size_t>(groups_per_cta) * Bmax * (D + 8)) * sizeof(float) +
-                            static_cast<size_t>(groups_per_cta) * L.max_rows * sizeof(size_t);
+        const size_t fixed = colpad * sizeof(float) +
+                             static_cast<size_t>(groups_per_cta) * L.max_rows * sizeof(size_t);
+        size_t smem = fixed + static_cast<size_t>(groups_per_cta) * Bmax * (D + 8) * sizeof(float);
+        // the blocked Gram's columns: an odd number of 16-byte units each, so
+        // that the 8 columns of a quarter warp start on different banks
+        // (without the odd unit, or in rows, where that does not fit)
+        FilterLaunch P = L;
+        P.gram_columns = 0;
+        if (wide && D >= 64 && Bmax < D) {
+            const int quads = (Bmax + 3) / 4;
+            for (int ldc : {4 * (quads | 1), 4 * quads}) {
+                const size_t bytes = fixed + (L.max_rows & 1) * sizeof(size_t) + static_cast<size_t>(D) * ldc * sizeof(float);
+                if (bytes > kFilterSharedLimit) continue;
+                P.gram_columns = ldc;
+                smem = bytes;
+                break;
+            }
+        }
         auto kernel = wide ? prepare_kernel<kPrepareWarps> : prepare_kernel<1>;
         cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(kernel),
                                                static_cast<int>(smem));
         if (err != cudaSuccess) return err;
         const int ctas = std::min((max_groups + groups_per_cta - 1) / groups_per_cta, 148 * 16);
-        kernel<<<ctas, 32 * kPrepareWarps, smem, stream>>>(L);
+        kernel<<<ctas, 32 * kPrepareWarps, smem, stream>>>(P);
         if ((err = cudaGetLastError()) != cudaSuccess) return err;
     }
     // jacobi

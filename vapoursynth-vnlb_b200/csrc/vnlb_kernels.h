@@ -207,6 +207,7 @@ struct FilterLaunch {
     int K, model_cap, rank, max_rows;
     int coupled;            // sample-major (coupled, C > 1) vs group path
     int models;             // models per group: 1, or the planes of an uncoupled clip
+    int gram_columns;       // set by launch_filter: prepare's model rows as columns of so many floats (0: rows)
     int nmax;               // largest eigen problem: model rows, or dim where a covariance model occurs
     int row_dim;            // filtered row width: patch_dim * planes (dim when coupled)
     int mixed;              // chosen forms: dual Gram on TF32 tensor cores (FP32 accumulation) and
