@@ -8,9 +8,9 @@
 //   1. approximate distance ||a||^2 + ||b||^2 - 2 a.b for every candidate:
 //      the dot products on the tensor cores (BF16 samples, FP32
 //      accumulation), the norms in FP32 from the FP32 samples;
-//   2. the CPU's sequential selection (find_similar_patches,
-//      core.cpp:1277-1359: the K-smallest front and the capped buffer) run on
-//      the approximate distances, frame by frame in the CPU's candidate order;
+//   2. the CPU's selection (find_similar_patches, core.cpp:1277-1359: the
+//      K-smallest front and the capped buffer) on the approximate distances,
+//      frame by frame in the CPU's candidate order;
 //   3. the exact FP32 SSD, in the CPU's arithmetic order (the bits the plain
 //      form computes), of every buffer entry a frame brings in;
 //   4. select_similar_patches (core.cpp:1200-1243) on those exact distances:
@@ -749,10 +749,204 @@ __device__ __forceinline__ float exact_distance(const MatchLaunch& L, const floa
 // Steps 2-4 for one anchor per warp, from the approximate distances.  The
 // capped buffer's slot s lives in lane s % 32, register s / 32 (CW registers:
 // buffers of up to 32 CW entries).
+// The CPU's sequential selection (find_similar_patches) on one anchor's
+// approximate distances, frame by frame in candidate order: the K-smallest
+// front and the capped buffer of up to 32 entries, slot i in lane i.  Returns
+// the entries; id is this lane's.
+__device__ __forceinline__ int select_replay(const MatchLaunch& L, const float* approx, int cells, int lane, int& id) {
+    constexpr int kSelectBatch = 8;  // chunks of 32 distances loaded at once
+    const int K = L.K;
+    const int cap = min(L.soft_cap, L.search_window * L.search_window * L.schedule_len);
+    int count = 0, worst_idx = 0, top_count = 0;
+    float worst = kInf, top_front = kInf;
+    unsigned reg_d = 0u, reg_top = 0u;  // bits of non-negative distances
+    id = 0;
+    const auto find_worst = [&] {  // the buffer's largest distance and its lowest slot
+        const unsigned m = __reduce_max_sync(0xffffffffu, reg_d);
+        worst = __uint_as_float(m);
+        worst_idx = __ffs(__ballot_sync(0xffffffffu, reg_d == m)) - 1;
+    };
+    const auto limit_now = [&] {
+        const float limit = top_count >= K ? std_max(L.tau, top_front) : kInf;
+        return count >= cap ? std_min(limit, worst) : limit;
+    };
+    for (int k = 0; k < L.schedule_len; ++k) {
+        const float* dk = approx + k * L.window_cells;
+        for (int base0 = 0; base0 < cells; base0 += 32 * kSelectBatch) {
+            float vals[kSelectBatch];
+#pragma unroll
+            for (int b = 0; b < kSelectBatch; ++b) {
+                const int idx = base0 + 32 * b + lane;
+                vals[b] = idx < cells ? __ldg(dk + idx) : kInf;
+            }
+#pragma unroll
+            for (int b = 0; b < kSelectBatch; ++b) {
+                const int base = base0 + 32 * b;
+                if (base >= cells) break;  // uniform
+                const float mine = vals[b];
+                unsigned pass = __ballot_sync(0xffffffffu, base + lane < cells && mine <= limit_now());
+                while (pass) {
+                    const int src_lane = __ffs(pass) - 1;
+                    pass &= pass - 1;
+                    const float d = __shfl_sync(0xffffffffu, mine, src_lane);
+                    if (!(d <= limit_now())) continue;
+                    const bool room = count < cap;
+                    if (room || d < worst) {
+                        if (lane == (room ? count : worst_idx)) {
+                            reg_d = __float_as_uint(d);
+                            id = (k << 20) | (base + src_lane);
+                        }
+                        if (room) ++count;
+                        if (count == cap) find_worst();
+                    }
+                    if (top_count < K) {
+                        if (lane == top_count) reg_top = __float_as_uint(d);
+                        if (++top_count == K) top_front = __uint_as_float(__reduce_max_sync(0xffffffffu, reg_top));
+                    } else if (d < top_front) {
+                        const unsigned f = __float_as_uint(top_front);
+                        const int owner = __ffs(__ballot_sync(0xffffffffu, lane < K && reg_top == f)) - 1;
+                        if (lane == owner) reg_top = __float_as_uint(d);
+                        top_front = __uint_as_float(__reduce_max_sync(0xffffffffu, reg_top));
+                    }
+                }
+            }
+        }
+    }
+    return count;
+}
+
+// The same selection for buffers of up to 32 CW entries: the front, and a log of
+// the candidates within the limit (the front's maximum, tau above it, and the
+// buffer's largest distance once it has been full).  The limit is taken once
+// per 32 candidates, which go into the log together; when the log is full, and
+// at the end, the buffer's capacity of smallest ones is kept, in candidate
+// order.  The replay, which moves the limit candidate by candidate and replaces
+// the buffer's worst entry each time, keeps the same ones, less those that
+// passed between two of its limits.  For buffers of 64 it costs less than
+// replacing the worst entry of several words at every record (57k anchors of
+// two and six planes 1.16 -> 0.82 and 1.55 -> 1.26 ms, 130k of two planes 2.08
+// -> 1.54 ms); for buffers of 32 the replay is the shorter one (33k anchors 246
+// against 465 us).
+template <int CW>
+__device__ __forceinline__ int select_log(const MatchLaunch& L, const float* approx, int cells, int lane, float* sd,
+                                          int* si, int (&id)[CW]) {
+    const int K = L.K;
+    const int cap = min(L.soft_cap, L.search_window * L.search_window * L.schedule_len);
+    int logged = 0, top_count = 0;
+    float top_front = kInf, worst = kInf;
+    unsigned reg_top = 0u;  // bits of non-negative distances order like them
+    constexpr int kLog = 64 * CW;  // entries of sd and si
+    const auto keep_smallest = [&] {
+        // the cap smallest of the log, by bisection on their bits
+        __syncwarp();
+        unsigned d[2 * CW];
+        int ids[2 * CW];
+        unsigned lo = 0xffffffffu, hi = 0u;
+#pragma unroll
+        for (int w = 0; w < 2 * CW; ++w) {
+            const int slot = 32 * w + lane;
+            d[w] = slot < logged ? __float_as_uint(sd[slot]) : 0xffffffffu;
+            ids[w] = slot < logged ? si[slot] : 0;
+            lo = min(lo, d[w]);
+            hi = max(hi, slot < logged ? d[w] : 0u);
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        // the cap-th smallest lies in [lo, hi]
+        int below = 0;  // entries under lo
+        while (lo < hi) {
+            const unsigned mid = lo + (hi - lo) / 2;
+            int count = 0;
+#pragma unroll
+            for (int w = 0; w < 2 * CW; ++w) count += __popc(__ballot_sync(0xffffffffu, d[w] <= mid));
+            if (count >= cap) {
+                hi = mid;
+            } else {
+                lo = mid + 1;
+                below = count;
+            }
+        }
+        __syncwarp();
+        int at = 0, equal = cap - below;  // entries equal to it that are kept, the first ones
+#pragma unroll
+        for (int w = 0; w < 2 * CW; ++w) {
+            const unsigned same = __ballot_sync(0xffffffffu, d[w] == lo);
+            const bool keep = d[w] < lo || (d[w] == lo && __popc(same & ((1u << lane) - 1u)) < equal);
+            const unsigned mask = __ballot_sync(0xffffffffu, keep);
+            if (keep) {
+                const int slot = at + __popc(mask & ((1u << lane) - 1u));
+                sd[slot] = __uint_as_float(d[w]);
+                si[slot] = ids[w];
+            }
+            at += __popc(mask);
+            equal -= min(equal, __popc(same));
+        }
+        __syncwarp();
+        logged = at;
+        worst = __uint_as_float(lo);
+    };
+
+    for (int k = 0; k < L.schedule_len; ++k) {
+        constexpr int kSelectBatch = 4;  // chunks of 32 distances loaded at once
+        const float* dk = approx + k * L.window_cells;
+        for (int base0 = 0; base0 < cells; base0 += 32 * kSelectBatch) {
+          float vals[kSelectBatch];
+#pragma unroll
+          for (int b = 0; b < kSelectBatch; ++b) {
+              const int idx = base0 + 32 * b + lane;
+              vals[b] = idx < cells ? __ldg(dk + idx) : kInf;
+          }
+#pragma unroll
+          for (int b = 0; b < kSelectBatch; ++b) {
+            const int base = base0 + 32 * b;
+            if (base >= cells) break;  // uniform
+            const int idx = base + lane;
+            const float mine = vals[b];
+            const float limit = fminf(top_count >= K ? std_max(L.tau, top_front) : kInf, worst);
+            const bool in = idx < cells && mine <= limit;
+            unsigned pass = __ballot_sync(0xffffffffu, in);
+            if (pass == 0u) continue;
+            if (logged + 32 > kLog) keep_smallest();
+            if (in) {
+                const int slot = logged + __popc(pass & ((1u << lane) - 1u));
+                sd[slot] = mine;
+                si[slot] = (k << 20) | idx;
+            }
+            logged += __popc(pass);
+            // the front takes the ones below its maximum
+            if (top_count >= K) pass &= __ballot_sync(0xffffffffu, mine < top_front);
+            while (pass) {
+                const int src_lane = __ffs(pass) - 1;
+                pass &= pass - 1;
+                const float d = __shfl_sync(0xffffffffu, mine, src_lane);
+                if (top_count < K) {
+                    if (lane == top_count) reg_top = __float_as_uint(d);
+                    if (++top_count < K) continue;
+                } else {
+                    if (!(d < top_front)) continue;
+                    const unsigned f = __float_as_uint(top_front);
+                    const int owner = __ffs(__ballot_sync(0xffffffffu, lane < K && reg_top == f)) - 1;
+                    if (lane == owner) reg_top = __float_as_uint(d);
+                }
+                top_front = __uint_as_float(__reduce_max_sync(0xffffffffu, reg_top));
+            }
+          }
+        }
+    }
+    if (logged > cap) keep_smallest();
+    __syncwarp();
+    const int n = logged;
+#pragma unroll
+    for (int w = 0; w < CW; ++w) id[w] = 32 * w + lane < n ? si[32 * w + lane] : 0;
+    __syncwarp();
+    return n;
+}
+
 template <int P, int CW>
 __global__ void __launch_bounds__(kTcThreads) tc_select_kernel(MatchLaunch L) {
-    __shared__ float sorted_d[kChosenWarps][32 * CW];
-    __shared__ int sorted_i[kChosenWarps][32 * CW];
+    constexpr int kSlots = CW == 1 ? 32 : 64 * CW;  // the sorted buffer, or select_log's log
+    __shared__ float sorted_d[kChosenWarps][kSlots];
+    __shared__ int sorted_i[kChosenWarps][kSlots];
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int gi = blockIdx.x * kChosenWarps + warp;
@@ -768,108 +962,20 @@ __global__ void __launch_bounds__(kTcThreads) tc_select_kernel(MatchLaunch L) {
     const float* approx = L.approx_dist + static_cast<size_t>(gi) * L.approx_stride;
     const float* anchor_frame = L.video + static_cast<size_t>(L.schedule[0] % L.ring) * L.channels * plane_values;
 
-    // selection state (the plain matcher's WarpSelect)
+    float* sd = sorted_d[warp];
+    int* si = sorted_i[warp];
     const int K = L.K;
-    struct {
-        int count, cap, worst_idx, top_count;
-        float worst, top_front;
-    } s;
-    s.count = 0;
-    s.cap = min(L.soft_cap, L.search_window * L.search_window * L.schedule_len);
-    s.worst_idx = 0;
-    s.worst = kInf;
-    s.top_count = 0;
-    s.top_front = kInf;
-    unsigned reg_d[CW], reg_top = 0u;  // bits of non-negative distances
     int reg_id[CW];
     float reg_exact[CW];
-#pragma unroll
-    for (int w = 0; w < CW; ++w) {
-        reg_d[w] = 0u;
-        reg_id[w] = 0;
-        reg_exact[w] = 0.0f;
-    }
-    // the buffer's largest distance and its lowest slot
-    auto find_worst = [&]() {
-        unsigned m = reg_d[0];
-#pragma unroll
-        for (int w = 1; w < CW; ++w) m = m > reg_d[w] ? m : reg_d[w];
-        const unsigned wmax = __reduce_max_sync(0xffffffffu, m);
-        s.worst = __uint_as_float(wmax);
-#pragma unroll
-        for (int w = CW - 1; w >= 0; --w) {
-            const unsigned hit = __ballot_sync(0xffffffffu, reg_d[w] == wmax);
-            if (hit) s.worst_idx = 32 * w + __ffs(hit) - 1;
-        }
-    };
-    auto put = [&](int slot, float d, int id) {
-#pragma unroll
-        for (int w = 0; w < CW; ++w)
-            if (slot >> 5 == w && lane == (slot & 31)) {
-                reg_d[w] = __float_as_uint(d);
-                reg_id[w] = id;
-            }
-    };
-
-    for (int k = 0; k < L.schedule_len; ++k) {
-        // the CPU's sequential selection over frame k (raster order) on the
-        // approximate distances: the K-smallest front and the capped buffer;
-        // kSelectBatch chunks of 32 candidates are loaded at once (the
-        // replay of a chunk is short next to a load's latency; fewer for the
-        // larger buffers, whose registers would spill)
-        constexpr int kSelectBatch = CW == 1 ? 8 : 4;
-        const float* dk = approx + k * L.window_cells;
-        for (int base0 = 0; base0 < cells; base0 += 32 * kSelectBatch) {
-          float vals[kSelectBatch];
-#pragma unroll
-          for (int b = 0; b < kSelectBatch; ++b) {
-              const int idx = base0 + 32 * b + lane;
-              vals[b] = idx < cells ? __ldg(dk + idx) : kInf;
-          }
-#pragma unroll
-          for (int b = 0; b < kSelectBatch; ++b) {
-            const int base = base0 + 32 * b;
-            if (base >= cells) break;  // uniform
-            const int idx = base + lane;
-            const float mine = vals[b];
-            float limit = s.top_count >= K ? std_max(L.tau, s.top_front) : kInf;
-            if (s.count >= s.cap) limit = std_min(limit, s.worst);
-            unsigned pass = __ballot_sync(0xffffffffu, idx < cells && mine <= limit);
-            while (pass) {
-                const int src_lane = __ffs(pass) - 1;
-                pass &= pass - 1;
-                const float d = __shfl_sync(0xffffffffu, mine, src_lane);
-                limit = s.top_count >= K ? std_max(L.tau, s.top_front) : kInf;
-                if (s.count >= s.cap) limit = std_min(limit, s.worst);
-                if (!(d <= limit)) continue;
-                const int id = (k << 20) | (base + src_lane);
-                if (s.count < s.cap) {
-                    put(s.count, d, id);
-                    s.count++;
-                    if (s.count == s.cap) find_worst();
-                } else if (d < s.worst) {
-                    put(s.worst_idx, d, id);
-                    find_worst();
-                }
-                if (s.top_count < K) {
-                    if (lane == s.top_count) reg_top = __float_as_uint(d);
-                    s.top_count++;
-                    if (s.top_count == K) s.top_front = __uint_as_float(__reduce_max_sync(0xffffffffu, reg_top));
-                } else if (d < s.top_front) {
-                    const unsigned f = __float_as_uint(s.top_front);
-                    const int owner = __ffs(__ballot_sync(0xffffffffu, lane < K && reg_top == f)) - 1;
-                    if (lane == owner) reg_top = __float_as_uint(d);
-                    s.top_front = __uint_as_float(__reduce_max_sync(0xffffffffu, reg_top));
-                }
-            }
-          }
-        }
-    }
+    int n;
+    if constexpr (CW == 1) n = select_replay(L, approx, cells, lane, reg_id[0]);
+    else n = select_log<CW>(L, approx, cells, lane, sd, si, reg_id);
     // exact FP32 distance of every entry left in the buffer, in the plain
     // form's arithmetic order: once, after the last frame
 #pragma unroll
     for (int w = 0; w < CW; ++w) {
-        if (32 * w + lane < s.count) {
+        reg_exact[w] = 0.0f;
+        if (32 * w + lane < n) {
             const int i = reg_id[w] & 0xfffff;
             const int cy = i / Wx;
             reg_exact[w] = exact_distance<P>(L, anchor_frame, anchor, L.schedule[reg_id[w] >> 20], yl + cy,
@@ -880,9 +986,6 @@ __global__ void __launch_bounds__(kTcThreads) tc_select_kernel(MatchLaunch L) {
     // select_similar_patches on the exact distances of the buffer: the K
     // smallest, the threshold max(tau, d_K), the entries within it, closest
     // first (ties by candidate order), at most the cap
-    float* sd = sorted_d[warp];
-    int* si = sorted_i[warp];
-    const int n = s.count;
     int S;
     if (K <= 1) {
         // similar <= 1: the anchor itself (core.cpp:1253-1257)
