@@ -5,162 +5,236 @@
 // (src/core/core.cpp:1851-1903, apply_frame_paste_mask at :980-1008).  The
 // match kernel has already turned every anchor's anchor-frame matches into the
 // list of later grid anchors they clear (its "victims"), so the mask only
-// needs one bit per grid anchor.
+// needs one bit per grid anchor, in shared memory.
 //
-// One warp walks the anchors in batches of 32 (lane k = anchor 32b+k): the
-// batch's alive word is resolved in order (an alive anchor clears its
-// in-batch victims), then alive anchors clear their later victims in the
-// shared bitmask, and the batch is compacted (ordered ballot) into the active
-// list with the exclusive prefix of retained rows.  The serial chain is
-// O(G/32) warp steps.  The other warps of the block stage the next chunk of
-// anchors (counts, rows, positions, first victims and each anchor's in-batch
-// victim mask) into shared memory while the walker resolves the current one,
-// so the walker reads only shared memory; one block barrier per chunk.
+// The order only binds anchors that can reach each other: a match lies within
+// reach_x columns of its anchor, so an anchor at x is decided once every
+// earlier grid row is decided up to x + reach_x.  One block walks the grid as
+// a wavefront: warp w takes grid rows w, w + 16, ... and goes along its row in
+// batches of 32 anchors, each batch after the row above has passed the reach
+// of the batch's last anchor (the rows further up are ahead of that row by the
+// same rule, so the row above is all a warp waits for).  A batch is resolved
+// in order among its own anchors (only those that name one another cost a
+// step), then its living anchors clear their later victims' bits.  The chain
+// is about two batches per grid row instead of every batch of the frame:
+// one walker over all batches took 390 us at 1920x1080 with step 8 (33k
+// anchors) and 1750 us at 960x540 with step 3 (57k anchors, more victims than
+// it held on chip); the wavefront takes 265 us and 590 us.
+//
+// The compaction (active list, exclusive prefix of retained rows, active
+// prefix per anchor) follows in two passes of the whole block over the bits.
 #include "vnlb_kernels.h"
 
 namespace vnlbgpu {
 namespace {
 
-constexpr int kPrefetch = 8;                   // victims staged per anchor
+constexpr int kHeld = 24;              // victims held in registers per anchor
 constexpr int kPasteThreads = 512;
-constexpr int kChunkBatches = 16;
-constexpr int kChunk = kChunkBatches * 32;     // anchors per staged chunk
-constexpr unsigned kLaterFlag = 1u << 30;      // in meta: a victim lies beyond the batch
+constexpr int kPasteWarps = kPasteThreads / 32;
+constexpr int kPasteSpinLimit = 1 << 22;  // polls of the row above before the walk gives up
 
-struct __align__(16) Chunk {
-    int meta[kChunk];           // victim count | kLaterFlag
-    int rows[kChunk];           // retained rows
-    unsigned mine[kChunk];      // in-batch victims, bit k = anchor 32b+k
-    int2 xy[kChunk];
-    int v[kPrefetch][kChunk];   // first victims, transposed
+// The victims of one batch's anchors, one anchor per lane.  A batch's counts
+// are loaded two batches ahead and the victims they name one batch ahead, so
+// that the walk waits for neither.
+struct PasteBatch {
+    int x, count;
+    int v[kHeld];
 };
 
-// Stages anchors [first, first + kChunk) with threads [t0, t0 + nt).
-__device__ __forceinline__ void stage_chunk(const PasteLaunch& L, Chunk& c, int first, int t0, int nt) {
-    for (int i = threadIdx.x - t0; i < kChunk; i += nt) {
-        const int j = first + i;
-        int n = 0, rows = 0;
-        int2 xy = make_int2(0, 0);
-        int v[kPrefetch];
-        if (j < L.groups) {
-            n = __ldg(L.victim_counts + j);
-            rows = __ldg(L.row_counts + j);
-            xy = __ldg(L.anchors + j);
-            // in bounds: every anchor owns victim_stride >= kPrefetch slots, so
-            // the first entries are loaded without waiting on the count
-            const int* vlist = L.victims + static_cast<size_t>(j) * L.victim_stride;
+__device__ __forceinline__ void load_counts(const PasteLaunch& L, int j, int end, int& x, int& count) {
+    x = j < end ? __ldg(&L.anchors[j].x) : 0;
+    count = j < end ? __ldg(L.victim_counts + j) : 0;
+}
+
+__device__ __forceinline__ void load_victims(const PasteLaunch& L, PasteBatch& b, int j) {
+    const int* list = L.victims + static_cast<size_t>(j) * L.victim_stride;
 #pragma unroll
-            for (int e = 0; e < kPrefetch; ++e) v[e] = __ldg(vlist + e);
-        }
-        const int batch_start = j & ~31;
-        unsigned mine = 0;
-        bool later = false;
-        if (j < L.groups) {
-            const int* vlist = L.victims + static_cast<size_t>(j) * L.victim_stride;
-            for (int e = 0; e < n; ++e) {
-                const int x = e < kPrefetch ? v[e] : __ldg(vlist + e);
-                if (x < batch_start + 32) mine |= 1u << (x - batch_start);
-                else later = true;
-            }
-        }
-        c.meta[i] = n | (later ? static_cast<int>(kLaterFlag) : 0);
-        c.rows[i] = rows;
-        c.mine[i] = mine;
-        c.xy[i] = xy;
-#pragma unroll
-        for (int e = 0; e < kPrefetch; ++e) c.v[e][i] = j < L.groups ? v[e] : 0;
-    }
+    for (int e = 0; e < kHeld; ++e) b.v[e] = e < b.count ? __ldg(list + e) : 0;
+}
+
+// Bits [j, j + 32) of the mask.
+__device__ __forceinline__ unsigned bits_at(const volatile unsigned* alive, int j, int words) {
+    const int w = j >> 5;
+    return __funnelshift_r(alive[w], w + 1 < words ? alive[w + 1] : 0u, j & 31);
+}
+
+// How far a warp's row has come, in shared memory: the row in the high half,
+// the column up to which all its anchors are decided in the low half.  The
+// release and acquire order the mask's bits around it; a fence in the polling
+// loop would also wait for the loads in flight.
+__device__ __forceinline__ void publish(unsigned long long* slot, int row, int x) {
+    const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(slot));
+    const unsigned long long v = static_cast<unsigned long long>(static_cast<unsigned>(row)) << 32 |
+                                 static_cast<unsigned>(x);
+    asm volatile("st.release.cta.shared::cta.u64 [%0], %1;" ::"r"(at), "l"(v) : "memory");
+}
+
+__device__ __forceinline__ unsigned long long progress(const unsigned long long* slot) {
+    const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(slot));
+    unsigned long long v;
+    asm volatile("ld.acquire.cta.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(at) : "memory");
+    return v;
 }
 
 __global__ void __launch_bounds__(kPasteThreads) paste_kernel(PasteLaunch L) {
-    extern __shared__ __align__(16) unsigned char paste_smem[];
-    Chunk* chunks = reinterpret_cast<Chunk*>(paste_smem);                 // two buffers
-    unsigned* alive = reinterpret_cast<unsigned*>(paste_smem + 2 * sizeof(Chunk));
+    extern __shared__ __align__(16) unsigned paste_smem[];
+    __shared__ unsigned long long passed[kPasteWarps];  // per row in flight
+    __shared__ int active_sum[kPasteWarps + 1], rows_sum[kPasteWarps + 1];
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
     const int words = (L.groups + 31) / 32;
-    const int nchunks = (L.groups + kChunk - 1) / kChunk;
+    unsigned* alive = paste_smem;
     for (int w = tid; w < words; w += kPasteThreads) {
         const int rem = L.groups - w * 32;
         alive[w] = rem >= 32 ? 0xffffffffu : ((1u << rem) - 1u);
     }
-    stage_chunk(L, chunks[0], 0, 0, kPasteThreads);
+    if (lane == 0) passed[warp] = static_cast<unsigned long long>(warp) << 32;  // its first row, nothing decided
     __syncthreads();
-
-    int running_active = 0;
-    int running_rows = 0;
-    for (int ci = 0; ci < nchunks; ++ci) {
-        if (warp != 0) {
-            if (ci + 1 < nchunks) stage_chunk(L, chunks[(ci + 1) & 1], (ci + 1) * kChunk, 32, kPasteThreads - 32);
-        } else {
-            const Chunk& c = chunks[ci & 1];
-            const int b_end = min(words, (ci + 1) * kChunkBatches);
-            for (int b = ci * kChunkBatches; b < b_end; ++b) {
-                const int base = (b - ci * kChunkBatches) * 32;
-                const int idx = base + lane;
-                const int j = b * 32 + lane;
-                const int batch_end = (b + 1) * 32;
-                const unsigned mine = c.mine[idx];
-                const int meta = c.meta[idx];
-                const int my_rows = c.rows[idx];
-                unsigned bits = alive[b];
-                if (__any_sync(0xffffffffu, mine != 0)) {
-                    // all 32 masks first (broadcast loads), then the ordered chain
-                    unsigned mk[32];
-                    const uint4* m4 = reinterpret_cast<const uint4*>(c.mine + base);
+    const unsigned long long* above = passed + (warp + kPasteWarps - 1) % kPasteWarps;
+    bool failed = false;
+    for (int row = warp; row < L.grid_rows; row += kPasteWarps) {
+        const int begin = L.row_first[row], end = L.row_first[row + 1];
+        PasteBatch b, next;
+        int x2, count2;
+        load_counts(L, begin + lane, end, b.x, b.count);
+        load_counts(L, begin + 32 + lane, end, next.x, next.count);
+        load_victims(L, b, begin + lane);
+        load_counts(L, begin + 64 + lane, end, x2, count2);
+        load_victims(L, next, begin + 32 + lane);
+        for (int j0 = begin; j0 < end; j0 += 32) {
+            const int j = j0 + lane;
+            const int n = min(32, end - j0);
+            // victims inside the batch, and whether there are later ones
+            unsigned mine = 0u;
+            bool later = false;
+            const int* list = L.victims + static_cast<size_t>(j) * L.victim_stride;
+            const int filled = static_cast<int>(__reduce_max_sync(0xffffffffu, b.count));
 #pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const uint4 t = m4[q];
-                        mk[4 * q] = t.x;
-                        mk[4 * q + 1] = t.y;
-                        mk[4 * q + 2] = t.z;
-                        mk[4 * q + 3] = t.w;
-                    }
-#pragma unroll
-                    for (int k = 0; k < 32; ++k)
-                        if ((bits >> k) & 1u) bits &= ~mk[k];
+            for (int e = 0; e < kHeld; ++e) {
+                if (e >= filled) break;  // uniform
+                if (e < b.count) {
+                    if (b.v[e] < j0 + n) mine |= 1u << (b.v[e] - j0);
+                    else later = true;
                 }
-                const bool me = j < L.groups && ((bits >> lane) & 1u);
-                if (me && (meta & static_cast<int>(kLaterFlag))) {
-                    const int n = meta & ~static_cast<int>(kLaterFlag);
-                    const int* vlist = L.victims + static_cast<size_t>(j) * L.victim_stride;
-                    for (int e = 0; e < n; ++e) {
-                        const int v = e < kPrefetch ? c.v[e][idx] : __ldg(vlist + e);
-                        if (v >= batch_end) atomicAnd(&alive[v >> 5], ~(1u << (v & 31)));
-                    }
+            }
+            for (int e = kHeld; e < b.count; ++e) {
+                const int v = __ldg(list + e);
+                if (v < j0 + n) mine |= 1u << (v - j0);
+                else later = true;
+            }
+            const int most = min(kHeld, static_cast<int>(__reduce_max_sync(0xffffffffu, later ? b.count : 0)));
+            const int last_x = __shfl_sync(0xffffffffu, b.x, n - 1);
+            const int next_x = __shfl_sync(0xffffffffu, next.x, 0);
+            // the row above has passed the reach of this batch's last anchor
+            if (row > 0) {
+                int spins = 0;
+                for (;;) {
+                    const unsigned long long p = progress(above);
+                    const int r = static_cast<int>(p >> 32), x = static_cast<int>(p & 0xffffffffu);
+                    if (r > row - 1 || (r == row - 1 && x > last_x + L.reach_x)) break;
+                    if (++spins >= kPasteSpinLimit) break;
                 }
-                // ordered compaction
-                const unsigned ballot = __ballot_sync(0xffffffffu, me);
-                const int rank = __popc(ballot & ((1u << lane) - 1u));
-                const int s = me ? my_rows : 0;
-                int prefix = s;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int v = __shfl_up_sync(0xffffffffu, prefix, o);
-                    if (lane >= o) prefix += v;
-                }
-                if (j < L.groups) L.active_prefix[j] = running_active + rank;
-                if (me) {
-                    const int a = running_active + rank;
-                    L.active[a] = j;
-                    L.active_xy[a] = c.xy[idx];
-                    L.row_offset[a] = running_rows + prefix - s;
-                }
-                running_active += __popc(ballot);
-                running_rows += __shfl_sync(0xffffffffu, prefix, 31);
+                failed |= spins >= kPasteSpinLimit;
                 __syncwarp();
             }
+            unsigned bits = bits_at(alive, j0, words);
+            if (n < 32) bits &= (1u << n) - 1u;
+            const unsigned before = bits;
+            for (unsigned m = __ballot_sync(0xffffffffu, mine != 0u); m; m &= m - 1) {
+                const int k = __ffs(m) - 1;
+                const unsigned kills = __shfl_sync(0xffffffffu, mine, k);
+                if ((bits >> k) & 1u) bits &= ~kills;
+            }
+            const unsigned dead = before & ~bits;
+            if (dead && lane < 2) {
+                const int sh = j0 & 31;
+                const unsigned part = lane == 0 ? dead << sh : (sh ? dead >> (32 - sh) : 0u);
+                if (part) atomicAnd(&alive[(j0 >> 5) + lane], ~part);
+            }
+            if (later && ((bits >> lane) & 1u)) {
+#pragma unroll
+                for (int e = 0; e < kHeld; ++e) {
+                    if (e >= most) break;  // uniform
+                    if (e < b.count && b.v[e] >= j0 + n) atomicAnd(&alive[b.v[e] >> 5], ~(1u << (b.v[e] & 31)));
+                }
+                for (int e = kHeld; e < b.count; ++e) {
+                    const int v = __ldg(list + e);
+                    if (v >= j0 + n) atomicAnd(&alive[v >> 5], ~(1u << (v & 31)));
+                }
+            }
+            __syncwarp();
+            if (lane == 0) publish(passed + warp, row, j0 + 32 < end ? next_x : 0x7fffffff);
+            // the batch after the next one
+            b = next;
+            next.x = x2;
+            next.count = count2;
+            load_victims(L, next, j + 64);
+            load_counts(L, j + 96, end, x2, count2);
         }
-        __syncthreads();
+        // this warp's next row: nothing of it is decided
+        if (row + kPasteWarps < L.grid_rows && lane == 0) publish(passed + warp, row + kPasteWarps, 0);
+    }
+    if (__syncthreads_or(failed)) {
+        if (tid == 0) atomicCAS(L.status, 0, kStatusPasteTimeout);
+    }
+    // compaction: a contiguous range of words per warp, first the sums ...
+    const int per_warp = (words + kPasteWarps - 1) / kPasteWarps;
+    const int w0 = warp * per_warp, w1 = min(words, w0 + per_warp);
+    int active = 0, rows = 0;
+#pragma unroll 4
+    for (int w = w0; w < w1; ++w) {
+        const unsigned bits = alive[w];
+        active += __popc(bits);
+        if ((bits >> lane) & 1u) rows += __ldg(L.row_counts + 32 * w + lane);
+    }
+    rows = __reduce_add_sync(0xffffffffu, rows);
+    if (lane == 0) {
+        active_sum[warp + 1] = active;
+        rows_sum[warp + 1] = rows;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        active_sum[0] = rows_sum[0] = 0;
+        for (int w = 1; w <= kPasteWarps; ++w) {
+            active_sum[w] += active_sum[w - 1];
+            rows_sum[w] += rows_sum[w - 1];
+        }
+    }
+    __syncthreads();
+    // ... then the positions
+    int running_active = active_sum[warp], running_rows = rows_sum[warp];
+#pragma unroll 2
+    for (int w = w0; w < w1; ++w) {
+        const unsigned bits = alive[w];
+        const int j = 32 * w + lane;
+        const bool me = (bits >> lane) & 1u;
+        const int s = me ? __ldg(L.row_counts + j) : 0;
+        const int rank = __popc(bits & ((1u << lane) - 1u));
+        int prefix = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, prefix, o);
+            if (lane >= o) prefix += v;
+        }
+        if (j < L.groups) L.active_prefix[j] = running_active + rank;
+        if (me) {
+            const int a = running_active + rank;
+            L.active[a] = j;
+            L.active_xy[a] = __ldg(L.anchors + j);
+            L.row_offset[a] = running_rows + prefix - s;
+        }
+        running_active += __popc(bits);
+        running_rows += __shfl_sync(0xffffffffu, prefix, 31);
     }
     if (tid == 0) {
-        L.row_offset[running_active] = running_rows;
-        L.active_prefix[L.groups] = running_active;
-        L.counters->active = running_active;
-        L.counters->rows = running_rows;
-        atomicAdd(L.totals, static_cast<unsigned long long>(running_active));
-        atomicAdd(L.totals + 1, static_cast<unsigned long long>(running_rows));
+        const int total_active = active_sum[kPasteWarps], total_rows = rows_sum[kPasteWarps];
+        L.row_offset[total_active] = total_rows;
+        L.active_prefix[L.groups] = total_active;
+        L.counters->active = total_active;
+        L.counters->rows = total_rows;
+        atomicAdd(L.totals, static_cast<unsigned long long>(total_active));
+        atomicAdd(L.totals + 1, static_cast<unsigned long long>(total_rows));
     }
 }
 
@@ -180,8 +254,8 @@ cudaError_t launch_anchor_map(const int2* anchors, int count, int width, int* ma
 }
 
 cudaError_t launch_paste(const PasteLaunch& L, cudaStream_t stream) {
-    const size_t smem = 2 * sizeof(Chunk) + static_cast<size_t>((L.groups + 31) / 32) * sizeof(unsigned);
-    if (smem > 227 * 1024) return cudaErrorInvalidValue;  // more grid anchors than the bitmask holds
+    const size_t smem = static_cast<size_t>((L.groups + 31) / 32) * sizeof(unsigned);
+    if (smem > 175 * 1024) return cudaErrorInvalidValue;  // more grid anchors than the bitmask holds
     cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(paste_kernel),
                                            static_cast<int>(smem));
     if (err != cudaSuccess) return err;

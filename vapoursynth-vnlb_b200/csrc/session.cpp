@@ -126,6 +126,8 @@ struct Grid {
     DeviceArray<Strip> d_strips;
     DeviceArray<TcStrip> d_strips_chosen;
     DeviceArray<int> d_map;  // [H][W] anchor index or -1
+    DeviceArray<int> d_row_first;  // first anchor of each grid row, then their number
+    int rows = 0;                  // grid rows
     // stack-tile reach tables (TileLaunch)
     DeviceArray<int2> d_tile_grid_rows;  // [tiles_y]
     DeviceArray<int2> d_tile_anchors;    // [grid rows][tiles_x]
@@ -1098,6 +1100,15 @@ struct Session {
                              grid->strips_chosen.size() * sizeof(TcStrip), cudaMemcpyHostToDevice),
                   "cudaMemcpy(strips)");
         }
+        std::vector<int> row_first;
+        for (size_t k = 0; k < a.size(); ++k)
+            if (k == 0 || a[k].y != a[k - 1].y) row_first.push_back(static_cast<int>(k));
+        grid->rows = static_cast<int>(row_first.size());
+        row_first.push_back(static_cast<int>(a.size()));
+        grid->d_row_first.allocate(row_first.size(), "cudaMalloc(grid rows)");
+        check(cudaMemcpy(grid->d_row_first.ptr, row_first.data(), row_first.size() * sizeof(int),
+                         cudaMemcpyHostToDevice),
+              "cudaMemcpy(grid rows)");
         grid->d_anchors.allocate(a.size(), "cudaMalloc(anchors)");
         grid->d_strips.allocate(grid->strips.size(), "cudaMalloc(strips)");
         check(cudaMemcpy(grid->d_anchors.ptr, a.data(), a.size() * sizeof(int2), cudaMemcpyHostToDevice),
@@ -1579,6 +1590,12 @@ struct Session {
         pl.victim_counts = lane.victim_counts.ptr;
         pl.victim_stride = victim_stride;
         pl.anchors = grid.d_anchors.ptr;
+        pl.row_first = grid.d_row_first.ptr;
+        pl.grid_rows = grid.rows;
+        // a match lies within search_window - 1 columns of its anchor (plus the
+        // search centre's way), and clears its neighbours' bits too
+        pl.reach_x = params.search_window + (flow_on() ? flow_reach.x : 0);
+        pl.status = d_status.ptr;
         pl.active = lane.active.ptr;
         pl.active_xy = lane.active_xy.ptr;
         pl.row_offset = lane.row_offset.ptr;
@@ -1910,6 +1927,8 @@ struct Session {
                 fail("VNLB CUDA: the tensor-core matcher timed out waiting for its MMAs");
             if (status == kStatusTmaTimeout)
                 fail("VNLB CUDA: the matcher timed out waiting for a tensor-memory-accelerator load");
+            if (status == kStatusPasteTimeout)
+                fail("VNLB CUDA: the paste mask timed out waiting for the grid row above");
             if (status == kStatusLogitsTimeout)
                 fail("VNLB CUDA: the network's tensor-core output layer timed out waiting for its MMAs");
             fail("VNLB CUDA: device status " + std::to_string(status));

@@ -174,6 +174,7 @@ constexpr int kStatusRankNotCovered = 1;  // fewer model rows than the rank
 constexpr int kStatusPasteCapacity = 2;   // too many anchors for the paste kernel
 constexpr int kStatusTensorTimeout = 3;   // an MMA completion wait ran out (tensor-core matcher)
 constexpr int kStatusTmaTimeout = 4;      // a tensor-memory-accelerator load wait ran out (plain matcher)
+constexpr int kStatusPasteTimeout = 6;    // the paste walk's wait for the grid row above ran out
 
 struct PasteLaunch {
     int groups;
@@ -182,6 +183,10 @@ struct PasteLaunch {
     const int* victim_counts;
     int victim_stride;
     const int2* anchors;
+    const int* row_first; // [grid_rows + 1] first anchor of each grid row
+    int grid_rows;
+    int reach_x;          // a victim lies within this many columns of its anchor
+    int* status;          // session status word
     // outputs
     int* active;          // [G] active anchor indices in raster order
     int2* active_xy;      // [G] their positions
