@@ -8,9 +8,11 @@ the row tiles, ranks and matrix sizes on both sides of each kernel's range.
 import numpy as np
 import pytest
 
+import mlp_fp64
 import oracle as O
 import synth
-from test_gpu_parity import bits, gpu_chain
+import vnlbgpu_lib as lib
+from test_gpu_parity import bits, gpu_chain, session_for
 
 pytestmark = pytest.mark.gpu
 
@@ -42,9 +44,42 @@ APPLY_TILES = [
 # rows), with fewer rows than the matrix they are stored in
 JACOBI = [(k, r) for k, r in ((1, 1), (2, 2), (7, 7), (8, 8), (9, 4), (15, 15), (23, 23), (24, 24), (25, 25), (31, 8))]
 
+# buffers of one, two and four words per lane and larger ones, fronts of up to
+# 32 and more, block sizes with and without a kernel of their own
+MATCH = [
+    ("buffer32", 48, 40, 3, 1, dict(group_size=8, rank=8, tau=3000.0)),
+    ("buffer33", 48, 40, 3, 1, dict(group_size=11, rank=8, cap_factor=3.0, tau=3000.0)),
+    ("buffer64", 48, 40, 3, 1, dict(patch_time=2, group_size=16, rank=8, tau=5000.0)),
+    ("buffer128", 48, 40, 3, 1, dict(patch_time=2, group_size=32, rank=8, tau=9000.0)),
+    ("buffer129", 48, 40, 3, 1, dict(patch_time=2, group_size=32, rank=8, cap_factor=4.03, tau=9000.0)),
+    ("front33", 48, 40, 3, 1, dict(patch_time=2, group_size=33, rank=8, cap_factor=1.5, tau=5000.0)),
+    ("block10", 53, 41, 3, 1, dict(block_size=10, block_step=5, patch_time=2, group_size=16, rank=15, tau=2000.0)),
+    ("block9", 48, 40, 3, 1, dict(block_size=9, patch_time=2, group_size=12, rank=8, tau=2000.0)),
+    ("block5_tau", 48, 40, 3, 1, dict(block_size=5, group_size=16, rank=8, tau=1200.0)),
+    # four planes and more: later planes from the list, from every candidate, and of none
+    ("planes6", 64, 48, 4, 3, dict(block_size=7, block_step=5, patch_time=2, bm_range=13, group_size=16, rank=15)),
+    ("planes6_all", 64, 48, 3, 3, dict(block_size=7, block_step=7, patch_time=2, group_size=16, rank=8, tau=90000.0)),
+    ("planes6_block10", 48, 40, 3, 3, dict(block_size=10, block_step=9, patch_time=2, group_size=16, rank=8)),
+    ("planes5", 48, 40, 7, 1, dict(patch_time=5, group_size=40, rank=8, cap_factor=1.0)),
+    # windows clipped to a few candidates
+    ("tiny_frame", 10, 9, 2, 1, dict(group_size=8, rank=2, block_step=2)),
+]
 
-def check(w, h, f, planes, sigma, kw, seed):
-    _, noisy = synth.make_clip(w, h, f, planes, sigma, seed=seed)
+# dense and sparse grids (step against window), many slots, odd planes
+GRIDS = [
+    ("step1", 40, 32, 2, 1, dict(block_size=6, block_step=1, group_size=8, rank=6, bm_range=4)),
+    ("step16_window5", 90, 70, 2, 1, dict(block_step=16, group_size=6, rank=4, bm_range=2)),
+    ("wide", 700, 17, 2, 1, dict(block_step=3, group_size=8, rank=6, bm_range=3)),
+    ("tall", 19, 400, 2, 1, dict(block_step=3, group_size=8, rank=6, bm_range=3)),
+    ("slots6", 45, 37, 6, 3, dict(patch_time=2, radius=2, group_size=12, rank=8, block_step=6)),
+    ("slots9_uncoupled", 45, 37, 9, 3, dict(radius=4, group_size=8, rank=6, bm_range=4, chroma=0)),
+    ("window_off", 45, 37, 3, 3, dict(weight_gamma=0.0, patch_time=2, group_size=12, rank=8)),
+]
+
+
+def check(w, h, f, planes, sigma, kw, seed, noisy=None):
+    if noisy is None:
+        _, noisy = synth.make_clip(w, h, f, planes, sigma, seed=seed)
     bp = O.cpu_params(O.BASIC, sigma, **kw)
     fp = O.cpu_params(O.FINAL, sigma, **kw)
     oracle = O.Oracle("port")
@@ -53,6 +88,12 @@ def check(w, h, f, planes, sigma, kw, seed):
     assert np.array_equal(bits(basic_stacks), bits(oracle.stage_stacks(O.BASIC, bp, noisy)))
     assert np.array_equal(bits(basic), bits(want_basic))
     assert np.array_equal(bits(final), bits(want_final))
+    # the same frames normalised on the device
+    for stage, p, ref, want in ((lib.STAGE_BASIC, bp, None, want_basic), (lib.STAGE_FINAL, fp, want_basic, want_final)):
+        s = session_for(stage, p, noisy, ref)
+        got = s.render_clip()
+        s.close()
+        assert np.array_equal(bits(got), bits(want))
 
 
 @pytest.mark.parametrize("name,w,h,f,planes,kw", APPLY_TILES, ids=[c[0] for c in APPLY_TILES])
@@ -63,3 +104,48 @@ def test_apply_row_tiles(name, w, h, f, planes, kw):
 @pytest.mark.parametrize("k,rank", JACOBI)
 def test_jacobi_sizes(k, rank):
     check(48, 40, 3, 1, 20.0, dict(patch_time=2, group_size=k, rank=rank, cap_factor=1.0), seed=k)
+
+
+@pytest.mark.parametrize("name,w,h,f,planes,kw", MATCH, ids=[c[0] for c in MATCH])
+def test_match_selection(name, w, h, f, planes, kw):
+    check(w, h, f, planes, 15.0, kw, seed=len(name) + 40)
+
+
+@pytest.mark.parametrize("planes,patch_time,tau", [(1, 1, 0.0), (1, 1, 400.0), (3, 2, 0.0)])
+def test_match_ties(planes, patch_time, tau):
+    """Flat areas and repeated columns: most distances tie, many at zero."""
+    rng = np.random.default_rng(planes + 10 * patch_time)
+    noisy = np.full((4, planes, 40, 48), 0.5, np.float32)
+    noisy[:, :, :, 24:] = np.tile(rng.random((4, planes, 40, 4)).astype(np.float32), (1, 1, 1, 6))
+    noisy[:, :, 8:14, 4:12] = rng.random((4, planes, 6, 8)).astype(np.float32)
+    check(48, 40, 4, planes, 10.0, dict(patch_time=patch_time, group_size=12, rank=8, tau=tau, block_step=5), 0, noisy)
+
+
+@pytest.mark.parametrize("name,w,h,f,planes,kw", GRIDS, ids=[c[0] for c in GRIDS])
+def test_grids_and_tiles(name, w, h, f, planes, kw):
+    check(w, h, f, planes, 15.0, kw, seed=len(name) + 70)
+
+
+@pytest.mark.parametrize("batch,inputs,hidden,layers,outputs", [
+    (1, 3, 5, 1, 7), (63, 45, 128, 3, 65), (129, 27, 64, 2, 1083), (300, 45, 128, 3, 5445), (700, 16, 16, 1, 16)])
+def test_network_products(batch, inputs, hidden, layers, outputs):
+    """Products with whole tiles, remainders and splits, against float64.  A
+    product sums at most 5445 terms in FP32: their rounding stays under
+    5445 * 2^-24 = 3.3e-4 of the sum of magnitudes."""
+    import torch
+
+    rng = np.random.default_rng(batch)
+    shape = (inputs, hidden, layers, outputs)
+    net = lib.MLP(*shape, max_batch=batch, seed=batch)
+    x = rng.normal(0.0, 1.0, (batch, inputs)).astype(np.float32)
+    t = rng.integers(0, outputs, (batch, 8)).astype(np.int32)
+    dx, dt = torch.from_numpy(x).cuda(), torch.from_numpy(t).cuda()
+    out = torch.empty((batch, outputs), device="cuda")
+    torch.cuda.synchronize()
+    grads, loss = net.gradients(dx.data_ptr(), dt.data_ptr(), batch, 8)
+    net.logits(dx.data_ptr(), batch, out.data_ptr())
+    want_loss, want = mlp_fp64.loss_and_gradients(net.get_weights(), shape, x, t)
+    z = mlp_fp64.forward_logits(net.get_weights(), shape, x)
+    assert abs(loss - want_loss) <= 3.3e-4 * max(1.0, abs(want_loss))
+    assert np.abs(grads - want).max() <= 3.3e-4 * np.abs(want).max()
+    assert np.abs(out.cpu().numpy() - z).max() <= 3.3e-4 * np.abs(z).max()
