@@ -140,25 +140,25 @@ __device__ __forceinline__ uint32_t to_tf32(float x) {
     return r;
 }
 
-// Dual Gram X X^T / B of up to 16 centred rows (row stride ldx, D a multiple
-// of 8) on the tensor cores, one warp: A = the rows (16 x 8 per step), B =
+// Dual Gram X X^T / B of up to 16 centred rows (row r, column k at X[r * rs + k *
+// cs], D a multiple of 8) on the tensor cores, one warp: A = the rows (16 x 8 per step), B =
 // their transpose in tiles of 8 columns; rows and columns past B are zero.
 // Lane (g, q) = (lane / 4, lane % 4) holds A rows g, g + 8 at columns q, q + 4
 // and the accumulators of rows g, g + 8 at columns 2q, 2q + 1.
-__device__ __forceinline__ void gram_tf32(const float* X, int ldx, int B, int D, float scale, float* gram,
+__device__ __forceinline__ void gram_tf32(const float* X, int rs, int cs, int B, int D, float scale, float* gram,
                                           int lane) {
     const int g = lane >> 2, q = lane & 3;
     for (int n0 = 0; n0 < B; n0 += 8) {
         float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         for (int k0 = 0; k0 < D; k0 += 8) {
             uint32_t a[4], b[2];
-            a[0] = g < B ? to_tf32(X[g * ldx + k0 + q]) : 0u;
-            a[1] = g + 8 < B ? to_tf32(X[(g + 8) * ldx + k0 + q]) : 0u;
-            a[2] = g < B ? to_tf32(X[g * ldx + k0 + q + 4]) : 0u;
-            a[3] = g + 8 < B ? to_tf32(X[(g + 8) * ldx + k0 + q + 4]) : 0u;
+            a[0] = g < B ? to_tf32(X[g * rs + (k0 + q) * cs]) : 0u;
+            a[1] = g + 8 < B ? to_tf32(X[(g + 8) * rs + (k0 + q) * cs]) : 0u;
+            a[2] = g < B ? to_tf32(X[g * rs + (k0 + q + 4) * cs]) : 0u;
+            a[3] = g + 8 < B ? to_tf32(X[(g + 8) * rs + (k0 + q + 4) * cs]) : 0u;
             const int n = n0 + g;  // B's column n is row n of X
-            b[0] = n < B ? to_tf32(X[n * ldx + k0 + q]) : 0u;
-            b[1] = n < B ? to_tf32(X[n * ldx + k0 + q + 4]) : 0u;
+            b[0] = n < B ? to_tf32(X[n * rs + (k0 + q) * cs]) : 0u;
+            b[1] = n < B ? to_tf32(X[n * rs + (k0 + q + 4) * cs]) : 0u;
             mma_tf32(acc, a, b);
         }
         const int c0 = n0 + 2 * q;
@@ -180,7 +180,7 @@ __device__ __forceinline__ void gram_tf32(const float* X, int ldx, int B, int D,
 // same order either way: the column sums and the centring by the thread that
 // owns the column, each Gram pair by one octet of lanes, each channel's
 // flat-area sums by one warp.
-template <int W>
+template <int W, int kHeld>
 __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunch L) {
     constexpr int kGroups = kPrepareWarps / W;  // groups per CTA
     constexpr int kT = 32 * W;                  // threads per group
@@ -192,13 +192,13 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
     size_t* bases_all = reinterpret_cast<size_t*>(sm + ((D + 3) & ~3));  // kGroups * max_rows
     // model row s, column col at X[s * rs + col * cs]: rows at a padded stride
     // (octets on different rows hit different banks), or, for the blocked dual
-    // Gram of a whole CTA, columns of ldc floats (PrepareColumns)
-    const int ldc = W > 1 ? L.gram_columns : 0;
+    // Gram, columns of ldc floats
+    const int ldc = L.gram_columns;
     const int rs = ldc > 0 ? 1 : D + 8, cs = ldc > 0 ? ldc : 1;
     const int slot = threadIdx.x / kT;          // this group's slot in the CTA
     const int t = threadIdx.x - slot * kT;      // thread within the group
-    float* X = reinterpret_cast<float*>(bases_all + kGroups * L.max_rows + (ldc > 0 ? L.max_rows & 1 : 0)) +
-               slot * Bmax * (D + 8);  // model rows; columns start on 16 bytes
+    float* X = reinterpret_cast<float*>(bases_all + kGroups * L.max_rows + (ldc > 0 ? kGroups * L.max_rows & 1 : 0)) +
+               slot * (ldc > 0 ? D * ldc : Bmax * (D + 8));  // model rows; columns start on 16 bytes
     size_t* bases = bases_all + slot * L.max_rows;
     for (int col = threadIdx.x; col < D; col += blockDim.x) coloff[col] = column_offset(L, col);
     __syncthreads();
@@ -345,26 +345,59 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
         // thread owns a column, whose rows' loads are in flight together
         const float inv_b = __fdiv_rn(1.0f, static_cast<float>(B));
         float* means = L.means + static_cast<size_t>(v) * 2 * D;
-        for (int col = t; col < D; col += kT) {
-            const float* src = model_video + cb + coloff[col];
-#pragma unroll 8
-            for (int s2 = 0; s2 < B; ++s2) X[s2 * rs + col * cs] = __ldg(src + bases[s2]);
-            float mm = 0.0f;
-#pragma unroll 8
-            for (int s2 = 0; s2 < B; ++s2) mm = __fadd_rn(mm, X[s2 * rs + col * cs]);
-            mm = __fmul_rn(mm, inv_b);
-            float center = mm;  // Basic: noisy mean; Final flat: basic mean
-            if (final_stage && !flat) {
+        if constexpr (kHeld > 0) {
+            // up to kHeld rows stay in registers until they are centred
+            for (int col = t; col < D; col += kT) {
+                const float* src = model_video + cb + coloff[col];
                 const float* noisy = L.noisy + cb + coloff[col];
-                float mn = 0.0f;
-#pragma unroll 8
-                for (int s2 = 0; s2 < B; ++s2) mn = __fadd_rn(mn, __ldg(noisy + bases[s2]));
-                center = __fmul_rn(mn, inv_b);
+                const bool own_center = final_stage && !flat;  // else the model rows' mean
+                float x[kHeld], y[kHeld];
+#pragma unroll
+                for (int s2 = 0; s2 < kHeld; ++s2) x[s2] = s2 < B ? __ldg(src + bases[s2]) : 0.0f;
+                if (own_center)
+#pragma unroll
+                    for (int s2 = 0; s2 < kHeld; ++s2) y[s2] = s2 < B ? __ldg(noisy + bases[s2]) : 0.0f;
+                float mm = 0.0f, mn = 0.0f;
+#pragma unroll
+                for (int s2 = 0; s2 < kHeld; ++s2)
+                    if (s2 < B) mm = __fadd_rn(mm, x[s2]);
+                mm = __fmul_rn(mm, inv_b);
+                if (own_center) {
+#pragma unroll
+                    for (int s2 = 0; s2 < kHeld; ++s2)
+                        if (s2 < B) mn = __fadd_rn(mn, y[s2]);
+                }
+                means[col] = mm;
+                means[D + col] = own_center ? __fmul_rn(mn, inv_b) : mm;
+                float4* out = reinterpret_cast<float4*>(X + col * ldc);
+#pragma unroll
+                for (int q = 0; q < kHeld / 4; ++q)
+                    if (4 * q < B)
+                        out[q] = make_float4(__fsub_rn(x[4 * q], mm), __fsub_rn(x[4 * q + 1], mm),
+                                             __fsub_rn(x[4 * q + 2], mm), __fsub_rn(x[4 * q + 3], mm));
             }
-            means[col] = mm;
-            means[D + col] = center;
+        } else {
+            for (int col = t; col < D; col += kT) {
+                const float* src = model_video + cb + coloff[col];
 #pragma unroll 8
-            for (int s2 = 0; s2 < B; ++s2) X[s2 * rs + col * cs] = __fsub_rn(X[s2 * rs + col * cs], mm);
+                for (int s2 = 0; s2 < B; ++s2) X[s2 * rs + col * cs] = __ldg(src + bases[s2]);
+                float mm = 0.0f;
+#pragma unroll 8
+                for (int s2 = 0; s2 < B; ++s2) mm = __fadd_rn(mm, X[s2 * rs + col * cs]);
+                mm = __fmul_rn(mm, inv_b);
+                float center = mm;  // Basic: noisy mean; Final flat: basic mean
+                if (final_stage && !flat) {
+                    const float* noisy = L.noisy + cb + coloff[col];
+                    float mn = 0.0f;
+#pragma unroll 8
+                    for (int s2 = 0; s2 < B; ++s2) mn = __fadd_rn(mn, __ldg(noisy + bases[s2]));
+                    center = __fmul_rn(mn, inv_b);
+                }
+                means[col] = mm;
+                means[D + col] = center;
+#pragma unroll 8
+                for (int s2 = 0; s2 < B; ++s2) X[s2 * rs + col * cs] = __fsub_rn(X[s2 * rs + col * cs], mm);
+            }
         }
         group_sync();
         if (L.rank > 0) {
@@ -372,8 +405,8 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
             float* gram = L.gram + static_cast<size_t>(v) * L.nmax * L.nmax;
             if (D >= 64 && B < D && L.mixed && W == 1 && B <= 16 && D % 8 == 0) {
                 // chosen forms: TF32 tensor-core Gram, FP32 accumulation
-                gram_tf32(X, rs, B, D, scale, gram, lane);
-            } else if (W > 1 && ldc > 0) {
+                gram_tf32(X, rs, cs, B, D, scale, gram, lane);
+            } else if (ldc > 0) {
                 // dual Gram (compute_gram_centered) in blocks of 4 x 4 pairs, an
                 // octet per block: lane j runs the pinned chain j of the 16
                 // pairs on two 16-byte loads per step, and the folds leave it
@@ -2352,21 +2385,30 @@ cudaError_t launch_filter(const FilterLaunch& L, int max_groups_in, cudaStream_t
                              static_cast<size_t>(groups_per_cta) * L.max_rows * sizeof(size_t);
         size_t smem = fixed + static_cast<size_t>(groups_per_cta) * Bmax * (D + 8) * sizeof(float);
         // the blocked Gram's columns: an odd number of 16-byte units each, so
-        // that the 8 columns of a quarter warp start on different banks
-        // (without the odd unit, or in rows, where that does not fit)
+        // that the 8 columns of a quarter warp start on different banks (without
+        // the odd unit where a CTA holds four groups, whose number counts more,
+        // or where it does not fit); rows where neither does
         FilterLaunch P = L;
         P.gram_columns = 0;
-        if (wide && D >= 64 && Bmax < D) {
+        if (D >= 64 && Bmax < D && (wide || (Bmax > 4 && Bmax <= 8))) {
             const int quads = (Bmax + 3) / 4;
-            for (int ldc : {4 * (quads | 1), 4 * quads}) {
-                const size_t bytes = fixed + (L.max_rows & 1) * sizeof(size_t) + static_cast<size_t>(D) * ldc * sizeof(float);
+            for (int ldc : {4 * (wide ? quads | 1 : quads), 4 * quads}) {
+                const size_t bytes = fixed + (groups_per_cta * L.max_rows & 1) * sizeof(size_t) +
+                                     static_cast<size_t>(groups_per_cta) * D * ldc * sizeof(float);
                 if (bytes > kFilterSharedLimit) continue;
                 P.gram_columns = ldc;
                 smem = bytes;
                 break;
             }
         }
-        auto kernel = wide ? prepare_kernel<kPrepareWarps> : prepare_kernel<1>;
+        // rows held in registers: with several columns per thread their loads
+        // overlap (57k groups of dimension 294 0.49 -> 0.35 and 0.91 -> 0.88 ms,
+        // 32k warps of dimension 192 191 -> 124 us); with one, the registers cost
+        // more blocks than that saves (130k groups of dimension 128, Final, 1.33
+        // -> 1.61 ms)
+        const bool held = P.gram_columns > 0 && Bmax <= 16 && D > 32 * kPrepareWarps;
+        auto kernel = !wide ? (P.gram_columns > 0 ? prepare_kernel<1, 8> : prepare_kernel<1, 0>)
+                            : (held ? prepare_kernel<kPrepareWarps, 16> : prepare_kernel<kPrepareWarps, 0>);
         cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(kernel),
                                                static_cast<int>(smem));
         if (err != cudaSuccess) return err;
