@@ -1232,7 +1232,7 @@ __host__ __device__ inline TileApplyLayout tile_apply_layout(int D, int Bmax, in
     a.means = off;   off += (2 * D + 3) & ~3;
     a.basis = off;   off += D * a.ldb;
     a.dual = off;    off += Bmax * comps;
-    a.scal = off;    off += 5 * comps;
+    a.scal = off;    off += 6 * comps;
     a.scores = off;  off += (max_rows + 3) & ~3;
     a.bases = off;   off += 2 * ((max_rows + 1) & ~1);
     a.tiles = off;
@@ -1397,6 +1397,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, kQ == 1 ? 4 : 2) apply_tile_k
     float* denom = coef + kComps;    // signal eigenvalue + membership noise
     float* inv_sqrt = denom + kComps;  // 1 / sqrt(eigenvalue), 0 below the floor
     float* terms = inv_sqrt + kComps;  // log1p(signal / membership noise)
+    float* shares = terms + kComps;    // signal / (signal + noise)
     float* scores = sm + lay.scores;
     size_t* bases = reinterpret_cast<size_t*>(sm + lay.bases);
     const int tid = threadIdx.x;
@@ -1470,6 +1471,7 @@ __global__ void __launch_bounds__(32 * kTileWarps, kQ == 1 ? 4 : 2) apply_tile_k
             denom[c] = __fadd_rn(signal, mem2);
             inv_sqrt[c] = lambda > kEigenFloor ? __fdiv_rn(1.0f, __fsqrt_rn(lambda)) : 0.0f;
             terms[c] = (membership_on && signal > 0.0f) ? cr_log1pf(__fdiv_rn(signal, mem2)) : 0.0f;
+            shares[c] = signal > 0.0f ? __fdiv_rn(signal, __fadd_rn(signal, sigma2)) : 0.0f;
             const float sigma_basic2 = kFinal ? model_noise2 : sigma2;
             const float threshold = __fmul_rn(P.variance_threshold, sigma2);
             float variance = lambda;
@@ -1526,13 +1528,11 @@ __global__ void __launch_bounds__(32 * kTileWarps, kQ == 1 ? 4 : 2) apply_tile_k
         // 346-358): the terms are ready, the sums run in component order
         if (tid == threads - 1) {
             float trace = 0.0f, volume = 0.0f;
+            // (a component without signal adds zero to both)
+#pragma unroll 4
             for (int c = 0; c < R; ++c) {
-                const float diff = __fsub_rn(eig[c], model_noise2);
-                const float lambda = diff > 0.0f ? diff : 0.0f;
-                if (lambda > 0.0f) {
-                    trace = __fadd_rn(trace, __fdiv_rn(lambda, __fadd_rn(lambda, sigma2)));
-                    volume = __fadd_rn(volume, terms[c]);
-                }
+                trace = __fadd_rn(trace, shares[c]);
+                volume = __fadd_rn(volume, terms[c]);
             }
             const float tau = __fadd_rn(
                 __fadd_rn(P.weight_epsilon, __fdiv_rn(static_cast<float>(D), static_cast<float>(B))), trace);
@@ -1654,10 +1654,18 @@ __global__ void __launch_bounds__(32 * kTileWarps, kQ == 1 ? 4 : 2) apply_tile_k
                 const float* qr = quot + lane * kComps;
                 const float* pr = square + lane * kComps;
                 float distance = 0.0f, projected = 0.0f;
-#pragma unroll 4
-                for (int c = 0; c < R; ++c) {
-                    distance = __fadd_rn(distance, qr[c]);
-                    projected = __fadd_rn(projected, pr[c]);
+#pragma unroll
+                for (int c0 = 0; c0 < kComps; c0 += 4) {
+                    if (c0 >= R) break;
+                    const float4 q4 = *reinterpret_cast<const float4*>(qr + c0);
+                    const float4 p4 = *reinterpret_cast<const float4*>(pr + c0);
+                    const float qs[4] = {q4.x, q4.y, q4.z, q4.w}, ps[4] = {p4.x, p4.y, p4.z, p4.w};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (c0 + c >= R) break;
+                        distance = __fadd_rn(distance, qs[c]);
+                        projected = __fadd_rn(projected, ps[c]);
+                    }
                 }
                 const float resid = __fsub_rn(norms[lane], projected);
                 distance = __fadd_rn(distance, __fdiv_rn(resid > 0.0f ? resid : 0.0f, mem2));
