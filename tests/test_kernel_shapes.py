@@ -127,11 +127,12 @@ def test_grids_and_tiles(name, w, h, f, planes, kw):
 
 
 @pytest.mark.parametrize("batch,inputs,hidden,layers,outputs", [
-    (1, 3, 5, 1, 7), (63, 45, 128, 3, 65), (129, 27, 64, 2, 1083), (300, 45, 128, 3, 5445), (700, 16, 16, 1, 16)])
+    (1, 3, 5, 1, 7), (63, 45, 128, 3, 65), (129, 27, 64, 2, 1083), (300, 45, 128, 3, 5445), (700, 16, 16, 1, 16),
+    (5, 27, 64, 2, 1536), (5, 27, 64, 2, 1537), (66, 27, 64, 2, 6144), (66, 27, 64, 2, 6201)])
 def test_network_products(batch, inputs, hidden, layers, outputs):
     """Products with whole tiles, remainders and splits, against float64.  A
-    product sums at most 5445 terms in FP32: their rounding stays under
-    5445 * 2^-24 = 3.3e-4 of the sum of magnitudes."""
+    product sums at most max(5445, outputs) terms in FP32: their rounding stays
+    under that many 2^-24 (3.3e-4 for 5445) of the sum of magnitudes."""
     import torch
 
     rng = np.random.default_rng(batch)
@@ -146,6 +147,7 @@ def test_network_products(batch, inputs, hidden, layers, outputs):
     net.logits(dx.data_ptr(), batch, out.data_ptr())
     want_loss, want = mlp_fp64.loss_and_gradients(net.get_weights(), shape, x, t)
     z = mlp_fp64.forward_logits(net.get_weights(), shape, x)
-    assert abs(loss - want_loss) <= 3.3e-4 * max(1.0, abs(want_loss))
-    assert np.abs(grads - want).max() <= 3.3e-4 * np.abs(want).max()
-    assert np.abs(out.cpu().numpy() - z).max() <= 3.3e-4 * np.abs(z).max()
+    bound = max(3.3e-4, outputs * 2.0**-24)
+    assert abs(loss - want_loss) <= bound * max(1.0, abs(want_loss))
+    assert np.abs(grads - want).max() <= bound * np.abs(want).max()
+    assert np.abs(out.cpu().numpy() - z).max() <= bound * np.abs(z).max()
