@@ -11,8 +11,8 @@
 // ascending, past descending: the CPU's candidate order) the CTA stages the
 // strip's search region of every needed plane in shared memory, each warp
 // computes the SSD of all its candidates in that frame with a register-tiled
-// sweep (lane task = one candidate column x KY candidate rows, reference patch
-// plane in registers), and then replays the CPU's sequential selection over
+// sweep (lane task = one candidate column x KY candidate rows, the reference
+// rows sliding along in registers), and then replays the CPU's sequential selection over
 // the frame's candidates in raster order.  The replay is exact: it keeps the
 // CPU's K-smallest heap front and its capped match buffer (same replacement
 // slot), and the 32 candidates of a chunk are first tested against the
