@@ -45,6 +45,14 @@ int vnlbgpu_diag_kernel_timing(vnlbgpu_session* session, int enable, double* ms,
  * active rows, up to `capacity` rows (*rows receives the true count). */
 int vnlbgpu_diag_filtered(vnlbgpu_session* session, int anchor, float* out, int capacity, int* rows, int* row_dim);
 
+/* Runs anchor frame `anchor` of a session with the tensor-core matcher and
+ * copies the approximate distances its selection ran on, [*groups][*stride]
+ * floats (up to `capacity` of them): candidate frame k (of schedule[0 ..
+ * *schedule_len), room for 32) of a grid anchor from k * *window_cells on, its
+ * search window's cells in raster order. */
+int vnlbgpu_diag_approx(vnlbgpu_session* session, int anchor, float* out, size_t capacity, int* groups, int* stride,
+                        int* window_cells, int* schedule, int* schedule_len);
+
 /* Test switch of the tensor-core matcher's bounded waits: with on != 0 its
  * MMA warp issues no MMA, so every wait for MMA completion runs out after
  * its iteration limit, the kernel returns with nothing in flight, and the

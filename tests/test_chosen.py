@@ -10,6 +10,8 @@ groups whose retained rows are exactly the plain form's is bounded from
 below, and the exact distances of rows both forms keep must be equal bit for
 bit.
 """
+import bisect
+
 import numpy as np
 import pytest
 
@@ -226,6 +228,92 @@ def test_tensor_core_buffers_of_96():
     plain = vnlbcu.Basic(noisy, sigma=5.0, **kw)
     tc = vnlbcu.Basic(noisy, sigma=5.0, form="chosen_tc", **kw)
     assert synth.psnr(plain, clean) - synth.psnr(tc, clean) <= 0.05
+
+
+def replayed_entries(distances, k, cap, tau):
+    """The capped buffer of find_similar_patches (core.cpp:1277-1359) after a
+    sequence of distances: the positions it holds."""
+    front, buf, ids = [], [], []
+    for i, d in enumerate(distances):
+        limit = max(tau, front[-1]) if len(front) == k else np.inf
+        if len(buf) == cap:
+            limit = min(limit, worst)
+        if not d <= limit:
+            continue
+        if len(buf) < cap:
+            buf.append(d)
+            ids.append(i)
+            worst = max(buf)
+        elif d < worst:
+            at = buf.index(worst)
+            buf[at], ids[at] = d, i
+            worst = max(buf)
+        if len(front) < k or d < front[-1]:
+            bisect.insort(front, d)
+            del front[k:]
+    return set(ids)
+
+
+def quantised(noisy, levels, period):
+    """Few sample values, repeated in space and time: most distances tie, at 0 and above."""
+    tile = np.round(noisy[:, :, :period, :period] * levels) / levels
+    out = np.tile(tile, (1, 1, noisy.shape[2] // period + 1, noisy.shape[3] // period + 1))
+    return np.ascontiguousarray(out[:, :, :noisy.shape[2], :noisy.shape[3]].astype(np.float32))
+
+
+@pytest.mark.parametrize("planes,sigma,kw,source", [
+    (3, 20.0, dict(), "noise"),
+    (1, 3.0, dict(block_size=8, block_step=8, group_size=16, bm_range=9, patch_time=2, rank=16, tau=3000.0), "noise"),
+    (1, 5.0, dict(block_size=8, block_step=8, group_size=24, bm_range=9, patch_time=2, rank=24, tau=200.0), "noise"),
+    (1, 25.0, dict(block_size=8, block_step=8, group_size=17, bm_range=7, radius=2, rank=8, cap_factor=2.0), "noise"),
+    (1, 25.0, dict(block_size=7, block_step=5, group_size=12, bm_range=9, rank=8, cap_factor=3.0), "tie"),
+    (1, 25.0, dict(block_size=8, block_step=5, group_size=24, bm_range=9, rank=8, tau=6000.0), "tie"),
+    (1, 25.0, dict(block_size=8, block_step=8, group_size=16, bm_range=9, rank=8), "flat"),
+], ids=["defaults_yuv", "buffer64_tau", "buffer96_tau", "buffer34", "ties36", "ties96_tau", "flat64"])
+def test_tensor_core_selection_is_the_replay(planes, sigma, kw, source):
+    """The rows kept from buffers of more than 32 entries: the CPU's sequential
+    selection, replayed here on the approximate distances the kernel selected
+    from, leaves a set of candidates; the rows are those of them whose distance is
+    at most max(tau, the K-th smallest).  Distances are taken in float64, so a
+    candidate counts as within the threshold only below it by 1e-5 of it: an FP32
+    sum of at most 294 squares, in chains of 8 and a fold, is off by less."""
+    _, noisy = synth.make_clip(112, 80, 4, planes, sigma, seed=94)
+    if source != "noise":
+        noisy = quantised(noisy, 4, 10 if source == "tie" else 80)
+    if source == "flat":
+        noisy[:, :, :, :70] = 0.25
+    params = vnlbcu.parse_parameters(lib.STAGE_BASIC, noisy, sigma, dict(kw, form="chosen_tc"))
+    frames, _, h, w = noisy.shape
+    size, depth, k = params.patch_size, params.patch_time, params.similar
+    window = params.search_window
+    s = lib.Session(params, w, h, frames, planes)
+    s.set_clip(lib.SOURCE_CLIP, noisy)
+    d = s.diag_anchor(1)
+    approx, schedule = s.diag_approx(1)
+    s.close()
+    cap = d["max_rows"]
+    assert 32 < cap <= 96 and len(approx) == len(d["xy"])
+    wx, wy = min(window, w - size + 1), min(window, h - size + 1)
+    luma = noisy[:, 0].astype(np.float64)
+    patch = lambda f, x, y: luma[f:f + depth, y:y + size, x:x + size]
+
+    def low(center, axis):
+        start, end = center - (window - 1) // 2, center + (window - 1) // 2
+        return max(0, start - (min(0, start) + max(0, end - (axis - size))))
+
+    for g, (ax, ay) in enumerate(d["xy"]):
+        rows = d["grid_rows"][g][: d["counts"][g]]
+        got = {(int(r["x"]), int(r["y"]), int(r["frame"])) for r in rows}
+        x0, y0 = low(ax, w), low(ay, h)
+        kept = {}
+        for i in replayed_entries(approx[g].reshape(-1).tolist(), k, cap, params.tau):
+            f, cell = schedule[i // (wx * wy)], i % (wx * wy)
+            x, y = x0 + cell % wx, y0 + cell // wx
+            kept[x, y, f] = float(((patch(f, x, y) - patch(1, ax, ay)) ** 2).sum())
+        threshold = max(params.tau, sorted(kept.values())[min(k, len(kept)) - 1])
+        assert got <= set(kept), (g, got - set(kept))
+        missing = [p for p, e in kept.items() if e < threshold * (1 - 1e-5) and p not in got]
+        assert not missing, (g, missing)
 
 
 def test_autotuned_tensor_core_session():

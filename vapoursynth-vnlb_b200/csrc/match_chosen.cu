@@ -746,25 +746,35 @@ __device__ __forceinline__ float exact_distance(const MatchLaunch& L, const floa
     return d;
 }
 
-// Steps 2-4 for one anchor per warp, from the approximate distances.  The
-// capped buffer's slot s lives in lane s % 32, register s / 32 (CW registers:
-// buffers of up to 32 CW entries).
 // The CPU's sequential selection (find_similar_patches) on one anchor's
 // approximate distances, frame by frame in candidate order: the K-smallest
-// front and the capped buffer of up to 32 entries, slot i in lane i.  Returns
-// the entries; id is this lane's.
-__device__ __forceinline__ int select_replay(const MatchLaunch& L, const float* approx, int cells, int lane, int& id) {
-    constexpr int kSelectBatch = 8;  // chunks of 32 distances loaded at once
+// front and the capped buffer of up to 32 CW entries, slot i in word i / 32 of
+// lane i % 32.  Returns the entries; id holds this lane's.
+template <int CW>
+__device__ __forceinline__ int select_replay(const MatchLaunch& L, const float* approx, int cells, int lane,
+                                             int (&id)[CW]) {
+    constexpr int kSelectBatch = CW == 1 ? 8 : 4;  // chunks of 32 distances loaded at once
     const int K = L.K;
     const int cap = min(L.soft_cap, L.search_window * L.search_window * L.schedule_len);
     int count = 0, worst_idx = 0, top_count = 0;
     float worst = kInf, top_front = kInf;
-    unsigned reg_d = 0u, reg_top = 0u;  // bits of non-negative distances
-    id = 0;
+    unsigned reg_d[CW], reg_top = 0u;  // bits of non-negative distances
+#pragma unroll
+    for (int w = 0; w < CW; ++w) {
+        reg_d[w] = 0u;
+        id[w] = 0;
+    }
     const auto find_worst = [&] {  // the buffer's largest distance and its lowest slot
-        const unsigned m = __reduce_max_sync(0xffffffffu, reg_d);
+        unsigned m = reg_d[0];
+#pragma unroll
+        for (int w = 1; w < CW; ++w) m = max(m, reg_d[w]);
+        m = __reduce_max_sync(0xffffffffu, m);
         worst = __uint_as_float(m);
-        worst_idx = __ffs(__ballot_sync(0xffffffffu, reg_d == m)) - 1;
+#pragma unroll
+        for (int w = CW - 1; w >= 0; --w) {
+            const unsigned hit = __ballot_sync(0xffffffffu, reg_d[w] == m);
+            if (hit) worst_idx = 32 * w + __ffs(hit) - 1;
+        }
     };
     const auto limit_now = [&] {
         const float limit = top_count >= K ? std_max(L.tau, top_front) : kInf;
@@ -792,10 +802,13 @@ __device__ __forceinline__ int select_replay(const MatchLaunch& L, const float* 
                     if (!(d <= limit_now())) continue;
                     const bool room = count < cap;
                     if (room || d < worst) {
-                        if (lane == (room ? count : worst_idx)) {
-                            reg_d = __float_as_uint(d);
-                            id = (k << 20) | (base + src_lane);
-                        }
+                        const int slot = room ? count : worst_idx;
+#pragma unroll
+                        for (int w = 0; w < CW; ++w)
+                            if (32 * w + lane == slot) {
+                                reg_d[w] = __float_as_uint(d);
+                                id[w] = (k << 20) | (base + src_lane);
+                            }
                         if (room) ++count;
                         if (count == cap) find_worst();
                     }
@@ -815,18 +828,19 @@ __device__ __forceinline__ int select_replay(const MatchLaunch& L, const float* 
     return count;
 }
 
-// The same selection for buffers of up to 32 CW entries: the front, and a log of
-// the candidates within the limit (the front's maximum, tau above it, and the
-// buffer's largest distance once it has been full).  The limit is taken once
-// per 32 candidates, which go into the log together; when the log is full, and
-// at the end, the buffer's capacity of smallest ones is kept, in candidate
-// order.  The replay, which moves the limit candidate by candidate and replaces
-// the buffer's worst entry each time, keeps the same ones, less those that
-// passed between two of its limits.  For buffers of 64 it costs less than
-// replacing the worst entry of several words at every record (57k anchors of
-// two and six planes 1.16 -> 0.82 and 1.55 -> 1.26 ms, 130k of two planes 2.08
-// -> 1.54 ms); for buffers of 32 the replay is the shorter one (33k anchors 246
-// against 465 us).
+// The replay's entries, from a log: what the replay offers to its buffer are the
+// candidates within max(tau, the front's maximum before them); the buffer keeps
+// the smallest `cap` of those.  So the front is moved candidate by candidate (an
+// SSD above its maximum never moves it), each chunk's candidates are held
+// against the front as it was before them and go into the log together, and when
+// the log is full, and at the end, its cap smallest are kept.  Only where equal
+// distances straddle that boundary does the replay's choice depend on which
+// slot it replaced last; such an anchor takes the replay itself (distances of 0
+// apart: a full buffer of those never changes, the first ones stay).  For
+// buffers of 64 the log costs less than replacing the worst entry of several
+// words at every record (57k anchors of two and six planes 1.16 -> 0.82 and
+// 1.55 -> 1.26 ms, 130k of two planes 2.08 -> 1.54 ms); for buffers of 32 the
+// replay is the shorter one (33k anchors 246 against 465 us).
 template <int CW>
 __device__ __forceinline__ int select_log(const MatchLaunch& L, const float* approx, int cells, int lane, float* sd,
                                           int* si, int (&id)[CW]) {
@@ -834,6 +848,7 @@ __device__ __forceinline__ int select_log(const MatchLaunch& L, const float* app
     const int cap = min(L.soft_cap, L.search_window * L.search_window * L.schedule_len);
     int logged = 0, top_count = 0;
     float top_front = kInf, worst = kInf;
+    bool cut = false;       // entries equal to the worst kept one were dropped
     unsigned reg_top = 0u;  // bits of non-negative distances order like them
     constexpr int kLog = 64 * CW;  // entries of sd and si
     const auto keep_smallest = [&] {
@@ -868,6 +883,7 @@ __device__ __forceinline__ int select_log(const MatchLaunch& L, const float* app
         }
         __syncwarp();
         int at = 0, equal = cap - below;  // entries equal to it that are kept, the first ones
+        cut = cut && __uint_as_float(lo) == worst;
 #pragma unroll
         for (int w = 0; w < 2 * CW; ++w) {
             const unsigned same = __ballot_sync(0xffffffffu, d[w] == lo);
@@ -879,6 +895,7 @@ __device__ __forceinline__ int select_log(const MatchLaunch& L, const float* app
                 si[slot] = ids[w];
             }
             at += __popc(mask);
+            cut |= __popc(same) > equal;
             equal -= min(equal, __popc(same));
         }
         __syncwarp();
@@ -903,17 +920,11 @@ __device__ __forceinline__ int select_log(const MatchLaunch& L, const float* app
             const int idx = base + lane;
             const float mine = vals[b];
             const float limit = fminf(top_count >= K ? std_max(L.tau, top_front) : kInf, worst);
-            const bool in = idx < cells && mine <= limit;
+            bool in = idx < cells && mine <= limit && !(cut && mine == worst);
             unsigned pass = __ballot_sync(0xffffffffu, in);
             if (pass == 0u) continue;
-            if (logged + 32 > kLog) keep_smallest();
-            if (in) {
-                const int slot = logged + __popc(pass & ((1u << lane) - 1u));
-                sd[slot] = mine;
-                si[slot] = (k << 20) | idx;
-            }
-            logged += __popc(pass);
-            // the front takes the ones below its maximum
+            // the front takes the ones below its maximum, and the candidates
+            // after each are held against the maximum it leaves
             if (top_count >= K) pass &= __ballot_sync(0xffffffffu, mine < top_front);
             while (pass) {
                 const int src_lane = __ffs(pass) - 1;
@@ -929,7 +940,16 @@ __device__ __forceinline__ int select_log(const MatchLaunch& L, const float* app
                     if (lane == owner) reg_top = __float_as_uint(d);
                 }
                 top_front = __uint_as_float(__reduce_max_sync(0xffffffffu, reg_top));
+                if (lane > src_lane && !(mine <= std_max(L.tau, top_front))) in = false;
             }
+            const unsigned mask = __ballot_sync(0xffffffffu, in);
+            if (logged + __popc(mask) > kLog) keep_smallest();
+            if (in) {
+                const int slot = logged + __popc(mask & ((1u << lane) - 1u));
+                sd[slot] = mine;
+                si[slot] = (k << 20) | idx;
+            }
+            logged += __popc(mask);
           }
         }
     }
@@ -939,9 +959,13 @@ __device__ __forceinline__ int select_log(const MatchLaunch& L, const float* app
 #pragma unroll
     for (int w = 0; w < CW; ++w) id[w] = 32 * w + lane < n ? si[32 * w + lane] : 0;
     __syncwarp();
+    if (cut && worst > 0.0f) return select_replay<CW>(L, approx, cells, lane, id);
     return n;
 }
 
+// Steps 2-4 for one anchor per warp, from the approximate distances.  The
+// capped buffer's slot s lives in lane s % 32, register s / 32 (CW registers:
+// buffers of up to 32 CW entries).
 template <int P, int CW>
 __global__ void __launch_bounds__(kTcThreads) tc_select_kernel(MatchLaunch L) {
     constexpr int kSlots = CW == 1 ? 32 : 64 * CW;  // the sorted buffer, or select_log's log
@@ -968,7 +992,7 @@ __global__ void __launch_bounds__(kTcThreads) tc_select_kernel(MatchLaunch L) {
     int reg_id[CW];
     float reg_exact[CW];
     int n;
-    if constexpr (CW == 1) n = select_replay(L, approx, cells, lane, reg_id[0]);
+    if constexpr (CW == 1) n = select_replay<CW>(L, approx, cells, lane, reg_id);
     else n = select_log<CW>(L, approx, cells, lane, sd, si, reg_id);
     // exact FP32 distance of every entry left in the buffer, in the plain
     // form's arithmetic order: once, after the last frame

@@ -1402,6 +1402,17 @@ struct Session {
         return pending;
     }
 
+    // The candidate frames of an anchor frame in the CPU's order: itself, later
+    // ones, earlier ones (compute_temporal_range / schedule_temporal_range)
+    int schedule_of(int anchor, int* schedule) const {
+        int low, high, n = 0;
+        temporal_range(frames, Pt, params.search_bwd, params.search_fwd, anchor, low, high);
+        schedule[n++] = anchor;
+        for (int f = anchor + 1; f <= high; ++f) schedule[n++] = f;
+        for (int f = anchor - 1; f >= low; --f) schedule[n++] = f;
+        return n;
+    }
+
     // One anchor frame on one lane: match -> paste mask -> filter -> stack
     // tiles.  Everything is enqueued on the lane's stream.  Returns the
     // stack's layout: 0 planar, else the floats of a pixel-interleaved one
@@ -1410,15 +1421,11 @@ struct Session {
         Grid& grid = grid_for(anchor);
         const int G = static_cast<int>(grid.anchors.size());
         cudaStream_t ls = lane.stream;
-        // schedule (compute_temporal_range / schedule_temporal_range)
         int low, high;
         temporal_range(frames, Pt, params.search_bwd, params.search_fwd, anchor, low, high);
         wait_frames(ls, low, high + Pt - 1);  // every sample the anchor frame reads is on the device
         int schedule[kMaxContributors];
-        int schedule_len = 0;
-        schedule[schedule_len++] = anchor;
-        for (int f = anchor + 1; f <= high; ++f) schedule[schedule_len++] = f;
-        for (int f = anchor - 1; f >= low; --f) schedule[schedule_len++] = f;
+        const int schedule_len = schedule_of(anchor, schedule);
         const float* search = stage == 1 ? ref : clip;
         MatchLaunch m{};
         m.video = search;
@@ -2885,6 +2892,37 @@ int vnlbgpu_diag_set_lanes(vnlbgpu_session* session, int lanes) {
         s.drain();
         s.lane_count = lanes <= 0 ? s.lanes_allocated : std::min(lanes, s.lanes_allocated);
         s.next_lane = 0;
+    });
+}
+
+int vnlbgpu_diag_approx(vnlbgpu_session* session, int anchor, float* out, size_t capacity, int* groups, int* stride,
+                        int* window_cells, int* schedule, int* schedule_len) {
+    return guarded([&]() {
+        if (!session || !groups || !stride || !window_cells || !schedule || !schedule_len)
+            vnlbgpu::fail("VNLB CUDA: null argument");
+        Session& s = session->impl;
+        std::lock_guard guard(s.lock);
+        vnlbgpu::check(cudaSetDevice(s.device), "cudaSetDevice");
+        s.require_sources();
+        if (anchor < 0 || anchor > s.frames - s.Pt) vnlbgpu::fail("VNLB CUDA: anchor frame out of range");
+        if (!s.chosen || s.flow_on()) vnlbgpu::fail("VNLB CUDA: the session does not run the tensor-core matcher");
+        vnlbgpu::DeviceArray<float> stack;
+        stack.allocate(s.stack_values(), "cudaMalloc(diag stack)");
+        s.fork();
+        Session::Lane& lane = s.lanes[0];
+        s.compute_anchor(anchor, stack.ptr, lane);
+        s.join();
+        s.check_status();
+        const int G = static_cast<int>(s.grid_for(anchor).anchors.size());
+        *groups = G;
+        *stride = s.approx_stride;
+        *window_cells = std::min(s.params.search_window, s.width - s.P + 1) *
+                        std::min(s.params.search_window, s.height - s.P + 1);
+        *schedule_len = s.schedule_of(anchor, schedule);
+        const size_t n = std::min(static_cast<size_t>(G) * s.approx_stride, capacity);
+        if (out && n > 0)
+            vnlbgpu::check(cudaMemcpy(out, lane.approx.ptr, n * sizeof(float), cudaMemcpyDeviceToHost), "copy");
+        s.invalidate();
     });
 }
 

@@ -71,7 +71,7 @@ EXPORTS = [
     "vnlbgpu_render_stack", "vnlbgpu_aggregate", "vnlbgpu_aggregate_frame_noalloc", "vnlbgpu_get_stats",
     "vnlbgpu_stream",
     "vnlbgpu_set_stream", "vnlbgpu_diag_anchor", "vnlbgpu_diag_kernel_timing", "vnlbgpu_diag_set_lanes",
-    "vnlbgpu_diag_filtered", "vnlbgpu_diag_stall_tensor_waits",
+    "vnlbgpu_diag_filtered", "vnlbgpu_diag_approx", "vnlbgpu_diag_stall_tensor_waits",
     "vnlbgpu_parse_mvtools_analysis", "vnlbgpu_parse_mvtools_vectors", "vnlbgpu_set_mvtools_analysis",
     "vnlbgpu_set_mvtools_frame", "vnlbgpu_shard_plan", "vnlbgpu_mlp_create", "vnlbgpu_mlp_destroy",
     "vnlbgpu_mlp_parameters", "vnlbgpu_mlp_get_weights", "vnlbgpu_mlp_set_weights", "vnlbgpu_mlp_gradients",
@@ -131,6 +131,8 @@ def load() -> ctypes.CDLL:
                                                        ctypes.c_void_p]
             lib.vnlbgpu_diag_set_lanes.argtypes = [ctypes.c_void_p, ctypes.c_int]
             lib.vnlbgpu_diag_stall_tensor_waits.argtypes = [ctypes.c_void_p, ctypes.c_int]
+            lib.vnlbgpu_diag_approx.argtypes = ([ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_size_t]
+                                                + [ctypes.c_void_p] * 5)
             lib.vnlbgpu_diag_filtered.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,
                                                   ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)]
             lib.vnlbgpu_parse_mvtools_analysis.argtypes = [ctypes.c_char_p, ctypes.c_size_t,
@@ -451,6 +453,18 @@ class Session:
         _check(self.lib.vnlbgpu_diag_filtered(self.handle, anchor, out.ctypes.data, rows.value, ctypes.byref(rows),
                                               ctypes.byref(dim)))
         return out[:rows.value]
+
+    def diag_approx(self, anchor: int):
+        """The approximate distances the tensor-core matcher selected from for
+        anchor frame `anchor`: ([groups][frames][window cells], frames)."""
+        groups, stride, cells, length = (ctypes.c_int() for _ in range(4))
+        schedule = (ctypes.c_int * 32)()
+        sizes = [ctypes.byref(groups), ctypes.byref(stride), ctypes.byref(cells), schedule, ctypes.byref(length)]
+        _check(self.lib.vnlbgpu_diag_approx(self.handle, anchor, None, 0, *sizes))
+        out = np.zeros((groups.value, stride.value), np.float32)
+        _check(self.lib.vnlbgpu_diag_approx(self.handle, anchor, out.ctypes.data, out.size, *sizes))
+        n = length.value
+        return out[:, :n * cells.value].reshape(groups.value, n, cells.value), list(schedule[:n])
 
     def diag_anchor(self, anchor: int):
         """Runs one anchor frame and returns (grid, active) read-backs."""
