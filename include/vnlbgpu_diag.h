@@ -53,6 +53,13 @@ int vnlbgpu_diag_filtered(vnlbgpu_session* session, int anchor, float* out, int 
 int vnlbgpu_diag_approx(vnlbgpu_session* session, int anchor, float* out, size_t capacity, int* groups, int* stride,
                         int* window_cells, int* schedule, int* schedule_len);
 
+/* The chosen forms' Jacobi rotations on the host: cosine and sine of `count`
+ * angles from (app, aqq, apq), as the kernels compute them (longhand == 0; the
+ * host takes 1 / sqrt(x) for the device's rsqrt(x)) or by the reference's steps
+ * in FP64.  Needs no device. */
+int vnlbgpu_diag_angles(const float* app, const float* aqq, const float* apq, int count, int longhand, float* cosines,
+                        float* sines);
+
 /* Test switch of the tensor-core matcher's bounded waits: with on != 0 its
  * MMA warp issues no MMA, so every wait for MMA completion runs out after
  * its iteration limit, the kernel returns with nothing in flight, and the

@@ -128,3 +128,44 @@ def test_synth_is_seeded_and_shaped():
     noise = (n1 - c1).std()
     assert noise == pytest.approx(20.0 / 255.0, rel=0.1)
     assert synth.psnr(c1, c1) == float("inf")
+
+
+# (app, aqq, apq) whose cosine or sine lies so close to the middle of two floats
+# that the shorter FP64 steps alone round it the other way
+CLOSE_ANGLES = """
+    0x1.c7cf06p+0 0x1.c7f0cap+0 -0x1.a9bc48p-4    0x1.d1beep+2 0x1.0ef1d6p-2 0x1.5f7c06p-9
+    0x1.e0176ap-10 0x1.e1540ep-10 0x1.afc502p+0   0x1.bca8b2p-11 0x1.342a98p-6 -0x1.194804p-14
+    0x1.3a129cp+0 0x1.3a2f82p+0 0x1.f5a4c2p+1     0x1.2474e6p-5 0x1.7fad84p+3 0x1.df4138p-15
+    0x1.47784ap+1 0x1.92d7f2p+2 -0x1.85c54p-11    0x1.3d9724p-7 0x1.3d9f6ap-7 0x1.d22408p-4
+    0x1.35b07p-4 0x1.4ede96p-4 0x1.e26346p-16     0x1.85ec12p-7 0x1.8649bp-7 -0x1.3df146p-10
+    0x1.c7f0b8p+0 0x1.cddcdap+0 0x1.7fae6ap-9     0x1.72dae6p-3 0x1.45c2dep+1 -0x1.82e426p-5
+    0x1.a27d88p-3 0x1.f1f944p-1 -0x1.0ccfap-1     0x1.0d2a8ep+1 0x1.0d2acp+1 0x1.eb2b3ep-16
+    0x1.16b8c2p-3 0x1.322c7ap-3 -0x1.d79b18p-13   0x1.d74da6p+2 0x1.d74dc8p+2 -0x1.ab0b94p-3"""
+
+
+def test_chosen_angles_round_like_the_longhand():
+    """The chosen forms' FP64 rotation takes fewer operations than the
+    reference's steps and must round to the same floats, near the middle of two
+    of them as well, and for equal diagonals, tiny sines and huge matrices."""
+    close = np.array([float.fromhex(v) for v in CLOSE_ANGLES.split()], np.float32).reshape(-1, 3).T
+    rng = np.random.default_rng(0)
+    n = 1 << 19
+    scale = np.float32(2.0) ** rng.integers(-40, 40, (3, n)).astype(np.float32)
+    wide = rng.uniform(-2.0, 2.0, (3, n)).astype(np.float32) * scale
+    near = rng.uniform(0.5, 2.0, (3, n)).astype(np.float32)
+    near[1] = near[0] * (1 + rng.uniform(-1e-3, 1e-3, n).astype(np.float32))
+    near[2] *= np.float32(2.0) ** rng.integers(-17, 3, n).astype(np.float32)
+    edges = np.array([(1, 1, 1), (1, 1, -1e-5), (0, 0, 3e38), (3e38, -3e38, 1e-5), (-3e38, 3e38, 8e-6),
+                      (3e38, 1, 8e-6), (0, 0, 1e-45), (5, 4, 0.5)], np.float32).T
+    values = np.concatenate([close, wide, near, edges], 1)
+    values[2][values[2] == 0] = 1.0  # pairs of 0 are not rotated
+    got, want = lib.diag_angles(*values, longhand=False), lib.diag_angles(*values, longhand=True)
+    for g, w in zip(got, want):
+        assert np.array_equal(g.view(np.uint32), w.view(np.uint32))
+    # the shorter steps alone do not pass: each of the close ones differs
+    app, aqq, apq = close.astype(np.float64)
+    d, b = aqq - app, 2.0 * apq
+    t = np.abs(b) / (np.abs(d) + np.sqrt(d * d + b * b)) * np.where((d != 0) & ((d < 0) != (b < 0)), -1.0, 1.0)
+    c = 1.0 / np.sqrt(1.0 + t * t)
+    k = len(app)
+    assert np.all((c.astype(np.float32) != want[0][:k]) | ((t * c).astype(np.float32) != want[1][:k]))

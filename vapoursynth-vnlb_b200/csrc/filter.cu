@@ -506,18 +506,13 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
 
 // The rotation (c, s) that zeroes apq (jacobi_rotate, linalg.cpp:152-196).
 // kMixed (chosen forms): in FP64, so that near-degenerate pairs (aqq - app
-// tiny against apq) keep their angle; t = sgn 2 apq / (|d| + sqrt(d^2 +
-// 4 apq^2)) is the same tangent with one division and two square roots.
+// tiny against apq) keep their angle.
 template <bool kMixed>
 __device__ __forceinline__ void jacobi_angle(float app, float aqq, float apq, float& c, float& s) {
     if constexpr (kMixed) {
-        const double d = static_cast<double>(aqq) - static_cast<double>(app);
-        const double b = 2.0 * static_cast<double>(apq);
-        const double t_abs = fabs(b) / (fabs(d) + sqrt(d * d + b * b));
-        const double t = d != 0.0 && (d < 0.0) != (b < 0.0) ? -t_abs : t_abs;
-        const double cd = rsqrt(1.0 + t * t);
-        c = static_cast<float>(cd);
-        s = static_cast<float>(t * cd);
+        const float2 r = angle_fp64(app, aqq, apq);
+        c = r.x;
+        s = r.y;
     } else {
         const float tau = __fdiv_rn(__fsub_rn(aqq, app), __fmul_rn(2.0f, apq));
         const float t_abs =

@@ -2895,6 +2895,19 @@ int vnlbgpu_diag_set_lanes(vnlbgpu_session* session, int lanes) {
     });
 }
 
+int vnlbgpu_diag_angles(const float* app, const float* aqq, const float* apq, int count, int longhand, float* cosines,
+                        float* sines) {
+    return guarded([&]() {
+        if (!app || !aqq || !apq || !cosines || !sines) vnlbgpu::fail("VNLB CUDA: null argument");
+        float2 (*angle)(float, float, float) = longhand ? vnlbgpu::angle_fp64_longhand : vnlbgpu::angle_fp64;
+        for (int i = 0; i < count; ++i) {
+            const float2 r = angle(app[i], aqq[i], apq[i]);
+            cosines[i] = r.x;
+            sines[i] = r.y;
+        }
+    });
+}
+
 int vnlbgpu_diag_approx(vnlbgpu_session* session, int anchor, float* out, size_t capacity, int* groups, int* stride,
                         int* window_cells, int* schedule, int* schedule_len) {
     return guarded([&]() {

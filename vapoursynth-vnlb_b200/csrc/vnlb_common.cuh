@@ -8,7 +8,9 @@
 // CPU uses a fused multiply-add.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 namespace vnlbgpu {
@@ -238,6 +240,52 @@ __host__ __device__ __forceinline__ float cr_expf(float x) { return static_cast<
 __host__ __device__ __forceinline__ float cr_logf(float x) { return static_cast<float>(log(static_cast<double>(x))); }
 __host__ __device__ __forceinline__ float cr_log1pf(float x) {
     return static_cast<float>(log1p(static_cast<double>(x)));
+}
+
+// The rotation that zeroes apq, jacobi_rotate's steps (linalg.cpp:152-196) in
+// FP64 and rounded once: (cosine, sine) of the chosen forms' angle.
+__host__ __device__ __noinline__ inline float2 angle_fp64_longhand(float app, float aqq, float apq) {
+    const double tau = (static_cast<double>(aqq) - static_cast<double>(app)) / (2.0 * static_cast<double>(apq));
+    const double t_abs = 1.0 / (fabs(tau) + sqrt(1.0 + tau * tau));
+    const double t = tau < 0.0 ? -t_abs : t_abs;
+    const double cd = 1.0 / sqrt(1.0 + t * t);
+    return make_float2(static_cast<float>(cd), static_cast<float>(t * cd));
+}
+
+// The same floats with one division and one square root less; the longhand is a
+// call, since inlined it takes the rotations' registers (3840x2160 gray, groups of
+// 16, Basic and Final of three frames: longhand everywhere 49.2 ms, inlined behind
+// the test 48.6, this 43.2; the filter alone changes).  With d = aqq - app and
+// b = 2 apq, t = sgn |b| / (|d| + sqrt(d^2 + b^2)).  Both ways are within 12
+// units of 2^-53 of the exact cosine and sine (each operation adds at most one,
+// rsqrt two, and a square root halves what came before), so they lie within 24
+// last places of each other, and round to the same float unless a rounding
+// boundary (the low 29 bits at one half) is as close; there, and for sines near
+// the subnormal floats, whose boundaries lie elsewhere, the longhand decides.
+__host__ __device__ __forceinline__ float2 angle_fp64(float app, float aqq, float apq) {
+    const double d = static_cast<double>(aqq) - static_cast<double>(app);
+    const double b = 2.0 * static_cast<double>(apq);
+    const double t_abs = fabs(b) / (fabs(d) + sqrt(d * d + b * b));
+    const double t = d != 0.0 && (d < 0.0) != (b < 0.0) ? -t_abs : t_abs;
+#ifdef __CUDA_ARCH__
+    const double cd = rsqrt(1.0 + t * t);
+    const double sd = t * cd;
+    const unsigned cl = __double2loint(cd), sl = __double2loint(sd);
+#else
+    const double cd = 1.0 / sqrt(1.0 + t * t);
+    const double sd = t * cd;
+    unsigned long long bits;
+    memcpy(&bits, &cd, sizeof(bits));
+    const unsigned cl = static_cast<unsigned>(bits);
+    memcpy(&bits, &sd, sizeof(bits));
+    const unsigned sl = static_cast<unsigned>(bits);
+#endif
+    constexpr unsigned kHalf = 1u << 28, kLow = 2 * kHalf - 1, kNear = 32u;
+    const float2 r = make_float2(static_cast<float>(cd), static_cast<float>(sd));
+    if ((cl & kLow) - (kHalf - kNear) <= 2 * kNear || (sl & kLow) - (kHalf - kNear) <= 2 * kNear ||
+        !(fabsf(r.y) >= 0x1p-120f))
+        return angle_fp64_longhand(app, aqq, apq);
+    return r;
 }
 
 // std::max / std::min on floats (first operand wins ties and NaNs).

@@ -71,7 +71,8 @@ EXPORTS = [
     "vnlbgpu_render_stack", "vnlbgpu_aggregate", "vnlbgpu_aggregate_frame_noalloc", "vnlbgpu_get_stats",
     "vnlbgpu_stream",
     "vnlbgpu_set_stream", "vnlbgpu_diag_anchor", "vnlbgpu_diag_kernel_timing", "vnlbgpu_diag_set_lanes",
-    "vnlbgpu_diag_filtered", "vnlbgpu_diag_approx", "vnlbgpu_diag_stall_tensor_waits",
+    "vnlbgpu_diag_filtered", "vnlbgpu_diag_approx", "vnlbgpu_diag_angles",
+    "vnlbgpu_diag_stall_tensor_waits",
     "vnlbgpu_parse_mvtools_analysis", "vnlbgpu_parse_mvtools_vectors", "vnlbgpu_set_mvtools_analysis",
     "vnlbgpu_set_mvtools_frame", "vnlbgpu_shard_plan", "vnlbgpu_mlp_create", "vnlbgpu_mlp_destroy",
     "vnlbgpu_mlp_parameters", "vnlbgpu_mlp_get_weights", "vnlbgpu_mlp_set_weights", "vnlbgpu_mlp_gradients",
@@ -131,6 +132,7 @@ def load() -> ctypes.CDLL:
                                                        ctypes.c_void_p]
             lib.vnlbgpu_diag_set_lanes.argtypes = [ctypes.c_void_p, ctypes.c_int]
             lib.vnlbgpu_diag_stall_tensor_waits.argtypes = [ctypes.c_void_p, ctypes.c_int]
+            lib.vnlbgpu_diag_angles.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2
             lib.vnlbgpu_diag_approx.argtypes = ([ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_size_t]
                                                 + [ctypes.c_void_p] * 5)
             lib.vnlbgpu_diag_filtered.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,
@@ -490,6 +492,15 @@ class Session:
                                                 ("weight", "f4")])
         return {"xy": xy, "counts": counts, "grid_rows": to_np(grid_rows, g * m).reshape(g, m) if g else None,
                 "max_rows": m, "active": active[:a], "active_rows": to_np(active_rows, r)}
+
+
+def diag_angles(app, aqq, apq, longhand: bool):
+    """vnlbgpu_diag_angles: (cosines, sines) of the chosen forms' rotations."""
+    app, aqq, apq = (_f32(np.asarray(v, np.float32)) for v in (app, aqq, apq))
+    c, s = np.empty_like(app), np.empty_like(app)
+    _check(load().vnlbgpu_diag_angles(app.ctypes.data, aqq.ctypes.data, apq.ctypes.data, app.size, int(longhand),
+                                      c.ctypes.data, s.ctypes.data))
+    return c, s
 
 
 def aggregate(stacks: np.ndarray, source: np.ndarray, search_bwd: int, search_fwd: int, patch_time: int,
