@@ -106,6 +106,20 @@ def test_jacobi_sizes(k, rank):
     check(48, 40, 3, 1, 20.0, dict(patch_time=2, group_size=k, rank=rank, cap_factor=1.0), seed=k)
 
 
+@pytest.mark.parametrize("k", [8, 16, 24, 32])
+def test_jacobi_groups_that_rotate_apart(k):
+    """Neighbouring groups of one warp rotate at different steps, some never:
+    noise of very different strength column by column, smooth ramps and repeated
+    rows, so that at every step some lanes update what others only read."""
+    rng = np.random.default_rng(k)
+    noise = rng.normal(0.0, 1.0, (4, 1, 40, 64))
+    strength = 10.0 ** -np.tile(np.repeat(np.arange(8) % 5, 8), 1)  # 1 ... 1e-4, 8 columns each
+    ramp = np.add.outer(np.arange(40) / 80.0, np.arange(64) / 128.0)
+    noisy = (ramp + 0.1 * noise * strength).astype(np.float32)
+    noisy[:, :, 20:30] = noisy[:, :, 20:21]
+    check(64, 40, 4, 1, 5.0, dict(patch_time=2, block_step=4, group_size=k, rank=k, cap_factor=1.0), 0, noisy)
+
+
 @pytest.mark.parametrize("name,w,h,f,planes,kw", MATCH, ids=[c[0] for c in MATCH])
 def test_match_selection(name, w, h, f, planes, kw):
     check(w, h, f, planes, 15.0, kw, seed=len(name) + 40)

@@ -775,16 +775,17 @@ __global__ void __launch_bounds__(32) jacobi_small_kernel(FilterLaunch L) {
                 for (int i = 0; i < kRows; ++i) {
                     // row r against column q: above the diagonal, below it, or
                     // (in the block of q) either, by lane; r = q reads (and
-                    // does not write) a slot of its own row
+                    // does not write) its own entry of vector q instead
                     const int r = i * kSeg + h;
-                    at[i] = tri + (i * kSeg + kSeg <= q  ? row_of[i] + q * kG
-                                   : i * kSeg > q         ? tri_at(q, 0) + r * kG
-                                   : r < q                ? row_of[i] + q * kG
-                                                          : tri_at(q, 0) + (r == q ? (q < N - 1 ? q + 1 : 0) : r) * kG);
-                    if (i == q / kSeg && q == N - 1 && r == q) at[i] = tri;
+                    at[i] = tri + (i * kSeg + kSeg <= q ? row_of[i] + q * kG
+                                   : i * kSeg > q        ? tri_at(q, 0) + r * kG
+                                   : r < q               ? row_of[i] + q * kG
+                                   : r > q               ? tri_at(q, 0) + r * kG
+                                                         : (kTri + N + q * N + r) * kG);
                     arq[i] = *at[i];
                     vrq[i] = vec[(q * N + r) * kG];
                 }
+                float dq = 0.0f;
                 if (rot) {
                     float c, s;
                     jacobi_angle<kMixed>(app, aqq, apq, c, s);
@@ -801,11 +802,11 @@ __global__ void __launch_bounds__(32) jacobi_small_kernel(FilterLaunch L) {
                     }
                     const float cc = __fmul_rn(c, c), ss = __fmul_rn(s, s);
                     const float cs2 = __fmul_rn(2.0f, __fmul_rn(c, s));
-                    if (h == 0)
-                        diag[q * kG] = __fadd_rn(__fadd_rn(__fmul_rn(ss, app), __fmul_rn(cs2, apq)), __fmul_rn(cc, aqq));
+                    dq = __fadd_rn(__fadd_rn(__fmul_rn(ss, app), __fmul_rn(cs2, apq)), __fmul_rn(cc, aqq));
                     app = __fadd_rn(__fsub_rn(__fmul_rn(cc, app), __fmul_rn(cs2, apq)), __fmul_rn(ss, aqq));
                 }
                 if constexpr (kSeg > 1) __syncwarp();
+                if (rot && h == 0) diag[q * kG] = dq;  // every lane has read the old one; read again at the next p
             }
             if (h == 0) diag[p * kG] = app;
 #pragma unroll
