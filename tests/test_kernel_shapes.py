@@ -120,6 +120,27 @@ def test_jacobi_groups_that_rotate_apart(k):
     check(64, 40, 4, 1, 5.0, dict(patch_time=2, block_step=4, group_size=k, rank=k, cap_factor=1.0), 0, noisy)
 
 
+@pytest.mark.parametrize("block", [3, 4, 5, 7])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_eigenvalues_beside_nan(block, value):
+    """One chroma sample that is no number, uncoupled planes: its column makes one
+    entry of the covariance's diagonal NaN beside finite ones, which have to be
+    sorted all the same.  Whatever that sample cannot reach (twice the window's
+    4 columns to either side, the block, the neighbours of a match) is the
+    oracle's, and the session renders on."""
+    kw = dict(block_size=block, block_step=2, group_size=9, rank=4, bm_range=2, chroma=0)
+    _, noisy = synth.make_clip(64, 32, 2, 3, 20.0, seed=block)
+    noisy[:, 1, 12, 6] = value
+    bp = O.cpu_params(O.BASIC, 20.0, **kw)
+    oracle = O.Oracle("port")
+    want = oracle.aggregate(oracle.stage_stacks(O.BASIC, bp, noisy), noisy, bp.search_bwd, bp.search_fwd, bp.patch_time)
+    s = session_for(lib.STAGE_BASIC, bp, noisy)
+    for _ in range(2):
+        got = s.render_clip()
+        assert np.array_equal(bits(got[..., 32:]), bits(want[..., 32:]))
+    s.close()
+
+
 @pytest.mark.parametrize("name,w,h,f,planes,kw", MATCH, ids=[c[0] for c in MATCH])
 def test_match_selection(name, w, h, f, planes, kw):
     check(w, h, f, planes, 15.0, kw, seed=len(name) + 40)

@@ -624,7 +624,11 @@ __global__ void __launch_bounds__(256) jacobi_kernel(FilterLaunch L, int seg, in
             }
         }
         // stable sort of the diagonal (descending), canonicalised top-rank
-        // eigenvectors (canonicalize_vector_row, linalg.cpp:198-227)
+        // eigenvectors (canonicalize_vector_row, linalg.cpp:198-227).  NaN
+        // beside numbers has no place in that order: positions coincide, and
+        // the ones left over keep an index of their own
+        for (int r = r0; r < B; r += seg) order[r] = r;
+        __syncwarp();
         for (int r = r0; r < B; r += seg) {
             const float dr = m[r * ld + r];
             int pos = 0;
@@ -820,7 +824,10 @@ __global__ void __launch_bounds__(32) jacobi_small_kernel(FilterLaunch L) {
     }
     // stable sort of the diagonal (descending), canonicalised top-rank
     // eigenvectors (canonicalize_vector_row, linalg.cpp:198-227); the sorted
-    // order goes where the triangle was
+    // order goes where the triangle was (positions that NaN leaves over keep an
+    // index of their own)
+    for (int r = h; r < B; r += kSeg) tri[r * kG] = __int_as_float(r);
+    __syncwarp();
     for (int r = h; r < B; r += kSeg) {
         const float dr = diag[r * kG];
         int pos = 0;
