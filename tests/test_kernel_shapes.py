@@ -34,6 +34,11 @@ APPLY_TILES = [
     # dimensions whose blocks hold four warps (768) and, in Final, two (1200)
     ("dim768", 64, 48, 2, 3, dict(block_size=16, group_size=6, rank=4, bm_range=2)),
     ("dim1200", 64, 48, 4, 1, dict(block_size=20, patch_time=3, group_size=6, rank=4, bm_range=2)),
+    # blocks that fill the shared memory to its last bytes but for the static arrays: four warps of
+    # row tiles (Final), and the dual Gram's columns with and without the odd unit
+    ("full_tiles", 24, 20, 9, 3, dict(block_size=7, patch_time=7, group_size=33, rank=4, bm_range=2, cap_factor=1.0)),
+    ("full_columns", 30, 26, 5, 3, dict(block_size=11, patch_time=3, group_size=48, rank=1, bm_range=4)),
+    ("full_columns_even", 32, 30, 6, 1, dict(block_size=13, patch_time=4, group_size=80, rank=1, bm_range=5)),
     # weights off, and only some on
     ("no_weights", 48, 40, 3, 1, dict(block_size=7, patch_time=2, group_size=12, rank=10, weight_alpha=0.0,
                                       weight_beta=0.0, weight_gamma=0.0)),

@@ -42,7 +42,9 @@ constexpr int kRecCols = 8;  // reconstruction columns held in registers per lan
 constexpr int kPrepareWarps = 4;
 constexpr float kEigenFloor = 128.0f * FLT_EPSILON;
 constexpr int kTileRows = 4;       // rows of a tile of dot products
-constexpr size_t kFilterSharedLimit = 227 * 1024;  // dynamic shared memory of one CTA on sm_100
+constexpr size_t kFilterSharedLimit = 227 * 1024;  // shared memory of one CTA on sm_100
+// ... of which prepare_kernel's and the apply kernels' static arrays take this much at most
+constexpr size_t kFilterStaticShared = 64;
 
 // dot_contiguous_highway (the pinned 8-lane order) computed by an octet of
 // lanes (j = lane & 7): lane j owns accumulator j; the fold follows reduce8.  All 8 lanes return the dot.
@@ -185,7 +187,8 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
     constexpr int kGroups = kPrepareWarps / W;  // groups per CTA
     constexpr int kT = 32 * W;                  // threads per group
     extern __shared__ __align__(16) float sm[];
-    __shared__ double s_sums[2 * 4];            // flat-area sums per warp (W > 1)
+    __shared__ double s_sums[2 * kPrepareWarps];  // flat-area sums per warp (W > 1)
+    static_assert(sizeof(s_sums) <= kFilterStaticShared);
     const int D = L.dim;
     const int Bmax = bmax_of(L);
     int* coloff = reinterpret_cast<int*>(sm);
@@ -2320,7 +2323,7 @@ int tile_apply_warps(const FilterLaunch& L) {
     const int Bmax = std::min(L.model_cap, L.max_rows);
     for (int warps = kTileWarps; warps >= 1; warps /= 2)
         if (static_cast<size_t>(tile_apply_layout(L.dim, Bmax, L.rank > 16 ? 2 : 1, L.max_rows, warps, L.stage == 1)
-                                    .bytes) <= kFilterSharedLimit)
+                                    .bytes) + kFilterStaticShared <= kFilterSharedLimit)
             return warps;
     return 0;
 }
@@ -2406,7 +2409,7 @@ cudaError_t launch_filter(const FilterLaunch& L, int max_groups_in, cudaStream_t
             for (int ldc : {4 * (wide ? quads | 1 : quads), 4 * quads}) {
                 const size_t bytes = fixed + (groups_per_cta * L.max_rows & 1) * sizeof(size_t) +
                                      static_cast<size_t>(groups_per_cta) * D * ldc * sizeof(float);
-                if (bytes > kFilterSharedLimit) continue;
+                if (bytes + kFilterStaticShared > kFilterSharedLimit) continue;
                 P.gram_columns = ldc;
                 smem = bytes;
                 break;
