@@ -151,6 +151,17 @@ def test_match_selection(name, w, h, f, planes, kw):
     check(w, h, f, planes, 15.0, kw, seed=len(name) + 40)
 
 
+def test_search_region_limit():
+    """The largest search region a session can be made for: the staged planes,
+    the window's distances, the reference patch and the buffer within 200 KB.
+    Four planes with 8 x 8 blocks and buffers of 64: windows up to 89 x 89."""
+    noisy = np.zeros((5, 1, 104, 120), np.float32)
+    kw = dict(patch_time=4, group_size=16, rank=1)
+    session_for(lib.STAGE_BASIC, O.cpu_params(O.BASIC, 20.0, bm_range=44, **kw), noisy).close()
+    with pytest.raises(lib.VNLBError, match="does not fit in shared memory"):
+        session_for(lib.STAGE_BASIC, O.cpu_params(O.BASIC, 20.0, bm_range=45, **kw), noisy)
+
+
 @pytest.mark.parametrize("planes,patch_time,tau", [(1, 1, 0.0), (1, 1, 400.0), (3, 2, 0.0)])
 def test_match_ties(planes, patch_time, tau):
     """Flat areas and repeated columns: most distances tie, many at zero."""

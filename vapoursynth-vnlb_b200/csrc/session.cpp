@@ -579,9 +579,12 @@ struct Session {
         prune_cap = 0;
         if (planes_n >= 4 && !approx && half >= 32 && half <= 0x7fff && resident(bytes(half)) == resident(bytes(0)))
             prune_cap = half;
-        // one anchor per block fits whatever fits without the rows' padding
-        const size_t padding = w > 1 ? 0 : 4 * static_cast<size_t>(planes_n * P * ((4 - P % 4) % 4) + 3 + prune_cap);
-        return bytes(prune_cap) <= 200 * 1024 + padding;
+        if (w > 1) return bytes(prune_cap) <= 200 * 1024;
+        // one anchor per block, the bound that decides whether a session can be
+        // made: without the padding of the reference rows and without the list,
+        // which both have room above it
+        probe.warp_floats = (cw0 * ch0 + planes_n * P * P + 2 * buffer_cap + 3) & ~3;
+        return match_shared_bytes(probe, w) <= 200 * 1024;
     }
     int prune_cap = 0;
     // flow-guided search: the strips' reservation widened by up to 16 columns
