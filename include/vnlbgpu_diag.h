@@ -66,6 +66,11 @@ int vnlbgpu_diag_angles(const float* app, const float* aqq, const float* apq, in
  * render raises "timed out".  0 restores normal matching. */
 int vnlbgpu_diag_stall_tensor_waits(vnlbgpu_session* session, int on);
 
+/* The same for the paste mask's walk: with on != 0 no grid row publishes how far
+ * it has come, so the wait of the row below runs out, the other rows stop
+ * waiting, no group is processed, and the render raises "timed out". */
+int vnlbgpu_diag_stall_paste_waits(vnlbgpu_session* session, int on);
+
 /* Limits the pipeline lanes the session uses to min(lanes, the lanes it
  * allocated) after waiting for its queued work; lanes <= 0 restores them all.
  * With one lane the anchor frames' kernels run one after another, so the

@@ -5,6 +5,8 @@ points on a small clip and must equal the CPU oracle bit for bit: dimensions
 that leave remainders of the 8-lane chains, row counts that leave remainders of
 the row tiles, ranks and matrix sizes on both sides of each kernel's range.
 """
+import time
+
 import numpy as np
 import pytest
 
@@ -175,6 +177,28 @@ def test_match_ties(planes, patch_time, tau):
 @pytest.mark.parametrize("name,w,h,f,planes,kw", GRIDS, ids=[c[0] for c in GRIDS])
 def test_grids_and_tiles(name, w, h, f, planes, kw):
     check(w, h, f, planes, 15.0, kw, seed=len(name) + 70)
+
+
+def test_paste_waits_run_out_and_report():
+    """The paste mask's waits for the grid row above are bounded: with rows told
+    to publish nothing the first wait runs out, all others give up with it (100
+    grid rows of 8 batches, 16 rows at a time, would wait 50 times as long), and
+    the render raises.  The session then renders as a fresh one does."""
+    kw = dict(block_step=4, group_size=8, rank=6, bm_range=3)
+    _, noisy = synth.make_clip(1000, 400, 2, 1, 15.0, seed=5)
+    bp = O.cpu_params(O.BASIC, 15.0, **kw)
+    fresh = session_for(lib.STAGE_BASIC, bp, noisy)
+    want = fresh.render_clip()
+    fresh.close()
+    s = session_for(lib.STAGE_BASIC, bp, noisy)
+    s.stall_paste_waits(True)
+    start = time.perf_counter()
+    with pytest.raises(lib.VNLBError, match="timed out waiting for the grid row above"):
+        s.render_clip()
+    assert time.perf_counter() - start < 2.0
+    s.stall_paste_waits(False)
+    assert np.array_equal(bits(s.render_clip()), bits(want))
+    s.close()
 
 
 @pytest.mark.parametrize("batch,inputs,hidden,layers,outputs", [

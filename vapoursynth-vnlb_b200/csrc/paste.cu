@@ -80,6 +80,7 @@ __global__ void __launch_bounds__(kPasteThreads) paste_kernel(PasteLaunch L) {
     extern __shared__ __align__(16) unsigned paste_smem[];
     __shared__ unsigned long long passed[kPasteWarps];  // per row in flight
     __shared__ int active_sum[kPasteWarps + 1], rows_sum[kPasteWarps + 1];
+    __shared__ volatile int gave_up;  // one warp's wait ran out: the others stop waiting too
     const int tid = threadIdx.x;
     const int warp = tid >> 5;
     const int lane = tid & 31;
@@ -89,6 +90,7 @@ __global__ void __launch_bounds__(kPasteThreads) paste_kernel(PasteLaunch L) {
         const int rem = L.groups - w * 32;
         alive[w] = rem >= 32 ? 0xffffffffu : ((1u << rem) - 1u);
     }
+    if (tid == 0) gave_up = 0;
     if (lane == 0) passed[warp] = static_cast<unsigned long long>(warp) << 32;  // its first row, nothing decided
     __syncthreads();
     const unsigned long long* above = passed + (warp + kPasteWarps - 1) % kPasteWarps;
@@ -127,15 +129,18 @@ __global__ void __launch_bounds__(kPasteThreads) paste_kernel(PasteLaunch L) {
             const int last_x = __shfl_sync(0xffffffffu, b.x, n - 1);
             const int next_x = __shfl_sync(0xffffffffu, next.x, 0);
             // the row above has passed the reach of this batch's last anchor
-            if (row > 0) {
+            if (row > 0 && !failed) {
                 int spins = 0;
                 for (;;) {
                     const unsigned long long p = progress(above);
                     const int r = static_cast<int>(p >> 32), x = static_cast<int>(p & 0xffffffffu);
                     if (r > row - 1 || (r == row - 1 && x > last_x + L.reach_x)) break;
-                    if (++spins >= kPasteSpinLimit) break;
+                    if (++spins >= kPasteSpinLimit || (spins % 256 == 0 && gave_up)) {
+                        failed = true;
+                        gave_up = 1;
+                        break;
+                    }
                 }
-                failed |= spins >= kPasteSpinLimit;
                 __syncwarp();
             }
             unsigned bits = bits_at(alive, j0, words);
@@ -164,7 +169,7 @@ __global__ void __launch_bounds__(kPasteThreads) paste_kernel(PasteLaunch L) {
                 }
             }
             __syncwarp();
-            if (lane == 0) publish(passed + warp, row, j0 + 32 < end ? next_x : 0x7fffffff);
+            if (lane == 0 && !L.stall) publish(passed + warp, row, j0 + 32 < end ? next_x : 0x7fffffff);
             // the batch after the next one
             b = next;
             next.x = x2;
@@ -173,10 +178,13 @@ __global__ void __launch_bounds__(kPasteThreads) paste_kernel(PasteLaunch L) {
             load_counts(L, j + 96, end, x2, count2);
         }
         // this warp's next row: nothing of it is decided
-        if (row + kPasteWarps < L.grid_rows && lane == 0) publish(passed + warp, row + kPasteWarps, 0);
+        if (row + kPasteWarps < L.grid_rows && lane == 0 && !L.stall) publish(passed + warp, row + kPasteWarps, 0);
     }
     if (__syncthreads_or(failed)) {
+        // the mask is not final: report it, and let no group through
         if (tid == 0) atomicCAS(L.status, 0, kStatusPasteTimeout);
+        for (int w = tid; w < words; w += kPasteThreads) alive[w] = 0u;
+        __syncthreads();
     }
     // compaction: a contiguous range of words per warp, first the sums ...
     const int per_warp = (words + kPasteWarps - 1) / kPasteWarps;

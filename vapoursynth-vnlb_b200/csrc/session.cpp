@@ -181,6 +181,7 @@ struct Session {
     bool allow_scatter = true;    // off while a diagnostic reads the filtered rows back
     bool force_plain_match = false;  // the learned form's training pairs: the full search
     bool stall_mma = false;          // test switch: the tensor-core matcher issues no MMA
+    bool stall_paste = false;        // test switch: the paste mask's rows publish nothing
     // learned form (VNLBGPU_FORM_LEARNED): the attached network, shortlist
     // size, recall threshold of the per-tile check, tile edge; the network
     // sees slots_max scheduled frames of search_channels planes
@@ -1606,6 +1607,7 @@ struct Session {
         // search centre's way), and clears its neighbours' bits too
         pl.reach_x = params.search_window + (flow_on() ? flow_reach.x : 0);
         pl.status = d_status.ptr;
+        pl.stall = stall_paste ? 1 : 0;
         pl.active = lane.active.ptr;
         pl.active_xy = lane.active_xy.ptr;
         pl.row_offset = lane.row_offset.ptr;
@@ -2882,6 +2884,16 @@ int vnlbgpu_diag_stall_tensor_waits(vnlbgpu_session* session, int on) {
         Session& s = session->impl;
         std::lock_guard guard(s.lock);
         s.stall_mma = on != 0;
+        s.invalidate();
+    });
+}
+
+int vnlbgpu_diag_stall_paste_waits(vnlbgpu_session* session, int on) {
+    return guarded([&]() {
+        if (!session) vnlbgpu::fail("VNLB CUDA: null argument");
+        Session& s = session->impl;
+        std::lock_guard guard(s.lock);
+        s.stall_paste = on != 0;
         s.invalidate();
     });
 }

@@ -171,7 +171,6 @@ struct FrameCounters {
 };
 
 constexpr int kStatusRankNotCovered = 1;  // fewer model rows than the rank
-constexpr int kStatusPasteCapacity = 2;   // too many anchors for the paste kernel
 constexpr int kStatusTensorTimeout = 3;   // an MMA completion wait ran out (tensor-core matcher)
 constexpr int kStatusTmaTimeout = 4;      // a tensor-memory-accelerator load wait ran out (plain matcher)
 constexpr int kStatusPasteTimeout = 6;    // the paste walk's wait for the grid row above ran out
@@ -187,6 +186,7 @@ struct PasteLaunch {
     int grid_rows;
     int reach_x;          // a victim lies within this many columns of its anchor
     int* status;          // session status word
+    int stall;            // for tests of the bounded waits: no row publishes how far it has come
     // outputs
     int* active;          // [G] active anchor indices in raster order
     int2* active_xy;      // [G] their positions

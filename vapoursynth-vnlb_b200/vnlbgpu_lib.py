@@ -72,7 +72,7 @@ EXPORTS = [
     "vnlbgpu_stream",
     "vnlbgpu_set_stream", "vnlbgpu_diag_anchor", "vnlbgpu_diag_kernel_timing", "vnlbgpu_diag_set_lanes",
     "vnlbgpu_diag_filtered", "vnlbgpu_diag_approx", "vnlbgpu_diag_angles",
-    "vnlbgpu_diag_stall_tensor_waits",
+    "vnlbgpu_diag_stall_tensor_waits", "vnlbgpu_diag_stall_paste_waits",
     "vnlbgpu_parse_mvtools_analysis", "vnlbgpu_parse_mvtools_vectors", "vnlbgpu_set_mvtools_analysis",
     "vnlbgpu_set_mvtools_frame", "vnlbgpu_shard_plan", "vnlbgpu_mlp_create", "vnlbgpu_mlp_destroy",
     "vnlbgpu_mlp_parameters", "vnlbgpu_mlp_get_weights", "vnlbgpu_mlp_set_weights", "vnlbgpu_mlp_gradients",
@@ -132,6 +132,7 @@ def load() -> ctypes.CDLL:
                                                        ctypes.c_void_p]
             lib.vnlbgpu_diag_set_lanes.argtypes = [ctypes.c_void_p, ctypes.c_int]
             lib.vnlbgpu_diag_stall_tensor_waits.argtypes = [ctypes.c_void_p, ctypes.c_int]
+            lib.vnlbgpu_diag_stall_paste_waits.argtypes = [ctypes.c_void_p, ctypes.c_int]
             lib.vnlbgpu_diag_angles.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 2 + [ctypes.c_void_p] * 2
             lib.vnlbgpu_diag_approx.argtypes = ([ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_size_t]
                                                 + [ctypes.c_void_p] * 5)
@@ -432,6 +433,10 @@ class Session:
     def stall_tensor_waits(self, on: bool):
         """vnlbgpu_diag_stall_tensor_waits: the tensor-core matcher's test switch."""
         _check(self.lib.vnlbgpu_diag_stall_tensor_waits(self.handle, 1 if on else 0))
+
+    def stall_paste_waits(self, on: bool):
+        """vnlbgpu_diag_stall_paste_waits: the paste mask's test switch."""
+        _check(self.lib.vnlbgpu_diag_stall_paste_waits(self.handle, 1 if on else 0))
 
     def autotune(self, anchor: int = 1) -> dict:
         """vnlbgpu_autotune: the fastest bit-identical strip width and apply
