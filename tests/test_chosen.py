@@ -316,6 +316,31 @@ def test_tensor_core_selection_is_the_replay(planes, sigma, kw, source):
         assert not missing, (g, missing)
 
 
+@pytest.mark.parametrize("form,kw", [("chosen", CPU_DEFAULTS), ("chosen_tc", CPU_DEFAULTS),
+                                     ("chosen_tc", dict(block_size=7))],
+                         ids=["chosen", "tc_buffer32", "tc_buffer64"])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_samples_that_are_no_numbers(form, kw, value):
+    """A NaN sample's approximate distances clamp to 0, so its patches are
+    selected and their exact distances are NaN: the rows still name patches of
+    the frame, each once, numbers before the rest, and the session renders on."""
+    _, noisy = synth.make_clip(128, 64, 4, 1, 10.0, seed=95)
+    noisy[1, 0, 30, 20] = value
+    params = vnlbcu.parse_parameters(lib.STAGE_BASIC, noisy, 10.0, dict(kw, form=form))
+    s = lib.Session(params, 128, 64, 4, 1)
+    s.set_clip(lib.SOURCE_CLIP, noisy)
+    d = s.diag_anchor(1)
+    p, depth = params.patch_size, params.patch_time
+    for g in range(len(d["counts"])):
+        r = d["grid_rows"][g][: d["counts"][g]]
+        assert len(r) > 0 and not np.isnan(r["distance"]).any() and sorted_rows(r)
+        assert len(set(zip(r["x"].tolist(), r["y"].tolist(), r["frame"].tolist()))) == len(r)
+        for name, top in (("x", 128 - p), ("y", 64 - p), ("frame", 4 - depth)):
+            assert r[name].min() >= 0 and r[name].max() <= top
+    s.render_clip()
+    s.close()
+
+
 def test_autotuned_tensor_core_session():
     """The autotuner times the tensor-core matcher's planes per shared-memory
     stage (YUV444, 3 planes: 3, 2 and 1 per stage) and keeps the fastest; the

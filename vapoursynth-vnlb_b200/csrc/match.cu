@@ -685,8 +685,9 @@ __global__ void __launch_bounds__(256, 3) match_kernel(MatchLaunch L, const __gr
                 if (lane < s.count && (reg_id[0] >> 20) == k) {
                     const int cell = reg_id[0] & 0xfffff;
                     const int cy = cell / Wx;
-                    reg_exact = exact_distance8(planes, plane_values, L.region_stride, xl - rx0 + (cell - cy * Wx),
-                                                yl - ry0 + cy, ref, planes_n);
+                    const float d = exact_distance8(planes, plane_values, L.region_stride, xl - rx0 + (cell - cy * Wx),
+                                                    yl - ry0 + cy, ref, planes_n);
+                    reg_exact = fminf(d, kInf);  // NaN ranks last: a rank of its own for every entry
                 }
             }
         } else {

@@ -1002,8 +1002,9 @@ __global__ void __launch_bounds__(kTcThreads) tc_select_kernel(MatchLaunch L) {
         if (32 * w + lane < n) {
             const int i = reg_id[w] & 0xfffff;
             const int cy = i / Wx;
-            reg_exact[w] = exact_distance<P>(L, anchor_frame, anchor, L.schedule[reg_id[w] >> 20], yl + cy,
-                                             xl + (i - cy * Wx), planes_n, plane_values);
+            const float d = exact_distance<P>(L, anchor_frame, anchor, L.schedule[reg_id[w] >> 20], yl + cy,
+                                              xl + (i - cy * Wx), planes_n, plane_values);
+            reg_exact[w] = fminf(d, kInf);  // NaN ranks last: a rank of its own for every entry
         }
     }
 
