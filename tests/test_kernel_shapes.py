@@ -226,3 +226,16 @@ def test_network_products(batch, inputs, hidden, layers, outputs):
     assert abs(loss - want_loss) <= bound * max(1.0, abs(want_loss))
     assert np.abs(grads - want).max() <= bound * np.abs(want).max()
     assert np.abs(out.cpu().numpy() - z).max() <= bound * np.abs(z).max()
+
+
+def test_network_workspace_follows_the_batch():
+    """A network for batches of one row holds no workspace for large ones: its
+    few small arrays stay within the driver's 2 MiB units."""
+    import torch
+
+    lib.MLP(3, 5, 1, 7, max_batch=1, seed=0)  # the library's kernels are loaded
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    net = lib.MLP(3, 5, 1, 7, max_batch=1, seed=0)
+    assert before - torch.cuda.mem_get_info()[0] <= 4 << 20
+    del net

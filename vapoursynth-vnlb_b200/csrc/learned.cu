@@ -175,14 +175,21 @@ __global__ void reduce_kernel(GemmArgs g) {
 constexpr int kGemmBlocks = 2 * 148;
 constexpr int kGemmMinSteps = 128;
 
+int gemm_splits(int M, int N, int K) {
+    const int tiles = ((N + kTileN - 1) / kTileN) * ((M + kTileM - 1) / kTileM);
+    return tiles < kGemmBlocks ? std::max(1, std::min((kGemmBlocks + tiles - 1) / tiles, K / kGemmMinSteps)) : 1;
+}
+
+size_t gemm_partial_floats(int M, int N, int K) {
+    const int splits = gemm_splits(M, N, K);
+    return splits > 1 ? splits * static_cast<size_t>(M) * (N + 1) : 0;
+}
+
 template <bool TA, bool TB, typename TypeA, typename TypeB>
 cudaError_t gemm(const TypeA* A, const TypeB* B, GemmArgs g, cudaStream_t stream) {
     if (g.M <= 0 || g.N <= 0) return cudaSuccess;
     dim3 grid((g.N + kTileN - 1) / kTileN, (g.M + kTileM - 1) / kTileM);
-    const int tiles = static_cast<int>(grid.x * grid.y);
-    g.splits = 1;
-    if (g.partial && tiles < kGemmBlocks)
-        g.splits = max(1, min((kGemmBlocks + tiles - 1) / tiles, g.K / kGemmMinSteps));
+    g.splits = g.partial ? gemm_splits(g.M, g.N, g.K) : 1;
     grid.z = g.splits;
     gemm_kernel<TA, TB, TypeA, TypeB><<<grid, kGemmThreads, 0, stream>>>(A, B, g);
     cudaError_t e = cudaGetLastError();
@@ -579,10 +586,18 @@ cudaError_t mlp_infer(const MlpDevice& net, const float* x, int batch, float* co
     return cudaGetLastError();
 }
 
-size_t mlp_workspace_floats() {
-    // a split product has fewer than kGemmBlocks tiles, and splits * tiles stays
-    // below twice that; a tile's share is its C and its rows' sums
-    return 2 * static_cast<size_t>(kGemmBlocks) * (kTileM * kTileN + kTileM);
+size_t mlp_workspace_floats(const MlpDevice& net, int max_batch) {
+    size_t most = 0;
+    for (int l = 0; l <= net.layers; ++l) {
+        const int fan_in = l == 0 ? net.inputs : net.hidden, width = l == net.layers ? net.outputs : net.hidden;
+        // the weight gradient's splits grow with the batch
+        most = std::max(most, gemm_partial_floats(width, fan_in, max_batch));
+        if (l == 0) continue;
+        // the input gradient's shrink as its rows' tiles become more
+        for (int rows = kTileM; rows < max_batch + kTileM && rows <= kTileM * kGemmBlocks; rows += kTileM)
+            most = std::max(most, gemm_partial_floats(std::min(rows, max_batch), fan_in, width));
+    }
+    return most;
 }
 
 cudaError_t mlp_backward(const MlpDevice& net, const float* x, int batch, float* const* acts, float* dlogits,

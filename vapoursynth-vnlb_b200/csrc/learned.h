@@ -29,8 +29,9 @@ cudaError_t mlp_forward(const MlpDevice& net, const float* x, int batch, float* 
 cudaError_t mlp_backward(const MlpDevice& net, const float* x, int batch, float* const* acts, float* dlogits,
                          const int* targets, int tk, float* loss, float* const* dacts, float* const* gw,
                          float* const* gb, float* workspace, cudaStream_t stream);
-// Floats of mlp_backward's workspace (partial products of its splits).
-size_t mlp_workspace_floats();
+// Floats of mlp_backward's workspace (partial products of its splits) for batches
+// of up to max_batch rows; with none the workspace may be null.
+size_t mlp_workspace_floats(const MlpDevice& net, int max_batch);
 
 // One Adam step (step counts from 1) on the FP32 weights wmaster / net.b,
 // refreshing the BF16 copies.

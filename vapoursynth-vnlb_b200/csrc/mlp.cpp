@@ -53,7 +53,7 @@ struct vnlbgpu_mlp {
     float* logits = nullptr;
     float* loss = nullptr;
     int* status = nullptr;  // the inference kernels' status word
-    float* workspace = nullptr;  // partial products of the backward GEMMs' splits
+    float* workspace = nullptr;  // partial products of the backward GEMMs' splits, after the logits
 
     int fan_in(int l) const { return l == 0 ? inputs : hidden; }
     int fan_out(int l) const { return l == layers ? outputs : hidden; }
@@ -78,7 +78,6 @@ struct vnlbgpu_mlp {
         if (logits) cudaFree(logits);
         if (loss) cudaFree(loss);
         if (status) cudaFree(status);
-        if (workspace) cudaFree(workspace);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -173,9 +172,11 @@ int vnlbgpu_mlp_create(int inputs, int hidden, int layers, int outputs, int max_
             m->acts[l] = vnlbgpu::device_alloc<float>(static_cast<size_t>(max_batch) * hidden, "cudaMalloc(MLP)");
             m->dacts[l] = vnlbgpu::device_alloc<float>(static_cast<size_t>(max_batch) * hidden, "cudaMalloc(MLP)");
         }
-        m->logits = vnlbgpu::device_alloc<float>(static_cast<size_t>(max_batch) * outputs, "cudaMalloc(MLP logits)");
+        const size_t logits = static_cast<size_t>(max_batch) * outputs;
+        const size_t partial = vnlbgpu::mlp_workspace_floats(m->net, max_batch);
+        m->logits = vnlbgpu::device_alloc<float>(logits + partial, "cudaMalloc(MLP logits)");
+        if (partial > 0) m->workspace = m->logits + logits;
         m->status = vnlbgpu::device_alloc<int>(1, "cudaMalloc(MLP status)");
-        m->workspace = vnlbgpu::device_alloc<float>(vnlbgpu::mlp_workspace_floats(), "cudaMalloc(MLP workspace)");
         vnlbgpu::check(cudaMemset(m->status, 0, sizeof(int)), "cudaMemset(MLP status)");
         m->loss = vnlbgpu::device_alloc<float>(static_cast<size_t>(max_batch), "cudaMalloc(MLP loss)");
         vnlbgpu::check(cudaStreamSynchronize(m->stream), "cudaStreamSynchronize(MLP)");
