@@ -178,10 +178,11 @@ __device__ __forceinline__ void gram_tf32(const float* X, int rs, int cs, int B,
 // prepare: W warps per group.  W = 1 runs four groups per CTA, one per warp;
 // W = 4 gives a CTA to one group, for model rows too large for four copies in
 // shared memory to leave room for more than a few warps per SM (block 7,
-// patch_time 2, YUV: 16 rows of 294 values).  Every value is computed in the
-// same order either way: the column sums and the centring by the thread that
-// owns the column, each Gram pair by one octet of lanes, each channel's
-// flat-area sums by one warp.
+// patch_time 2, YUV: 16 rows of 294 values).  The column sums and the centring
+// are the thread's that owns the column and each Gram dot is one octet's chains
+// and fold (blocks of 4 x 4 pairs per octet where the columns fit), in the same
+// order either way; only the flat-area sums, doubles that the group's warps share
+// by rows, differ between W = 1 and W = 4 in their last bits.
 template <int W, int kHeld>
 __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunch L) {
     constexpr int kGroups = kPrepareWarps / W;  // groups per CTA
@@ -527,9 +528,9 @@ __device__ __forceinline__ void jacobi_angle(float app, float aqq, float apq, fl
 }
 
 // ---------------------------------------------------------------------------
-// jacobi: topk_symmetric_eigen_jacobi (linalg.cpp:447-519) for many groups per
-// warp.  A group owns a segment of `seg` lanes (a power of two >= its rows,
-// at most 32); lane r of the segment owns matrix rows r, r + seg, ...
+// jacobi: topk_symmetric_eigen_jacobi (linalg.cpp:447-519) for matrices of more
+// than 32 rows.  A group owns a segment of `seg` lanes (16 or 32, jacobi_shape);
+// lane r of the segment owns matrix rows r, r + seg, ...
 __global__ void __launch_bounds__(256) jacobi_kernel(FilterLaunch L, int seg, int ld, int gstride) {
     extern __shared__ __align__(16) float sm[];
     const int N = L.nmax;  // largest matrix dimension (model rows, or the dimension for covariance models)
@@ -539,7 +540,6 @@ __global__ void __launch_bounds__(256) jacobi_kernel(FilterLaunch L, int seg, in
     const int groups_per_warp = 32 / seg;
     const int slot = (threadIdx.x >> 5) * groups_per_warp + lane / seg;  // group slot in the CTA
     const int r0 = lane % seg;
-    const unsigned seg_mask = seg == 32 ? 0xffffffffu : (((1u << seg) - 1u) << ((lane / seg) * seg));
     float* m = sm + static_cast<size_t>(slot) * gstride;
     float* v = m + N * ld;
     int* order = reinterpret_cast<int*>(v + N * ld);
@@ -672,20 +672,22 @@ __global__ void __launch_bounds__(256) jacobi_kernel(FilterLaunch L, int seg, in
             }
         }
         __syncwarp();
-        (void)seg_mask;
     }
 }
 
 // ---------------------------------------------------------------------------
 // jacobi, kSeg lanes per group, for matrices up to N x N (N = 8 to 32).  The
 // rotations of a group are one chain of dependent divisions and square roots:
-// latency bounds it, so as many groups as fit in shared memory are in flight,
-// and few lanes repeat each angle.  Against jacobi_kernel (B200, one launch
-// alone): N = 8, 32k groups 155 -> 81 us; N = 16, 57k groups 1.08 -> 0.65 ms,
-// 0.6k groups 421 -> 218 us; with FP64 angles, 130k groups, 5.0 -> 2.85 ms.  The strict upper triangle, the diagonal and the vectors lie in
-// shared memory as [element][group].  Lane h owns rows i kSeg + h; its part of
-// row p and of vector p stays in registers while q runs over an unrolled loop,
-// and the samples a rotation will need are loaded before its angle is known.
+// latency bounds it (14k groups of 16 rows: issue slots 25% busy, 45% with FP64
+// angles, whose pipe is 15% busy; a warp waits for its own last result), so as
+// many groups as fit in shared memory are in flight, and few lanes repeat each
+// angle.  Against jacobi_kernel (B200, one launch alone, the lanes per group that
+// are launched): N = 8, 32k groups 155 -> 81 us; N = 16, 57k groups 1.08 -> 0.66
+// ms, 0.6k groups 421 -> 218 us; with FP64 angles, 130k groups, 5.0 -> 3.15 ms.
+// The strict upper triangle, the diagonal and the vectors lie in shared memory as
+// [element][group].  Lane h owns rows i kSeg + h; its part of row p and of vector
+// p stays in registers while q runs over an unrolled loop, and the samples a
+// rotation will need are loaded before its angle is known.
 // For row r = p the update works on the stale copy of (p, q); the write-back of
 // row p replaces it.  Same rotations in the same order on the same values as
 // jacobi_kernel, element by element.
@@ -1208,8 +1210,10 @@ __global__ void __launch_bounds__(kApplyThreads, 3) apply_kernel(FilterLaunch L)
 // shared loads (B200, one launch alone, 57k groups of dimension 294, rank 15):
 // Basic 2.75 -> 1.19 ms, Final 3.72 -> 2.17 ms; 130k groups of dimension 128,
 // rank 16: 6.7 -> 2.87 and 7.7 -> 3.34 ms.
-// Bound by shared-memory wavefronts and FP32 issue, so the layouts serve wide
-// loads: the basis is [column][component], padded to 4 mod 8 quads so that the
+// Now bound by latency: 16 (Basic) and 12 (Final) warps of an SM issue in 43 and
+// 34% of its slots and wait for the samples, the shared loads and the barriers
+// between a group's phases; the FMA pipe is 26 and 21% busy.  The layouts serve
+// wide loads: the basis is [column][component], padded to 4 mod 8 quads so that the
 // 8 columns of a quarter warp start on different banks, and a warp's tile of
 // kTileRows rows is [column][row].  One 16-byte load then brings four
 // components (or all four rows) of a column.  Lane (j, g) runs the pinned
@@ -2264,26 +2268,16 @@ __global__ void combine_weights_kernel(FilterLaunch L) {
     }
 }
 
-// Segment width, row stride and per-group floats of the Jacobi kernel for
-// matrices up to N x N.  A segment of `seg` lanes per group, each lane owning
-// rows r0, r0 + seg, ...; two rows per lane from 8 rows up, which halves the
-// rotation parameters every lane recomputes.  Rows are padded to N + 1 and
-// groups to gstride floats: for N = 8 (segments of 4, 8 groups per warp,
-// gstride = 4 mod 32) the lanes of a warp touch 32 distinct banks.  Wider
-// segments when a warp's groups would not fit in shared memory (N > 119: one
-// group per warp).
+// Segment width, row stride and per-group floats of jacobi_kernel for matrices of
+// N > 32 rows: two groups per warp while both fit in shared memory (N up to 119),
+// else one.  Rows are padded to N + 1.
 struct JacobiShape {
     int seg, ld, gstride;
 };
 JacobiShape jacobi_shape(int N) {
-    int seg = 1;
-    while (seg < N && seg < 32) seg <<= 1;
-    if (seg >= 8) seg /= 2;
-    seg = std::max(seg, 1);
     const int ld = N + 1;
-    int gstride = 2 * N * ld + N;
-    if (seg == 4) gstride += ((4 - gstride % 32) + 32) % 32;
-    while (seg < 32 && static_cast<size_t>(32 / seg) * gstride * sizeof(float) > kFilterSharedLimit) seg <<= 1;
+    const int gstride = 2 * N * ld + N;
+    const int seg = 2 * static_cast<size_t>(gstride) * sizeof(float) > kFilterSharedLimit ? 32 : 16;
     return JacobiShape{seg, ld, gstride};
 }
 
@@ -2316,8 +2310,9 @@ cudaError_t launch_apply_warp(const FilterLaunch& L, int max_groups, cudaStream_
 // Warps per block of the row-tile apply for this shape, 0 where the
 // row-per-warp kernel runs: no rank, ranks above 32, dimensions of 16 and less
 // (their dots have an order of their own), and shapes whose block does not fit
-// even with one warp.  Fewer warps than kTileWarps only where four do not fit
-// (dimensions of about 1500 and more), so that such shapes keep the kernel.
+// even with one warp.  Fewer warps than kTileWarps only where four do not fit, so
+// that such shapes keep the kernel: with 64 rows from dimension 1456 (Basic) or
+// 1033 (Final) at ranks up to 16, from 1003 or 777 above.
 int tile_apply_warps(const FilterLaunch& L) {
     if (L.rank < 1 || L.rank > 32 || L.dim <= 16) return 0;
     const int Bmax = std::min(L.model_cap, L.max_rows);
@@ -2350,7 +2345,7 @@ size_t filter_shared_bytes(const FilterLaunch& L) {
     const int groups_per_cta = rows_bytes > 8 * 1024 ? 1 : kPrepareWarps;
     size_t need = (colpad + static_cast<size_t>(groups_per_cta) * Bmax * (D + 8)) * sizeof(float) +
                   static_cast<size_t>(groups_per_cta) * L.max_rows * sizeof(size_t);
-    if (R > 0) {
+    if (R > 0 && L.nmax > 32) {  // the smaller ones' kernel takes 25 KB at most
         const JacobiShape js = jacobi_shape(L.nmax);
         need = std::max(need, static_cast<size_t>(32 / js.seg) * js.gstride * sizeof(float));
     }
@@ -2438,7 +2433,8 @@ cudaError_t launch_filter(const FilterLaunch& L, int max_groups_in, cudaStream_t
             // leave fewer rows per lane and more warps to hide its latency
             // (1, 2 and 4 lanes: N = 8, 32k groups 77, 81, 86 us; N = 16, 57k
             // groups 0.95, 0.65, 0.66 ms, 0.6k groups 440, 290, 218 us, and
-            // with FP64 angles, 130k groups, 4.1, 3.55, 2.85 ms)
+            // with FP64 angles, 130k groups, 4.1, 3.55, 2.85 ms, the angles then
+            // without the test of their rounding)
             cudaError_t err;
             if (N <= 8) err = launch_jacobi_small<8, 2>(L, max_groups, stream);
             else if (N <= 16) err = launch_jacobi_small<16, 4>(L, max_groups, stream);
@@ -2446,9 +2442,6 @@ cudaError_t launch_filter(const FilterLaunch& L, int max_groups_in, cudaStream_t
             else err = launch_jacobi_small<32, 8>(L, max_groups, stream);
             if (err != cudaSuccess) return err;
         } else {
-            // a segment of `seg` lanes per group, each lane owning rows r0, r0 + seg,
-            // ...; two rows per lane from 8 rows up, which halves the rotation
-            // parameters every lane recomputes
             const JacobiShape js = jacobi_shape(N);
             const int seg = js.seg, ld = js.ld, gstride = js.gstride;
             const size_t per_group = static_cast<size_t>(gstride) * sizeof(float);

@@ -327,7 +327,9 @@ __device__ __forceinline__ void tma_load_tile(uint32_t dst, const CUtensorMap* m
 // of 64 in shared memory, with one lane running the final partial sort, took
 // half of the kernel: 57k anchors at 960x540 YUV (block 7, a 27 x 27 window,
 // two frames) 3.08 ms for the two planes of Basic and 5.98 ms for the six of
-// Final, now 1.66 and 3.45 ms (FP32 issue alone: 0.7 and 2.0 ms).  Blocks of
+// Final, now 1.66 and 3.45 ms (its FP32 operations alone: 0.7 and 2.0 ms).  Bound
+// by issue: 75% of the slots in both (480x272, same parameters), the FMA pipe 37
+// and 47% busy, the integer and compare pipe 40 and 27%.  Blocks of
 // 10 took 9.2 ms for 83k anchors in the run-time loop, now 2.0 ms.  kPrune:
 // the later planes of candidates that can still pass only (MatchLaunch::
 // prune_cap > 0); its state costs registers, so the others do without.

@@ -253,9 +253,10 @@ __host__ __device__ __noinline__ inline float2 angle_fp64_longhand(float app, fl
 }
 
 // The same floats with one division and one square root less; the longhand is a
-// call, since inlined it takes the rotations' registers (3840x2160 gray, groups of
-// 16, Basic and Final of three frames: longhand everywhere 49.2 ms, inlined behind
-// the test 48.6, this 43.2; the filter alone changes).  With d = aqq - app and
+// call, since inlined it slows every rotation of an unrolled loop (3840x2160 gray,
+// groups of 16, Basic and Final of three frames, against the shorter steps without
+// the test: this 1.02, inlined behind the test 1.13, longhand everywhere 1.14 of
+// the whole pass).  With d = aqq - app and
 // b = 2 apq, t = sgn |b| / (|d| + sqrt(d^2 + b^2)).  Both ways are within 12
 // units of 2^-53 of the exact cosine and sine (each operation adds at most one,
 // rsqrt two, and a square root halves what came before), so they lie within 24

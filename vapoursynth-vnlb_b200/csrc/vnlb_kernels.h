@@ -74,7 +74,7 @@ struct MatchLaunch {
     int buffer_cap;       // match buffer capacity per warp
     int warp_floats;      // shared floats per warp
     int prune_cap;        // plain matcher, several planes: candidates (at most) whose later planes are computed
-                          // from a list instead of for the whole window; 0: no list (see match_prune_cap)
+                          // from a list instead of for the whole window; 0: no list (see Session::match_width_fits)
     int approx;           // chosen form in this matcher: approximate distances, exact re-rank
     // tensor-core form (match_chosen.cu)
     int tiles_x;          // 8-column candidate blocks per strip
