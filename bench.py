@@ -546,11 +546,11 @@ def measure_frame_path(form, args, ranks, noisy, local, threads=8):
 # the Basic and Final launches; the filter class sums prepare, Jacobi and
 # apply.  None where no capture of the current kernels exists.
 TRAFFIC_PER_LAUNCH = {
-    ("cpu", "match/plain"): 57.4e6,        # match_kernel<8,0,0>: Basic 31.8 MB, Final 83.0 MB
-    ("cpu", "match/chosen_tc"): 342.7e6,   # strip offsets + tc_distance + tc_select: 286.9 / 398.5 MB
-    ("cpu", "filter/plain"): 492.8e6,      # prepare + jacobi + apply: Basic 402.0 MB, Final 583.6 MB
-    ("cpu", "filter/chosen"): 503.9e6,     # the same, apply adding rows into pixel-interleaved stacks:
-    ("cpu", "filter/chosen_tc"): 503.9e6,  # 415.3 / 592.5 MB
+    ("cpu", "match/plain"): 57.4e6,        # match_kernel<8,0,0,1,0>: Basic 31.7 MB, Final 83.0 MB
+    ("cpu", "match/chosen_tc"): 342.3e6,   # strip offsets + tc_distance + tc_select: 286.6 / 397.9 MB
+    ("cpu", "filter/plain"): 500.1e6,      # prepare + jacobi + apply: Basic 405.8 MB, Final 594.4 MB
+    ("cpu", "filter/chosen"): 510.8e6,     # the same, apply adding rows into pixel-interleaved stacks:
+    ("cpu", "filter/chosen_tc"): 510.8e6,  # 418.4 / 603.2 MB
 }
 TRAFFIC_SOURCE = ("ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum "
                   "--clock-control none python bench.py --profile-case --form chosen_tc (and --form plain)")

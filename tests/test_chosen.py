@@ -124,9 +124,9 @@ def test_tensor_core_matcher_on_vnlbcu_defaults(stage, tau):
     distance (the chosen forms' step 4).  With tau raised to 1e8 (above any
     distance of 294 samples in [-0.5, 1.5]) every candidate passes the
     threshold, so every group keeps a full buffer of 64
-    rows: the buffer's second register per lane and the replacement of its
-    worst entry carry the selection, and the plain form's heap replay leaves
-    rows past the K-th unsorted where the tensor-core path sorts them, which
+    rows: the log of candidates and the 64 smallest kept of it carry the
+    selection, and the plain form's heap replay leaves rows past the K-th
+    unsorted where the tensor-core path sorts them, which
     shows that path ran."""
     _, noisy = synth.make_clip(128, 96, 5, 3, 20.0, seed=86)
     ref = vnlbcu.Basic(noisy, sigma=20.0) if stage == lib.STAGE_FINAL else None
@@ -197,7 +197,7 @@ def test_tensor_core_waits_run_out_and_report():
 
 def test_tensor_core_buffers_of_96():
     """group_size 24 with cap factor 4: buffers of 96 entries, three slots per
-    lane in the selection replay (the mixed stream's sigma-5 setting); rank
+    lane in the selection (the mixed stream's sigma-5 setting); rank
     24, patch_time 2 on a gray clip (two planes).  Rows agree with the plain
     form's on most groups with its exact distance bits, and the output is
     within 0.05 dB of the plain form's."""
