@@ -510,11 +510,11 @@ __global__ void __launch_bounds__(32 * kPrepareWarps) prepare_kernel(FilterLaunc
 
 // The rotation (c, s) that zeroes apq (jacobi_rotate, linalg.cpp:152-196).
 // kMixed (chosen forms): in FP64, so that near-degenerate pairs (aqq - app
-// tiny against apq) keep their angle.
-template <bool kMixed>
+// tiny against apq) keep their angle; kInline for short unrolled loops.
+template <bool kMixed, bool kInline>
 __device__ __forceinline__ void jacobi_angle(float app, float aqq, float apq, float& c, float& s) {
     if constexpr (kMixed) {
-        const float2 r = angle_fp64(app, aqq, apq);
+        const float2 r = kInline ? angle_fp64(app, aqq, apq) : angle_fp64_call(app, aqq, apq);
         c = r.x;
         s = r.y;
     } else {
@@ -591,8 +591,8 @@ __global__ void __launch_bounds__(256) jacobi_kernel(FilterLaunch L, int seg, in
                         __syncwarp();
                         if (rot) {
                             float c, s;
-                            if (L.mixed) jacobi_angle<true>(app, aqq, apq, c, s);
-                            else jacobi_angle<false>(app, aqq, apq, c, s);
+                            if (L.mixed) jacobi_angle<true, true>(app, aqq, apq, c, s);
+                            else jacobi_angle<false, true>(app, aqq, apq, c, s);
                             for (int r = r0; r < B; r += seg) {
                                 if (r != p && r != q) {
                                     const float arp = m[r * ld + p];
@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(32) jacobi_small_kernel(FilterLaunch L) {
                 float dq = 0.0f;
                 if (rot) {
                     float c, s;
-                    jacobi_angle<kMixed>(app, aqq, apq, c, s);
+                    jacobi_angle<kMixed, N <= 8>(app, aqq, apq, c, s);
 #pragma unroll
                     for (int i = 0; i < kRows; ++i) {
                         const bool own = i == q / kSeg && i * kSeg + h == q;

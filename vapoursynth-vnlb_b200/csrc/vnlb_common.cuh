@@ -253,10 +253,7 @@ __host__ __device__ __noinline__ inline float2 angle_fp64_longhand(float app, fl
 }
 
 // The same floats with one division and one square root less; the longhand is a
-// call, since inlined it slows every rotation of an unrolled loop (3840x2160 gray,
-// groups of 16, Basic and Final of three frames, against the shorter steps without
-// the test: this 1.02, inlined behind the test 1.13, longhand everywhere 1.14 of
-// the whole pass).  With d = aqq - app and
+// call, off the usual path.  With d = aqq - app and
 // b = 2 apq, t = sgn |b| / (|d| + sqrt(d^2 + b^2)).  Both ways are within 12
 // units of 2^-53 of the exact cosine and sine (each operation adds at most one,
 // rsqrt two, and a square root halves what came before), so they lie within 24
@@ -287,6 +284,14 @@ __host__ __device__ __forceinline__ float2 angle_fp64(float app, float aqq, floa
         !(fabsf(r.y) >= 0x1p-120f))
         return angle_fp64_longhand(app, aqq, apq);
     return r;
+}
+
+// As a call: a loop of rotations unrolled over 16 columns or more spends its time
+// on fetching the steps otherwise (Basic and Final of a gray clip of three frames,
+// inlined and called: 3840x2160, groups of 16, 46.8 and 43.0 ms; groups of 24, 181
+// and 129 ms; over 8 columns 2.20 and 2.22 ms at 1280x720).
+__host__ __device__ __noinline__ inline float2 angle_fp64_call(float app, float aqq, float apq) {
+    return angle_fp64(app, aqq, apq);
 }
 
 // std::max / std::min on floats (first operand wins ties and NaNs).
