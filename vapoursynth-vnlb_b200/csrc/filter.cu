@@ -678,12 +678,12 @@ __global__ void __launch_bounds__(256) jacobi_kernel(FilterLaunch L, int seg, in
 // ---------------------------------------------------------------------------
 // jacobi, kSeg lanes per group, for matrices up to N x N (N = 8 to 32).  The
 // rotations of a group are one chain of dependent divisions and square roots:
-// latency bounds it (14k groups of 16 rows: issue slots 25% busy, 45% with FP64
-// angles, whose pipe is 15% busy; a warp waits for its own last result), so as
+// latency bounds it (14k groups of 16 rows: issue slots 25% busy, 49% with FP64
+// angles, whose pipe is 16% busy; a warp waits for its own last result), so as
 // many groups as fit in shared memory are in flight, and few lanes repeat each
 // angle.  Against jacobi_kernel (B200, one launch alone, the lanes per group that
 // are launched): N = 8, 32k groups 155 -> 81 us; N = 16, 57k groups 1.08 -> 0.66
-// ms, 0.6k groups 421 -> 218 us; with FP64 angles, 130k groups, 5.0 -> 3.15 ms.
+// ms, 0.6k groups 421 -> 218 us; with FP64 angles, 130k groups, 5.0 -> 2.4 ms.
 // The strict upper triangle, the diagonal and the vectors lie in shared memory as
 // [element][group].  Lane h owns rows i kSeg + h; its part of row p and of vector
 // p stays in registers while q runs over an unrolled loop, and the samples a
